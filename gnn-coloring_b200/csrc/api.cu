@@ -122,7 +122,7 @@ void gc_graph_free_buffers(gc_graph *g) {
                     g->frontier2, g->removed, g->leaf_list, g->vorder, g->rank,     g->p64,      g->seg_voff,
                     g->seg_stat,  g->fmask,    g->jprec, g->class_first,
                     g->gnn_ctr,   g->hub_aux, g->jpsplit, g->part_tiles, g->giant_off, g->hub_stage,
-                    g->row_of,    g->Er,      g->vrow};
+                    g->row_of,    g->Er,      g->vrow,    g->flow_q};
     for (void *p : bufs) gc_dev_free(ctx, p);
 }
 
@@ -276,6 +276,54 @@ gc_status reupload_overlapped(gc_ctx *ctx, gc_graph *g, const uint32_t *V, const
     return GC_OK;
 }
 
+// Colors by the current keys: the dataflow kernels where the graph allows them, else the tickets.  The
+// dataflow's result stands only once the state shows that it did not stall (`*unread` is then true:
+// the caller reads the state, and calls color_by_tickets when flow_stall is set).
+gc_status color_by_keys(gc_ctx *ctx, gc_graph *g, bool *unread) {
+    // Culberson rounds on the library's own colors have a path of their own
+    *unread = gc_flow_eligible(g) && !(g->key_kind == 100 && ctx->jp_classes);
+    if (!*unread) return gc_jp_color(g);
+    gc_status s = gc_jp_flow(g);
+    if (s != GC_OK) return s;
+    g->has_colors = true;
+    g->colors_ours = true;
+    return GC_OK;
+}
+
+gc_status color_by_tickets(gc_ctx *ctx, gc_graph *g) {
+    gc_status s = gc_reset_state(ctx);
+    return s == GC_OK ? gc_jp_color(g) : s;
+}
+
+// The coloring by the current keys (when `first`), then `rounds` Culberson rounds, then the color count
+// when it is asked for.  The last coloring's errors, stall flag and statistics come back in one read.
+gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *colors_used) {
+    gc_status s;
+    if ((s = gc_reset_state(ctx)) != GC_OK) return s;
+    bool unread = false;  // a dataflow coloring whose stall flag has not been read
+    for (int it = first ? 0 : 1; it <= rounds; it++) {
+        if (unread) {  // the next keys are these colors
+            if ((s = gc_read_state(ctx)) != GC_OK) return s;
+            if (ctx->hstate->flow_stall && (s = color_by_tickets(ctx, g)) != GC_OK) return s;
+            unread = false;
+        }
+        if (it > 0) {
+            if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
+            g->has_keys = true;
+        }
+        if ((s = color_by_keys(ctx, g, &unread)) != GC_OK) return s;
+    }
+    for (;;) {
+        if (colors_used && (s = gc_queue_color_stats(g)) != GC_OK) return s;
+        if ((s = gc_read_state(ctx)) != GC_OK) return s;
+        if (!unread || !ctx->hstate->flow_stall) break;
+        if ((s = color_by_tickets(ctx, g)) != GC_OK) return s;
+        unread = false;
+    }
+    if (colors_used) g->colors_used = *colors_used = gc_colors_of_state(g);
+    return GC_OK;
+}
+
 }  // namespace
 
 
@@ -318,6 +366,8 @@ gc_status gc_ctx_create(int device, gc_ctx **out) {
     // tuning of the coloring kernel's polling (defaults measured on B200)
     if (const char *e = getenv("GC_JP_CTAS_PER_SM")) ctx->jp_ctas_per_sm = atoi(e);
     if (const char *e = getenv("GC_JP_TIGHT")) ctx->jp_tight = (unsigned int)strtoul(e, nullptr, 10);
+    if (const char *e = getenv("GC_JP_FLOW")) ctx->flow_max_deg = (uint32_t)strtoul(e, nullptr, 10);
+    if (const char *e = getenv("GC_JP_FLOW_CTAS")) ctx->flow_ctas_per_sm = std::max(1, atoi(e));
     if (const char *e = getenv("GC_JP_CLASSES")) ctx->jp_classes = atoi(e) != 0;
     if (const char *e = getenv("GC_JP_DECIDE")) ctx->jp_decide = atoi(e) != 0;
     if (const char *e = getenv("GC_JP_LIGHT_WARPS")) ctx->jp_light_warps = atoi(e);
@@ -676,42 +726,14 @@ gc_status gc_color(gc_ctx *ctx, gc_graph *g, int recolor, int *colors_used) {
     if (!ctx || !g || g->ctx != ctx || recolor < 0) return GC_ERR_INVALID;
     if (!g->has_keys) return gc_fail(ctx, GC_ERR_STATE, "no priorities: call gc_priority or gc_priority_set first");
     DeviceGuard dg(ctx);
-    gc_status s;
-    if ((s = gc_reset_state(ctx)) != GC_OK) return s;
-    if ((s = gc_jp_color(g)) != GC_OK) return s;
-    for (int it = 0; it < recolor; it++) {
-        if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
-        if ((s = gc_jp_color(g)) != GC_OK) return s;
-    }
-    if ((s = gc_read_state(ctx)) != GC_OK) return s;
-    if (colors_used) {
-        int C = 0;
-        if ((s = gc_validate_device(g, &C)) != GC_OK) return s;
-        *colors_used = C;
-        g->colors_used = C;
-    }
-    return GC_OK;
+    return color_rounds(ctx, g, true, recolor, colors_used);
 }
 
 gc_status gc_recolor(gc_ctx *ctx, gc_graph *g, int iters, int *colors_used) {
     if (!ctx || !g || g->ctx != ctx || iters < 0) return GC_ERR_INVALID;
     if (!g->has_colors) return gc_fail(ctx, GC_ERR_STATE, "no coloring to recolor");
     DeviceGuard dg(ctx);
-    gc_status s;
-    if ((s = gc_reset_state(ctx)) != GC_OK) return s;
-    for (int it = 0; it < iters; it++) {
-        if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
-        g->has_keys = true;
-        if ((s = gc_jp_color(g)) != GC_OK) return s;
-    }
-    if ((s = gc_read_state(ctx)) != GC_OK) return s;
-    if (colors_used) {
-        int C = 0;
-        if ((s = gc_validate_device(g, &C)) != GC_OK) return s;
-        *colors_used = C;
-        g->colors_used = C;
-    }
-    return GC_OK;
+    return color_rounds(ctx, g, false, iters, colors_used);
 }
 
 gc_status gc_validate(gc_ctx *ctx, gc_graph *g, int *max_color) {

@@ -49,6 +49,9 @@ struct gc_ctx {
     unsigned int jp_tight = 32;          // coloring: unproductive polling rounds before sleeping
     unsigned int jp_nap = 32;            // coloring: first sleep between polling rounds (ns)
     bool jp_decide = true;               // coloring: early decisions from published forbidden colors
+    uint32_t flow_max_deg = 128;         // coloring: graphs with a smaller maximum degree go by dataflow (0: none; GC_JP_FLOW)
+    int flow_ctas_per_sm = 8;            // dataflow kernel: CTAs per SM at most (GC_JP_FLOW_CTAS)
+    int flow_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each dataflow kernel
     bool jp_classes = true;              // Culberson rounds: class by class instead of tickets
     uint32_t jp_core_max = 32768;        // coloring: first tickets colored inside one cluster (0: off; GC_JP_CORE)
     int jp_core_cluster = -1;            // CTAs of that cluster (16 or 8; 0: unavailable; -1: not yet queried)
@@ -118,6 +121,7 @@ struct gc_graph {
     uint32_t *part_tiles = nullptr; // heavy tickets per tile of the split (prefix)
     uint32_t *class_first = nullptr;  // Culberson rounds: first ticket position of each key (old color)
     size_t class_cap = 0;
+    uint32_t *flow_q = nullptr;       // dataflow coloring: queue counters and slots (k_flow.cu)
     // forbidden colors 1..256 published by waiting vertices of the ordered coloring kernel:
     // GC_JP_MASK_WORDS words per vertex, each (epoch << 32 | 32 color bits); the word after the
     // last vertex's holds the epoch counter, advanced once per coloring run
@@ -235,8 +239,15 @@ gc_status gc_priority_gnn(gc_graph *g, const gc_model *m);         // GraphSAGE 
 gc_status gc_gnn_rows_begin(gc_graph *g);
 gc_status gc_gnn_row_ids(gc_graph *g, uint32_t first, uint32_t count);
 gc_status gc_jp_color(gc_graph *g);                                // JP by current keys (k_jp.cu)
+// JP by current keys as a dataflow, on graphs of small maximum degree (k_flow.cu).  Queued only: once
+// the state has been read, a set flow_stall means that the colors are incomplete and gc_jp_color must
+// run instead.
+bool gc_flow_eligible(const gc_graph *g);
+gc_status gc_jp_flow(gc_graph *g);
 gc_status gc_keys_from_colors(gc_graph *g);                        // Culberson step (k_jp.cu)
 gc_status gc_validate_device(gc_graph *g, int *max_color);         // (k_jp.cu)
+gc_status gc_queue_color_stats(gc_graph *g);  // the validation kernel alone, into a reset state (k_jp.cu)
+int gc_colors_of_state(const gc_graph *g);    // its result once the state has been read
 // Vertex sorts (k_sort.cu): descending key, ascending id on ties, over the vertices a filter keeps.
 enum { SORT_KEEP_ALL = 0, SORT_KEEP_INNER = 1, SORT_KEEP_DEG_AT_MOST = 2 };
 gc_status gc_sort_vertices(gc_graph *g, const uint32_t *keys, int key_bits, int filter, uint32_t max_deg,

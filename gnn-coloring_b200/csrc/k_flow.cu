@@ -1,0 +1,348 @@
+// Jones-Plassmann on graphs of small maximum degree, as a dataflow (reference src/coloring.c:223-330).
+//
+// Meshes, geometric and Erdos-Renyi graphs have short neighbour lists, and their priority DAG is often
+// a wavefront: on a stencil the priority follows the vertex id, so the vertices that are ready at one
+// time lie far apart in the priority order.  Kernels that hand vertices out in priority order (k_jp.cu)
+// then see only the few ready ones inside their window.  Here a vertex is handed out when it is ready:
+//
+//   1. init - one pass over the edges.  Each vertex records which of its neighbours precede it, as a
+//             bit mask, and how many do (rem, in its counter word).  Sources (no predecessor) take
+//             color 1 and are queued.
+//   2. flow - a warp takes a queued vertex u, one lane per neighbour.  It subtracts one from rem of
+//             every successor.  It goes on with the first successor whose rem it took to zero and
+//             queues the others, then reads the predecessors' colors and stores the smallest color
+//             none of them has.
+//
+// rem counts predecessors that have STARTED, not those that are done: the subtractions go out before
+// u's own color is known, so a successor's neighbour ids are fetched while u still waits.  A vertex
+// therefore polls its predecessors' colors (all held by running warps); the color is itself the whole
+// message, so no fences are needed.
+//
+// The queue is FLOW_QUEUES arrays, vertex v in array v mod FLOW_QUEUES, each with its own head and tail
+// counter: a single counter serves an atomic every 0.7 ns, which alone would cost 10 ms for 16.8 M
+// vertices.  FLOW_QUEUES is odd so that the regular strides of a mesh spread over the arrays.  Every
+// vertex is either queued in its array once or gone on with once (the array's skip counter), so an
+// array is done after as many vertices as it has, and warps take its slots in order: a slot below the
+// tail always belongs to a running warp.  Arrays are served by the warps whose number (in the order in
+// which the CTAs start) has that remainder: the first four CTAs that run serve them all, so the kernel
+// advances whatever else occupies the GPU.
+//
+// A CSR that is not symmetric (a caller's mistake that the upload does not check) can leave vertices
+// that never become ready.  Idle warps watch the counters; when none moves for a while they set
+// DevState::flow_stall and every warp leaves.  The host then runs the ticket kernels, whose waits
+// only follow each vertex's own list.
+//
+// What bounds it: on a wavefront the chain of hops, each a counter atomic, then the neighbour ids, then
+// the next atomic (about 1.7 us); elsewhere the vertices in flight (one per warp, 2 to 3 us each).
+// Measured on a B200, coloring kernels of one job, tickets (sort, cluster core, streams, ticket kernel,
+// leaves) -> dataflow: 256^3 stencil with GNN4 keys 272 -> 11 ms, 97 x 61 x 113 stencil first fit
+// 8.9 -> 1.1 ms, random geometric 2^23 GNN4 4.0 -> 2.7 ms, Erdos-Renyi 65,536 LF 0.36 -> 0.13 ms.
+// Measured and not kept: eight lanes per vertex and four vertices per warp (hops of 3.3 us: the longer
+// code path of a lane is on the chain), a separate 16-byte record (hops of 1.9 us), a slot taken
+// before the color is stored, four slots taken at once under backlog.
+#include <algorithm>
+
+#include "gc_internal.h"
+
+namespace {
+using namespace gc;
+
+constexpr uint32_t FLOW_QUEUES = 31;
+constexpr uint32_t FLOW_PAD = 32;  // words between counters: one 128-byte line each
+constexpr uint32_t FLOW_CTA = 3 * FLOW_QUEUES * FLOW_PAD;  // the CTAs' start counter
+constexpr uint32_t FLOW_SLOTS = FLOW_CTA + FLOW_PAD;       // first queue slot
+constexpr int FLOW_THREADS = 256;
+
+// A vertex's counter word: rem in bits 48..63, the degree in bits 32..47, the first CSR entry below.
+// The subtraction that makes a successor ready so returns where its neighbour list is, and the list is
+// on its way one load earlier.  rem is the top field: one subtraction too many (a self-loop, a CSR that
+// is not symmetric) wraps there and leaves the others alone.
+constexpr unsigned long long FLOW_ONE = 1ull << 48;
+// W words of 32 mask bits per vertex (bit j of word w: neighbour 32 w + j precedes).
+constexpr int FLOW_WIDE = 4;
+template <int W>
+struct FlowMask;
+template <>
+struct FlowMask<1> {
+    using T = uint32_t;
+    static __device__ __forceinline__ void get(T t, uint32_t *m) { m[0] = t; }
+    static __device__ __forceinline__ T put(const uint32_t *m) { return m[0]; }
+};
+template <>
+struct FlowMask<2> {
+    using T = uint2;
+    static __device__ __forceinline__ void get(T t, uint32_t *m) { m[0] = t.x, m[1] = t.y; }
+    static __device__ __forceinline__ T put(const uint32_t *m) { return make_uint2(m[0], m[1]); }
+};
+template <>
+struct FlowMask<4> {
+    using T = uint4;
+    static __device__ __forceinline__ void get(T t, uint32_t *m) { m[0] = t.x, m[1] = t.y, m[2] = t.z, m[3] = t.w; }
+    static __device__ __forceinline__ T put(const uint32_t *m) { return make_uint4(m[0], m[1], m[2], m[3]); }
+};
+
+__device__ __forceinline__ uint32_t *flow_head(uint32_t *fq, uint32_t k) { return fq + k * FLOW_PAD; }
+__device__ __forceinline__ uint32_t *flow_tail(uint32_t *fq, uint32_t k) { return fq + (FLOW_QUEUES + k) * FLOW_PAD; }
+__device__ __forceinline__ uint32_t *flow_skip(uint32_t *fq, uint32_t k) { return fq + (2 * FLOW_QUEUES + k) * FLOW_PAD; }
+
+// Queues vertex v: slots hold v + 1, so that the zeroed buffer reads as empty.
+__device__ __forceinline__ void flow_push(uint32_t *fq, uint32_t stride, uint32_t v) {
+    const uint32_t k = v % FLOW_QUEUES;
+    const uint32_t at = atomicAdd(flow_tail(fq, k), 1u);
+    if (at < stride) st_relaxed_u32(fq + FLOW_SLOTS + (size_t)k * stride + at, v + 1u);
+}
+
+// Four lanes per vertex, vertices in id order (records, CSR offsets and rows stream).
+template <int W>
+__global__ void __launch_bounds__(FLOW_THREADS) k_flow_init(const uint32_t *__restrict__ V, const uint32_t *__restrict__ E,
+                                                            const uint32_t *__restrict__ key, uint32_t N,
+                                                            unsigned long long *__restrict__ word,
+                                                            typename FlowMask<W>::T *__restrict__ mask,
+                                                            int *__restrict__ color,
+                                                            uint32_t *__restrict__ fq, uint32_t stride) {
+    constexpr int LOADS = 8;
+    const int lane = threadIdx.x & 31, q = lane & 3, qbase = lane & ~3;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint64_t keep = l2_keep_policy();  // the keys (4N bytes) stay in L2 while E streams past
+    for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 8; base < N; base += nwarps * 8) {
+        const uint32_t u = base + (lane >> 2);
+        const bool valid = u < N;
+        const uint32_t beg = valid ? V[u] : 0u, d = valid ? V[u + 1] - beg : 0u;
+        const uint32_t ku = valid ? key[u] : 0u;
+        const uint32_t dmax = __reduce_max_sync(0xffffffffu, d);
+        uint32_t m[W];
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+            m[w] = 0;
+            if (32u * w >= dmax) continue;
+            uint32_t v[LOADS], kv[LOADS];
+#pragma unroll
+            for (int k = 0; k < LOADS; k++) {
+                const uint32_t i = 32 * w + 4 * k + q;
+                v[k] = i < d ? ld_stream(E + beg + i) : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < LOADS; k++) kv[k] = 32 * w + 4 * k + q < d ? ld_keep(key + v[k], keep) : 0u;
+#pragma unroll
+            for (int k = 0; k < LOADS; k++) {
+                const bool pk = 32 * w + 4 * k + q < d && precedes(kv[k], v[k], ku, u);
+                m[w] |= ((__ballot_sync(0xffffffffu, pk) >> qbase) & 0xfu) << (4 * k);
+            }
+            cnt += __popc(m[w]);
+        }
+        if (valid && q == 0) {
+            word[u] = (unsigned long long)cnt * FLOW_ONE | (unsigned long long)d << 32 | beg;
+            mask[u] = FlowMask<W>::put(m);
+            color[u] = cnt == 0 ? 1 : 0;
+            if (cnt == 0) flow_push(fq, stride, u);
+        }
+    }
+}
+
+// Vertices started or queued so far; every lane gets it.
+__device__ __forceinline__ uint32_t flow_progress(uint32_t *fq, int lane) {
+    return __reduce_add_sync(0xffffffffu, lane < (int)FLOW_QUEUES ? ld_relaxed_u32(flow_tail(fq, lane)) +
+                                                                        ld_relaxed_u32(flow_skip(fq, lane))
+                                                                  : 0u);
+}
+
+// One more fruitless poll of a warp: true when the warp must leave.  After `check` polls the warp
+// compares the tails with their last sum; unchanged means that nothing moves.
+struct FlowWait {
+    uint32_t spins = 0, seen = 0xffffffffu;
+    __device__ __forceinline__ bool give_up(uint32_t *fq, DevState *st, uint32_t check, int lane) {
+        ++spins;
+        if ((spins & 1023u) == 0 && __shfl_sync(0xffffffffu, lane == 0 ? ld_relaxed_u32(&st->flow_stall) : 0u, 0)) return true;
+        if (spins <= check) return false;
+        const uint32_t now = flow_progress(fq, lane);
+        if (now == seen) {
+            if (lane == 0) st_relaxed_u32(&st->flow_stall, 1u);
+            return true;
+        }
+        seen = now;
+        spins = 0;
+        return false;
+    }
+};
+
+template <int W>
+__global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsigned long long *word,
+                                                          const typename FlowMask<W>::T *__restrict__ mask,
+                                                          const uint32_t *__restrict__ E, int *color, uint32_t *fq,
+                                                          uint32_t N, uint32_t stride, DevState *st, uint32_t check) {
+    constexpr unsigned int FULL = 0xffffffffu;
+    __shared__ uint32_t cta_s;
+    if (threadIdx.x == 0) cta_s = atomicAdd(fq + FLOW_CTA, 1u);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const uint32_t k = (cta_s * (FLOW_THREADS / 32) + (threadIdx.x >> 5)) % FLOW_QUEUES;
+    const uint32_t nk = k < N ? (N - k + FLOW_QUEUES - 1) / FLOW_QUEUES : 0u;  // vertices of this array
+    uint32_t *head = flow_head(fq, k), *skip = flow_skip(fq, k);
+    const uint32_t *slots = fq + FLOW_SLOTS + (size_t)k * stride;
+    FlowWait fw;
+    uint32_t u, d, v[W];  // the vertex, its degree, and this lane's neighbours (entries 32 w + lane)
+    typename FlowMask<W>::T mt;
+    auto fetch = [&](uint32_t lo, uint32_t hi) {  // from the vertex's counter word
+        d = hi & 0xffffu;
+#pragma unroll
+        for (int w = 0; w < W; w++) v[w] = 32u * w + lane < d ? ld_stream(E + lo + 32 * w + lane) : 0u;
+        mt = __ldg(mask + u);
+    };
+    for (;;) {
+        // a queued vertex: take a slot and wait until it is filled, or can no longer be (vertices that a
+        // warp went on with leave that many slots at the array's end unfilled)
+        uint32_t slot = 0, u1 = 0;
+        if (lane == 0) slot = atomicAdd(head, 1u);
+        slot = __shfl_sync(FULL, slot, 0);
+        if (slot >= nk) return;
+        for (;;) {
+            u1 = __shfl_sync(FULL, lane == 0 ? ld_relaxed_u32(slots + slot) : 0u, 0);
+            if (u1) break;
+            if ((fw.spins & 7u) == 7u && slot + min(nk, __shfl_sync(FULL, lane == 0 ? ld_relaxed_u32(skip) : 0u, 0)) >= nk) return;
+            if (fw.give_up(fq, st, check, lane)) return;
+        }
+        fw.spins = 0;
+        u = u1 - 1u;
+        {
+            const unsigned long long wu = __ldcg(word + u);
+            fetch((uint32_t)wu, (uint32_t)(wu >> 32));
+        }
+        for (;;) {  // u, then a successor that u made ready, and so on
+            uint32_t m[W], wait = 0;  // wait, bit w: entry 32 w + lane is a predecessor without a color
+            FlowMask<W>::get(mt, m);
+            uint32_t got[W];             // predecessors' colors
+            unsigned long long old[W];   // successors' counter words before this subtraction
+            uint32_t keep[W];            // (v[] is refilled for the next vertex below)
+#pragma unroll
+            for (int w = 0; w < W; w++) {  // all in flight
+                got[w] = 0;
+                old[w] = 0;
+                keep[w] = v[w];
+                if (32u * w + lane < d) {
+                    if ((m[w] >> lane) & 1u) {
+                        wait |= 1u << w;
+                        got[w] = (uint32_t)ld_relaxed(color + v[w]);
+                    } else {
+                        old[w] = atomicAdd(word + v[w], 0ull - FLOW_ONE);
+                    }
+                }
+            }
+            // the warp goes on with one ready successor (its list is on the way while u's color is made)
+            // and queues the others
+            const uint32_t self = u;
+            bool more = false;
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                bool ready = (uint32_t)(old[w] >> 48) == 1u;
+                const unsigned int rm = __ballot_sync(FULL, ready);
+                if (!rm) continue;
+                if (!more) {
+                    more = true;
+                    const int first = __ffs(rm) - 1;
+                    u = __shfl_sync(FULL, keep[w], first);
+                    const uint32_t lo = __shfl_sync(FULL, (uint32_t)old[w], first);
+                    const uint32_t hi = __shfl_sync(FULL, (uint32_t)(old[w] >> 32), first);
+                    fetch(lo, hi);
+                    if (lane == first) {
+                        ready = false;
+                        atomicAdd(flow_skip(fq, u % FLOW_QUEUES), 1u);
+                    }
+                }
+                if (ready) flow_push(fq, stride, keep[w]);
+            }
+            uint32_t used[W];
+#pragma unroll
+            for (int x = 0; x < W; x++) used[x] = 0;
+            FlowWait cw;
+            for (;;) {
+#pragma unroll
+                for (int w = 0; w < W; w++) {
+                    if (((wait >> w) & 1u) && got[w]) {
+                        wait &= ~(1u << w);
+#pragma unroll
+                        for (int x = 0; x < W; x++)
+                            if (W == 1 || ((got[w] - 1u) >> 5) == (uint32_t)x) used[x] |= 1u << ((got[w] - 1u) & 31u);
+                    }
+                }
+                if (!__any_sync(FULL, wait != 0u)) break;
+                if (cw.give_up(fq, st, check, lane)) return;
+#pragma unroll
+                for (int w = 0; w < W; w++)
+                    if ((wait >> w) & 1u) got[w] = (uint32_t)ld_relaxed(color + keep[w]);
+            }
+            int c = 0;
+#pragma unroll
+            for (int x = 0; x < W; x++) {
+                const uint32_t all = __reduce_or_sync(FULL, used[x]);
+                if (c == 0 && ~all) c = 32 * x + __ffs(~all);
+            }
+            if (lane == 0) st_relaxed(color + self, c);
+            if (!more) break;
+        }
+    }
+}
+
+template <int W>
+gc_status flow_run(gc_graph *g, uint32_t stride) {
+    gc_ctx *ctx = g->ctx;
+    gc_status s;
+    // counter words in the first half of the ticket records' buffer; masks in the second half (up to 8
+    // bytes per vertex), else in the ticket streams' buffer
+    unsigned long long *word = reinterpret_cast<unsigned long long *>(g->jprec);
+    using MaskT = typename FlowMask<W>::T;
+    MaskT *mask = W <= 2 ? reinterpret_cast<MaskT *>(word + g->cap_N) : reinterpret_cast<MaskT *>(g->jpsplit);
+    int &occ = ctx->flow_blocks_per_sm[W == FLOW_WIDE ? 2 : W - 1];
+    if (!occ) {
+        if ((s = gc_check_cuda(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jp_flow<W>, FLOW_THREADS, 0),
+                               "occupancy")) != GC_OK)
+            return s;
+        if (occ < 1) occ = 1;
+    }
+    if ((s = gc_check_cuda(ctx, cudaMemsetAsync(g->flow_q, 0, 4 * ((size_t)FLOW_SLOTS + (size_t)FLOW_QUEUES * stride),
+                                                ctx->stream), "flow queues")) != GC_OK)
+        return s;
+    const uint32_t N = g->N;
+    {
+        ProfScope ps(ctx, "flow_init", ctx->stream);
+        const uint32_t blocks = std::min<uint32_t>((uint32_t)ctx->num_sms * 8, (N + 63) / 64);
+        k_flow_init<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(g->V, g->E, g->key, N, word, mask, g->color, g->flow_q,
+                                                                 stride);
+    }
+    {
+        ProfScope ps(ctx, "jp_flow", ctx->stream);
+        // at least four CTAs (a warp for every array); a warp per four vertices at most
+        const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)std::min(occ, ctx->flow_ctas_per_sm);
+        const uint32_t blocks = std::max<uint32_t>(4u, std::min<uint32_t>(most, (N + 31) / 32));
+        k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->color, g->flow_q, N, stride,
+                                                               ctx->dstate, std::min<uint32_t>(ctx->spin_limit, 1u << 16));
+    }
+    ctx->launches += 2;
+    return gc_check_launch(ctx, "jp flow");
+}
+
+}  // namespace
+
+// Which graphs go by dataflow: a maximum degree below 64 always (Erdos-Renyi of mean degree 16 to 24 and
+// 0.2 to 4 M vertices, whole call: 0.20 to 1.74 ms against 0.44 to 2.01 with tickets); below 128 up to
+// FLOW_WIDE_MAX_N vertices, since the wide kernel keeps half as many vertices in flight (mean degree
+// 32, 0.5 M vertices: 0.59 against 0.71 ms; 1 M: 1.15 against 1.02).  Larger degrees would put long
+// lists on the chain, and power-law graphs have their chains colored inside one cluster (k_jp_core).
+// Plain graphs only: a batch is captured, and the stall flag needs the host.
+constexpr uint32_t FLOW_WIDE_MAX_N = 1u << 19;
+
+bool gc_flow_eligible(const gc_graph *g) {
+    const uint32_t widest = g->N <= FLOW_WIDE_MAX_N ? 32u * FLOW_WIDE : 64u;
+    return g->n_seg == 0 && g->N > 0 && g->max_deg < std::min(g->ctx->flow_max_deg, widest);
+}
+
+gc_status gc_jp_flow(gc_graph *g) {
+    gc_ctx *ctx = g->ctx;
+    gc_status s;
+    const bool wide = g->max_deg >= 64;
+    const uint32_t stride = (g->N + FLOW_QUEUES - 1) / FLOW_QUEUES;
+    if ((s = gc_alloc(ctx, &g->jprec, g->cap_N, "vertex records")) != GC_OK) return s;
+    if (wide && (s = gc_alloc(ctx, &g->jpsplit, g->cap_N, "vertex records")) != GC_OK) return s;
+    if ((s = gc_alloc(ctx, &g->flow_q, (size_t)g->cap_N + FLOW_QUEUES + FLOW_SLOTS, "flow queues")) != GC_OK) return s;
+    return wide ? flow_run<FLOW_WIDE>(g, stride) : g->max_deg >= 32 ? flow_run<2>(g, stride) : flow_run<1>(g, stride);
+}

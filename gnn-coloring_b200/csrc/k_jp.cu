@@ -1494,10 +1494,16 @@ gc_status gc_validate_device(gc_graph *g, int *max_color) {
     if ((s = gc_reset_state(ctx)) != GC_OK) return s;
     if ((s = launch_color_stats(g, nullptr, 0)) != GC_OK) return s;
     if ((s = gc_read_state(ctx)) != GC_OK) return s;
-    int C = (int)ctx->hstate->max_color;
-    if (C < 1) C = 1;
-    *max_color = ctx->hstate->invalid ? 0 : C;
+    *max_color = gc_colors_of_state(g);
     return GC_OK;
+}
+
+gc_status gc_queue_color_stats(gc_graph *g) { return g->N ? launch_color_stats(g, nullptr, 0) : GC_OK; }
+
+int gc_colors_of_state(const gc_graph *g) {
+    const gc::DevState *h = g->ctx->hstate;
+    if (g->N == 0) return 1;
+    return h->invalid ? 0 : std::max((int)h->max_color, 1);
 }
 
 gc_status gc_segment_stats(gc_graph *g) {
