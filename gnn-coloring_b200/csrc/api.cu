@@ -120,7 +120,7 @@ void gc_graph_free_buffers(gc_graph *g) {
     void *bufs[] = {g->key,       g->color,  g->P,        g->pc,       g->order,    g->sort_buf, g->sort_hist,
                     g->big,       g->hubs,   g->x,        g->y,        g->t01,      g->deg_rem,  g->frontier,
                     g->frontier2, g->removed, g->leaf_list, g->vorder, g->rank,     g->p64,      g->seg_voff,
-                    g->seg_stat,  g->fmask,    g->jprec, g->class_first,
+                    g->seg_stat,  g->fmask,    g->jprec, g->round_ctr,
                     g->gnn_ctr,   g->hub_aux, g->jpsplit, g->part_tiles, g->giant_off, g->hub_stage,
                     g->row_of,    g->Er,      g->vrow,    g->flow_q};
     for (void *p : bufs) gc_dev_free(ctx, p);
@@ -280,8 +280,7 @@ gc_status reupload_overlapped(gc_ctx *ctx, gc_graph *g, const uint32_t *V, const
 // dataflow's result stands only once the state shows that it did not stall (`*unread` is then true:
 // the caller reads the state, and calls color_by_tickets when flow_stall is set).
 gc_status color_by_keys(gc_ctx *ctx, gc_graph *g, bool *unread) {
-    // Culberson rounds on the library's own colors have a path of their own
-    *unread = gc_flow_eligible(g) && !(g->key_kind == 100 && ctx->jp_classes);
+    *unread = gc_flow_eligible(g);
     if (!*unread) return gc_jp_color(g);
     gc_status s = gc_jp_flow(g);
     if (s != GC_OK) return s;
@@ -301,17 +300,26 @@ gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *co
     gc_status s;
     if ((s = gc_reset_state(ctx)) != GC_OK) return s;
     bool unread = false;  // a dataflow coloring whose stall flag has not been read
-    for (int it = first ? 0 : 1; it <= rounds; it++) {
-        if (unread) {  // the next keys are these colors
-            if ((s = gc_read_state(ctx)) != GC_OK) return s;
-            if (ctx->hstate->flow_stall && (s = color_by_tickets(ctx, g)) != GC_OK) return s;
+    if (first && (s = color_by_keys(ctx, g, &unread)) != GC_OK) return s;
+    for (int it = 0; it < rounds;) {
+        // the next keys are these colors: they must be known to stand
+        const bool by_class = gc_rounds_eligible(g);
+        for (;;) {
+            if (by_class && (s = gc_queue_max_color(g)) != GC_OK) return s;
+            if ((by_class || unread) && (s = gc_read_state(ctx)) != GC_OK) return s;
+            if (!unread || !ctx->hstate->flow_stall) break;
+            if ((s = color_by_tickets(ctx, g)) != GC_OK) return s;
             unread = false;
         }
-        if (it > 0) {
-            if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
-            g->has_keys = true;
+        unread = false;
+        if (by_class) {
+            if ((s = gc_culberson_rounds(g, rounds - it, ctx->hstate->first_colors)) != GC_OK) return s;
+            break;
         }
+        if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
+        g->has_keys = true;
         if ((s = color_by_keys(ctx, g, &unread)) != GC_OK) return s;
+        it++;
     }
     for (;;) {
         if (colors_used && (s = gc_queue_color_stats(g)) != GC_OK) return s;

@@ -275,9 +275,13 @@ gc_status queue_pipeline(gc_batch *b, gc_heuristic h, const gc_model *m, int rec
     g->key_kind = (int)h;
     g->has_keys = true;
     if ((s = gc_jp_color(g)) != GC_OK) return s;
-    for (int it = 0; it < recolor; it++) {
-        if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
-        if ((s = gc_jp_color(g)) != GC_OK) return s;
+    if (recolor > 0 && gc_rounds_eligible(g)) {
+        if ((s = gc_culberson_rounds(g, recolor, g->max_deg + 1)) != GC_OK) return s;
+    } else {
+        for (int it = 0; it < recolor; it++) {
+            if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
+            if ((s = gc_jp_color(g)) != GC_OK) return s;
+        }
     }
     if ((s = gc_segment_stats(g)) != GC_OK) return s;
     if (b->G && (s = gc_check_cuda(ctx, cudaMemcpyAsync(b->h_stat, g->seg_stat, sizeof(int32_t) * 2 * b->G,

@@ -51,6 +51,7 @@ struct gc_ctx {
     bool jp_decide = true;               // coloring: early decisions from published forbidden colors
     uint32_t flow_max_deg = 128;         // coloring: graphs with a smaller maximum degree go by dataflow (0: none; GC_JP_FLOW)
     int flow_ctas_per_sm = 8;            // dataflow kernel: CTAs per SM at most (GC_JP_FLOW_CTAS)
+    int round_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each Culberson kernel
     int flow_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each dataflow kernel
     bool jp_classes = true;              // Culberson rounds: class by class instead of tickets
     uint32_t jp_core_max = 32768;        // coloring: first tickets colored inside one cluster (0: off; GC_JP_CORE)
@@ -119,8 +120,7 @@ struct gc_graph {
     uint4 *jprec = nullptr;         // per ticket: (vertex, first CSR entry, predecessor count, 0)
     uint4 *jpsplit = nullptr;       // the tickets after the core: heavy stream from the front, light from the back
     uint32_t *part_tiles = nullptr; // heavy tickets per tile of the split (prefix)
-    uint32_t *class_first = nullptr;  // Culberson rounds: first ticket position of each key (old color)
-    size_t class_cap = 0;
+    uint32_t *round_ctr = nullptr;    // Culberson rounds: work counters (k_round.cu)
     uint32_t *flow_q = nullptr;       // dataflow coloring: queue counters and slots (k_flow.cu)
     // forbidden colors 1..256 published by waiting vertices of the ordered coloring kernel:
     // GC_JP_MASK_WORDS words per vertex, each (epoch << 32 | 32 color bits); the word after the
@@ -245,6 +245,11 @@ gc_status gc_jp_color(gc_graph *g);                                // JP by curr
 bool gc_flow_eligible(const gc_graph *g);
 gc_status gc_jp_flow(gc_graph *g);
 gc_status gc_keys_from_colors(gc_graph *g);                        // Culberson step (k_jp.cu)
+// Culberson rounds on the library's own colors, class by class (k_round.cu); queued only.  `colors`: at
+// least the number of colors now (gc_queue_max_color leaves it in the state's first_colors).
+bool gc_rounds_eligible(const gc_graph *g);
+gc_status gc_queue_max_color(gc_graph *g);
+gc_status gc_culberson_rounds(gc_graph *g, int rounds, uint32_t colors);
 gc_status gc_validate_device(gc_graph *g, int *max_color);         // (k_jp.cu)
 gc_status gc_queue_color_stats(gc_graph *g);  // the validation kernel alone, into a reset state (k_jp.cu)
 int gc_colors_of_state(const gc_graph *g);    // its result once the state has been read

@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_sweep(SortIn in, int shif
             const uint32_t d = digit_of(k[s], shift, mask);
             const uint32_t dst = gbase[d] + wcnt[warp][d] + pos[s];
             if (dst < in.N) {
-                kout[dst] = k[s];
+                if (kout) kout[dst] = k[s];
                 vout[dst] = v[s];
             } else {
                 raise_error(st, ERR_BOUND, dst);
@@ -393,7 +393,7 @@ gc_status gc_sort_vertices(gc_graph *g, const uint32_t *keys, int key_bits, int 
     for (int p = 0; p < passes; p++) {
         in.first = (p == 0);
         uint32_t *kout = (p & 1) ? k1 : k0, *vout = (p & 1) ? v1 : v0;
-        if (p == passes - 1) vout = out;  // last pass writes the result directly
+        if (p == passes - 1) vout = out, kout = nullptr;  // the last pass writes the result directly, without the keys
         k_sort_sweep<<<ntiles, SORT_THREADS, 0, ctx->stream>>>(in, 8 * p, mask, bases + p * RADIX,
                                                                 status + (size_t)p * ntiles * RADIX, tile_ctr + p,
                                                                 kout, vout, ctx->dstate);
