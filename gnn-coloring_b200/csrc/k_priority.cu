@@ -7,6 +7,8 @@
 //
 // Keys are uint32; the coloring orders vertices by (key, id) descending, exactly like the
 // reference's double comparisons on these integer-valued priorities.
+#include <algorithm>
+
 #include "gc_internal.h"
 
 namespace {
@@ -35,127 +37,357 @@ __global__ void k_simple_keys(const uint32_t *__restrict__ V, uint32_t N, int h,
 // delta + 1.  Removal within a round depends only on the degrees at the round's start and the
 // decrements commute, so the keys equal the reference's at any thread count.
 //
-// Round state lives on the device so that rounds can be queued without host round trips:
-// kernels of a round that finds nothing left to do return immediately.
+// All rounds run in one cooperative kernel, a CTA of 1,024 threads per SM: filter, barrier, decrement,
+// barrier.  A power-law graph has hundreds of rounds, most of which remove a few vertices, so a round
+// is bound by its latencies: two grid barriers and a few dependent loads.
+//   - Once the remaining vertices fit the threads (four each), every thread keeps its own: the filter
+//     reads their degrees, and the warp that finds removed vertices of up to PEEL_WARP_DEG neighbours
+//     decrements them itself after the barrier, eight lanes each; larger ones go to a list whose
+//     vertices share all threads evenly.  Before that (large graphs, the
+//     first rounds), the filter scans a list of the remaining vertices and puts all removed ones on lists.
+//   - The decrements go to every neighbour without asking whether it is still there (nothing reads a
+//     removed vertex's degree again), so nothing waits for their results.
+//   - SL tries delta + 1 first; only when that removes nothing does it look for the smallest remaining
+//     degree (one more barrier).
+//   - When no vertex remains, the last round's decrements are left out.
+//   - The barrier's counter and the round's counts are one 16-byte word, polled together by one thread
+//     per CTA.
+// Measured (B200), three launches per round queued in batches -> this: SL on R-MAT of 2^20 vertices and
+// edge factor 16 (217 rounds) 8.2 -> 1.9 ms, on Erdos-Renyi 65,536 (16 rounds) 0.41 -> 0.10 ms.  A round
+// of the former takes about 5.5 us when it removes little (the barriers 3.8 of them) and 10 us when it
+// removes thousands (decrements of the same hubs, one at a time).  All removed vertices on lists: 2.2 ms;
+// a whole warp for every kept one: 2.3 ms.
+constexpr uint32_t GONE = 0xffffffffu;
+constexpr uint32_t NO_DEGREE = 0xffffffffu;
+constexpr int PEEL_THREADS = 1024;
+constexpr int PEEL_ITEMS = 4;              // vertices a thread keeps
+constexpr uint32_t PEEL_WARP_DEG = 64;
+constexpr unsigned int PEEL_WAIT_LIMIT = 1u << 24;  // polls of one barrier
+
 struct PeelState {
-    unsigned int alive;      // vertices still in the graph
-    unsigned int next;       // survivors appended this round
-    unsigned int removed;    // vertices removed this round
-    unsigned int delta;
-    unsigned int min_deg;    // smallest survivor degree after this round's decrements
-    unsigned int parity;     // which alive buffer is current
-    unsigned int rounds;
-    unsigned int log_mode;
+    uint4 slot[3];         // round r in slot r mod 3, cleared a round ahead: arrivals at the filter's barrier,
+                           // removed vertices on the short list (or kept by their warps), on the long list, packed
+    unsigned int pad0[20];
+    unsigned int arrived;  // arrivals at the other barriers so far
+    unsigned int pad1[31];
+    unsigned int min_deg[3];  // smallest remaining degree, when a round needs it (slots as above)
+    unsigned int min0;     // smallest degree of the graph
+    unsigned int failed;   // a barrier wait expired
+    unsigned int rounds;   // rounds run (written at the end)
 };
 
-constexpr uint32_t NOT_REMOVED = 0xffffffffu;
+__device__ __forceinline__ void red_release(unsigned int *p) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+}
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint4 ld_relaxed_v4(const uint4 *p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ bool peel_expired(PeelState *ps, unsigned int &spins) {
+    return ++spins > PEEL_WAIT_LIMIT || ((spins & 255u) == 0 && gc::ld_relaxed_u32(&ps->failed));
+}
 
-__global__ void k_peel_init(const uint32_t *__restrict__ V, uint32_t N, uint32_t *__restrict__ deg,
-                            uint32_t *__restrict__ alive, uint32_t *__restrict__ key, PeelState *ps) {
-    uint32_t local_min = 0xffffffffu;
-    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < N; u += gridDim.x * blockDim.x) {
-        uint32_t d = V[u + 1] - V[u];
+// Grid barriers: every CTA's earlier writes are visible to all after them.  False when the wait expired
+// (in some CTA).  One thread per CTA polls (thousands of warps asking one address would queue for
+// microseconds).  The first kind arrives at a round's slot and returns it: its counts are complete when
+// all CTAs have arrived, since each adds to them before it arrives.
+__device__ __forceinline__ bool peel_slot_barrier(PeelState *ps, uint4 *slot, uint4 &got) {
+    __shared__ uint4 got_s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        red_release(&slot->x);
+        unsigned int spins = 0;
+        uint4 v;
+        while ((v = ld_relaxed_v4(slot)).x != gridDim.x)
+            if (peel_expired(ps, spins)) {
+                gc::st_relaxed_u32(&ps->failed, 1u);
+                v.x = 0;
+                break;
+            }
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        got_s = v;
+    }
+    __syncthreads();
+    got = got_s;
+    return got.x != 0;
+}
+// `read`: a word to return in `value` (may be null).
+__device__ __forceinline__ bool peel_barrier(PeelState *ps, unsigned int &target, const unsigned int *read, unsigned int &value) {
+    __shared__ unsigned int ok, value_s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        target += gridDim.x;
+        red_release(&ps->arrived);
+        unsigned int spins = 0, good = 1;
+        while ((int)(ld_acquire(&ps->arrived) - target) < 0)
+            if (peel_expired(ps, spins)) {
+                gc::st_relaxed_u32(&ps->failed, 1u);
+                good = 0;
+                break;
+            }
+        ok = good;
+        if (read) value_s = gc::ld_relaxed_u32(read);
+    }
+    __syncthreads();
+    if (read) value = value_s;
+    return ok;
+}
+
+// One degree off the neighbours E[j], E[j + step], ... below end.
+__device__ __forceinline__ void peel_neighbours(const uint32_t *__restrict__ E, uint32_t j, uint32_t end, uint32_t step,
+                                                uint32_t *deg) {
+    for (; j < end && end - j > 3 * step; j += 4 * step) {
+        const uint32_t a = ld_stream(E + j), b = ld_stream(E + j + step), c = ld_stream(E + j + 2 * step),
+                       d = ld_stream(E + j + 3 * step);
+        atomicSub(deg + a, 1u);
+        atomicSub(deg + b, 1u);
+        atomicSub(deg + c, 1u);
+        atomicSub(deg + d, 1u);
+    }
+    for (; j < end; j += step) {
+        atomicSub(deg + ld_stream(E + j), 1u);
+        if (end - j <= step) break;
+    }
+}
+
+__global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__restrict__ V, const uint32_t *__restrict__ E,
+                                                         uint32_t N, int log_mode, uint32_t *deg, uint32_t *list0,
+                                                         uint32_t *list1, uint32_t *removed, uint32_t *__restrict__ key,
+                                                         PeelState *ps) {
+    constexpr unsigned int FULL = 0xffffffffu;
+    constexpr int ITEMS = PEEL_ITEMS;
+    __shared__ unsigned int cta_min;
+    __shared__ uint2 own[PEEL_THREADS / 32][32 * ITEMS];  // per warp: the lists it decrements
+    const int lane = threadIdx.x & 31;
+    const unsigned int lt = (1u << lane) - 1u;
+    const uint32_t tid = blockIdx.x * PEEL_THREADS + threadIdx.x, threads = gridDim.x * PEEL_THREADS;
+    unsigned int target = 0, value = 0;
+    // the smallest of the threads' values, for all
+    auto grid_min = [&](uint32_t v, unsigned int *at) {
+        if (threadIdx.x == 0) cta_min = NO_DEGREE;
+        __syncthreads();
+        v = __reduce_min_sync(FULL, v);
+        if (lane == 0 && v != NO_DEGREE) atomicMin(&cta_min, v);
+        __syncthreads();
+        if (threadIdx.x == 0 && cta_min != NO_DEGREE) atomicMin(at, cta_min);
+        return peel_barrier(ps, target, at, value);
+    };
+    uint32_t low = NO_DEGREE;
+    for (uint32_t u = tid; u < N; u += threads) {
+        const uint32_t d = V[u + 1] - V[u];
         deg[u] = d;
-        alive[u] = u;
-        key[u] = NOT_REMOVED;
-        local_min = min(local_min, d);
+        list0[u] = u;
+        low = min(low, d);
     }
-    local_min = __reduce_min_sync(0xffffffffu, local_min);
-    if ((threadIdx.x & 31) == 0) atomicMin(&ps->min_deg, local_min);
-}
-
-__global__ void k_peel_start(PeelState *ps, uint32_t N, int log_mode) {
-    // first threshold from the smallest degree
-    uint32_t m = ps->min_deg;
-    uint32_t delta = 0;
+    if (!grid_min(low, &ps->min0)) return;
+    uint32_t delta = value;
     if (log_mode) {
-        while (delta < 32 && (1ull << delta) < (unsigned long long)m) delta++;
-    } else {
-        delta = m;
+        delta = 0;
+        while (delta < 32 && (1ull << delta) < (unsigned long long)value) delta++;
     }
-    ps->alive = N;
-    ps->next = 0;
-    ps->removed = 0;
-    ps->delta = delta;
-    ps->min_deg = 0xffffffffu;
-    ps->parity = 0;
-    ps->rounds = 0;
-    ps->log_mode = log_mode;
-}
-
-// Split the alive list into survivors and removed vertices.
-__global__ void k_peel_filter(uint32_t *__restrict__ alive0, uint32_t *__restrict__ alive1,
-                              uint32_t *__restrict__ removed, const uint32_t *__restrict__ deg,
-                              uint32_t *__restrict__ key, PeelState *ps) {
-    const uint32_t n = ps->alive;
-    if (n == 0) return;
-    const uint32_t delta = ps->delta;
-    const unsigned long long thr = ps->log_mode ? (1ull << delta) : (unsigned long long)delta;
-    const uint32_t *cur = ps->parity ? alive1 : alive0;
-    uint32_t *nxt = ps->parity ? alive0 : alive1;
-    const int lane = threadIdx.x & 31;
-    uint32_t local_min = 0xffffffffu;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        uint32_t i = base + threadIdx.x;
-        bool valid = i < n;
-        uint32_t u = valid ? cur[i] : 0;
-        uint32_t d = valid ? deg[u] : 0;
-        bool rm = valid && (unsigned long long)d <= thr;
-        bool keep = valid && !rm;
-        if (rm) key[u] = delta;
-        if (keep) local_min = min(local_min, d);
-        // warp-aggregated appends
-        unsigned int mrm = __ballot_sync(0xffffffffu, rm), mkeep = __ballot_sync(0xffffffffu, keep);
-        unsigned int brm = 0, bkeep = 0;
-        if (lane == 0) {
-            if (mrm) brm = atomicAdd(&ps->removed, __popc(mrm));
-            if (mkeep) bkeep = atomicAdd(&ps->next, __popc(mkeep));
+    uint32_t alive = N, len = N, r = 0;
+    uint32_t *cur = list0, *other = list1;
+    uint32_t u[ITEMS], d[ITEMS], beg[ITEMS], end[ITEMS];
+    uint4 got;
+    bool done = false;
+    auto round_end = [&]() {  // once the decrements are out; the slots of the round after next are free
+        if (tid == 0) {
+            ps->slot[(r + 2) % 3] = make_uint4(0u, 0u, 0u, 0u);
+            ps->min_deg[(r + 2) % 3] = NO_DEGREE;
         }
-        brm = __shfl_sync(0xffffffffu, brm, 0);
-        bkeep = __shfl_sync(0xffffffffu, bkeep, 0);
-        unsigned int lt = (1u << lane) - 1u;
-        if (rm) removed[brm + __popc(mrm & lt)] = u;
-        if (keep) nxt[bkeep + __popc(mkeep & lt)] = u;
+        return peel_barrier(ps, target, nullptr, value);
+    };
+    auto threshold = [&]() { return !log_mode ? delta : delta < 32 ? 1u << delta : 0xffffffffu; };
+    // The neighbours of n listed vertices (list[0], list[dir], ...), each shared by as many lanes as there are
+    // for it: a power of two, at least `few`.
+    auto decrement = [&](const uint32_t *list, int dir, uint32_t n, uint32_t few) {
+        const uint32_t most = threads / n;
+        const uint32_t lanes = most <= few ? few : 1u << (31 - __clz(most)), groups = threads / lanes;
+        if (tid < groups * lanes)
+            for (uint32_t i = tid / lanes; i < n; i += groups) {
+                const uint32_t x = __ldcg(list + (long long)dir * i);
+                peel_neighbours(E, V[x] + (tid & (lanes - 1u)), V[x + 1], lanes, deg);
+            }
+    };
+    // ---- the remaining vertices on a list
+    for (bool pack = false; len > threads * ITEMS; r++) {
+        uint4 *sl = &ps->slot[r % 3];
+        const uint32_t thr = threshold();
+        // short: at most 16 neighbours for each of the lanes a vertex is sure to get in the decrement (a
+        // removed vertex has about as many neighbours as the threshold)
+        const uint32_t few = thr <= 8 ? 4u : thr <= 32 ? 8u : 32u, long_deg = 16u * few;
+        low = NO_DEGREE;
+        for (uint32_t base = (tid & ~31u) * ITEMS; base < len; base += threads * ITEMS) {
+#pragma unroll
+            for (int k = 0; k < ITEMS; k++) {
+                const uint32_t i = base + 32 * k + lane;
+                u[k] = i < len ? __ldcg(cur + i) : GONE;
+            }
+#pragma unroll
+            for (int k = 0; k < ITEMS; k++) d[k] = u[k] != GONE ? __ldcg(deg + u[k]) : 0u;
+#pragma unroll
+            for (int k = 0; k < ITEMS; k++) {  // (lists of the removed ones, all in flight)
+                beg[k] = end[k] = 0;
+                if (u[k] != GONE && d[k] <= thr) {
+                    beg[k] = V[u[k]];
+                    end[k] = V[u[k] + 1];
+                    key[u[k]] = delta;
+                    if (!pack) cur[base + 32 * k + lane] = GONE;
+                }
+            }
+            uint32_t kept = 0, shorts = 0, longs = 0;
+#pragma unroll
+            for (int k = 0; k < ITEMS; k++) {
+                const bool there = u[k] != GONE, rm = there && d[k] <= thr, is_long = end[k] - beg[k] > long_deg;
+                if (there && !rm) low = min(low, d[k]);
+                shorts += __popc(__ballot_sync(FULL, rm && !is_long));
+                longs += __popc(__ballot_sync(FULL, is_long));
+                if (pack) kept += __popc(__ballot_sync(FULL, there && !rm));
+            }
+            if (shorts | longs) {
+                uint32_t at = 0;
+                if (lane == 0 && shorts) at = atomicAdd(&sl->y, shorts);
+                if (lane == 1 && longs) at = atomicAdd(&sl->z, longs);
+                uint32_t as = __shfl_sync(FULL, at, 0), al = __shfl_sync(FULL, at, 1);
+#pragma unroll
+                for (int k = 0; k < ITEMS; k++) {
+                    const bool rm = u[k] != GONE && d[k] <= thr, is_long = end[k] - beg[k] > long_deg;
+                    const unsigned int ms = __ballot_sync(FULL, rm && !is_long), ml = __ballot_sync(FULL, is_long);
+                    if (rm && !is_long) removed[as + __popc(ms & lt)] = u[k];
+                    if (is_long) removed[N - 1u - (al + __popc(ml & lt))] = u[k];
+                    as += __popc(ms);
+                    al += __popc(ml);
+                }
+            }
+            if (pack && kept) {
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(&sl->w, kept);
+                at = __shfl_sync(FULL, at, 0);
+#pragma unroll
+                for (int k = 0; k < ITEMS; k++) {
+                    const bool keep = u[k] != GONE && d[k] > thr;
+                    const unsigned int mk = __ballot_sync(FULL, keep);
+                    if (keep) other[at + __popc(mk & lt)] = u[k];
+                    at += __popc(mk);
+                }
+            }
+        }
+        if (!peel_slot_barrier(ps, sl, got)) return;
+        const uint32_t ns = got.y, nl = got.z;
+        if (pack) {
+            len = got.w;
+            uint32_t *t = cur;
+            cur = other;
+            other = t;
+        }
+        alive -= ns + nl;
+        if (alive == 0) {
+            done = true;
+            break;
+        }
+        if (nl) decrement(removed + (N - 1u), -1, nl, PEEL_THREADS);
+        if (ns) decrement(removed, 1, ns, few);
+        pack = alive < len - len / 4 || alive <= threads * ITEMS;
+        if (ns + nl == 0 && !log_mode) {  // nothing has this degree: the next threshold is the smallest left
+            if (!grid_min(low, &ps->min_deg[r % 3])) return;
+            delta = max(delta, value);
+        } else {
+            delta++;
+        }
+        if (!round_end()) return;
     }
-    local_min = __reduce_min_sync(0xffffffffu, local_min);
-    if (lane == 0 && local_min != 0xffffffffu) atomicMin(&ps->min_deg, local_min);
-}
-
-// Each removed vertex takes one degree off every neighbour that is still in the graph.
-// One warp per removed vertex; neighbours are read coalesced.
-__global__ void k_peel_decrement(const uint32_t *__restrict__ V, const uint32_t *__restrict__ E,
-                                 const uint32_t *__restrict__ removed, uint32_t *__restrict__ deg,
-                                 const uint32_t *__restrict__ key, PeelState *ps) {
-    if (ps->alive == 0) return;
-    const uint32_t n = ps->removed;
-    const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    uint32_t local_min = 0xffffffffu;
-    for (uint32_t i = warp; i < n; i += nwarps) {
-        uint32_t u = removed[i];
-        for (uint32_t j = V[u] + lane; j < V[u + 1]; j += 32) {
-            uint32_t v = ld_stream(E + j);
-            if (key[v] != NOT_REMOVED) continue;  // removed now or earlier
-            uint32_t d = atomicSub(&deg[v], 1u) - 1u;
-            local_min = min(local_min, d);
+    // ---- each thread keeps its vertices (neighbouring list entries in different warps: the list is close to
+    // id order, and vertices that leave together are often neighbours in it)
+    if (!done) {
+        const uint32_t slot0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = threads >> 5;
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const uint32_t i = ((uint32_t)k * 32u + lane) * warps + slot0;
+            u[k] = i < len ? __ldcg(cur + i) : GONE;
+            beg[k] = end[k] = 0;
+            if (u[k] != GONE) {
+                beg[k] = V[u[k]];
+                end[k] = V[u[k] + 1];
+            }
         }
     }
-    local_min = __reduce_min_sync(0xffffffffu, local_min);
-    if (lane == 0 && local_min != 0xffffffffu) atomicMin(&ps->min_deg, local_min);
-}
-
-__global__ void k_peel_advance(PeelState *ps) {
-    if (ps->alive == 0) return;
-    uint32_t delta = ps->delta + 1;
-    if (!ps->log_mode && ps->min_deg != 0xffffffffu && ps->min_deg > delta) delta = ps->min_deg;
-    ps->delta = delta;
-    ps->alive = ps->next;
-    ps->next = 0;
-    ps->removed = 0;
-    ps->min_deg = 0xffffffffu;
-    ps->parity ^= 1u;
-    ps->rounds++;
+    for (; !done; r++) {
+        uint4 *sl = &ps->slot[r % 3];
+        const uint32_t thr = threshold();
+        low = NO_DEGREE;
+        // rm, bit k: vertex k leaves now and this warp decrements its neighbours; bit 4 + k: it goes on the list
+        uint32_t rm = 0, cnt = 0, longs = 0;
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) d[k] = u[k] != GONE ? __ldcg(deg + u[k]) : NO_DEGREE;
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const bool there = u[k] != GONE, out = there && d[k] <= thr;
+            const bool is_long = out && end[k] - beg[k] > PEEL_WARP_DEG;
+            if (out) {
+                key[u[k]] = delta;
+                rm |= (is_long ? 16u : 1u) << k;
+            } else if (there) {
+                low = min(low, d[k]);
+            }
+            cnt += __popc(__ballot_sync(FULL, out && !is_long));
+            longs += __popc(__ballot_sync(FULL, is_long));
+        }
+        if (lane == 0 && cnt) atomicAdd(&sl->y, cnt);
+        if (longs) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&sl->z, longs);
+            at = __shfl_sync(FULL, at, 0);
+#pragma unroll
+            for (int k = 0; k < ITEMS; k++) {
+                const bool is_long = (rm >> k) & 16u;
+                const unsigned int ml = __ballot_sync(FULL, is_long);
+                if (is_long) removed[N - 1u - (at + __popc(ml & lt))] = u[k];
+                at += __popc(ml);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++)
+            if ((rm >> k) & 17u) u[k] = GONE;
+        if (!peel_slot_barrier(ps, sl, got)) return;
+        const uint32_t ns = got.y, nl = got.z;
+        alive -= ns + nl;
+        if (alive == 0) {
+            r++;
+            break;
+        }
+        if (nl) decrement(removed + (N - 1u), -1, nl, 32u);
+        if (cnt) {  // the warp's own: their lists packed, eight lanes each
+            uint2 *mine = own[threadIdx.x >> 5];
+            uint32_t at = 0;
+#pragma unroll
+            for (int k = 0; k < ITEMS; k++) {
+                const bool here = (rm >> k) & 1u;
+                const unsigned int mk = __ballot_sync(FULL, here);
+                if (here) mine[at + __popc(mk & lt)] = make_uint2(beg[k], end[k]);
+                at += __popc(mk);
+            }
+            __syncwarp();
+            for (uint32_t i = lane >> 3; i < cnt; i += 4) peel_neighbours(E, mine[i].x + (lane & 7), mine[i].y, 8u, deg);
+            __syncwarp();
+        }
+        if (ns + nl == 0 && !log_mode) {
+            if (!grid_min(low, &ps->min_deg[r % 3])) return;
+            delta = max(delta, value);
+        } else {
+            delta++;
+        }
+        if (!round_end()) return;
+    }
+    if (tid == 0) ps->rounds = r ? r : 1u;
 }
 
 }  // namespace
@@ -178,42 +410,39 @@ gc_status gc_priority_peel(gc_graph *g, bool log_thresholds) {
     if ((s = gc_alloc(ctx, &g->deg_rem, g->cap_N, "peel degrees")) != GC_OK) return s;
     if ((s = gc_alloc(ctx, &g->frontier, g->cap_N, "peel list")) != GC_OK) return s;
     if ((s = gc_alloc(ctx, &g->frontier2, g->cap_N, "peel list")) != GC_OK) return s;
-    if ((s = gc_alloc(ctx, &g->removed, g->cap_N + sizeof(PeelState) / 4 + 1, "peel removed list")) != GC_OK)
-        return s;
+    const size_t state_at = ((size_t)g->cap_N + 31) & ~(size_t)31;  // words: the state starts a 128-byte line
+    if ((s = gc_alloc(ctx, &g->removed, state_at + sizeof(PeelState) / 4, "peel removed list")) != GC_OK) return s;
     // the round state sits behind the removed list
-    PeelState *ps = reinterpret_cast<PeelState *>(g->removed + g->cap_N);
-    PeelState init{};
-    init.min_deg = 0xffffffffu;
-    if ((s = gc_check_cuda(ctx, cudaMemcpyAsync(ps, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream),
+    PeelState *ps = reinterpret_cast<PeelState *>(g->removed + state_at);
+    PeelState host{};
+    host.min0 = NO_DEGREE;
+    for (auto &m : host.min_deg) m = NO_DEGREE;
+    if ((s = gc_check_cuda(ctx, cudaMemcpyAsync(ps, &host, sizeof(host), cudaMemcpyHostToDevice, ctx->stream),
                            "peel state")) != GC_OK)
         return s;
-    const int grid = ctx->num_sms * 8;
-    k_peel_init<<<grid, 256, 0, ctx->stream>>>(g->V, N, g->deg_rem, g->frontier, g->key, ps);
-    k_peel_start<<<1, 1, 0, ctx->stream>>>(ps, N, log_thresholds ? 1 : 0);
-    ctx->launches += 2;
-    if ((s = gc_check_launch(ctx, "peel init")) != GC_OK) return s;
-    // Rounds are queued in batches; a batch past the last round costs only empty launches.
-    PeelState host{};
-    uint32_t queued = 0;
-    uint32_t batch = log_thresholds ? 16 : 32;
-    for (;;) {
-        ProfScope prof(ctx, "peel_rounds", ctx->stream);
-        for (uint32_t r = 0; r < batch; r++) {
-            k_peel_filter<<<grid, 256, 0, ctx->stream>>>(g->frontier, g->frontier2, g->removed, g->deg_rem,
-                                                        g->key, ps);
-            k_peel_decrement<<<grid, 256, 0, ctx->stream>>>(g->V, g->E, g->removed, g->deg_rem, g->key, ps);
-            k_peel_advance<<<1, 1, 0, ctx->stream>>>(ps);
-            ctx->launches += 3;
-        }
-        queued += batch;
-        if ((s = gc_check_launch(ctx, "peel round")) != GC_OK) return s;
-        if ((s = gc_check_cuda(ctx, cudaMemcpyAsync(&host, ps, sizeof(host), cudaMemcpyDeviceToHost, ctx->stream),
-                               "peel state")) != GC_OK)
+    {
+        ProfScope prof(ctx, "peel", ctx->stream);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        // every SM; fewer for graphs of less than 256 vertices per CTA (the barriers get cheaper)
+        cfg.gridDim = dim3(std::max<uint32_t>(1u, std::min<uint32_t>((uint32_t)ctx->num_sms, N / 256)));
+        cfg.blockDim = dim3(PEEL_THREADS);
+        cfg.stream = ctx->stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const uint32_t *V = g->V, *E = g->E;
+        if ((s = gc_check_cuda(ctx, cudaLaunchKernelEx(&cfg, k_peel, V, E, N, log_thresholds ? 1 : 0, g->deg_rem,
+                                                       g->frontier, g->frontier2, g->removed, g->key, ps),
+                               "peel")) != GC_OK)
             return s;
-        if ((s = gc_check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "peel rounds")) != GC_OK) return s;
-        if (host.alive == 0) break;
-        if (queued > 2 * (N + 64)) return gc_fail(ctx, GC_ERR_DEVICE, "peeling did not terminate");
-        batch = batch < 256 ? batch * 2 : batch;
+        ctx->launches++;
     }
+    if ((s = gc_check_cuda(ctx, cudaMemcpyAsync(&host, ps, sizeof(host), cudaMemcpyDeviceToHost, ctx->stream),
+                           "peel state")) != GC_OK)
+        return s;
+    if ((s = gc_check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "peel rounds")) != GC_OK) return s;
+    if (host.failed || !host.rounds) return gc_fail(ctx, GC_ERR_DEVICE, "peeling did not terminate");
     return GC_OK;
 }
