@@ -386,7 +386,7 @@ void gc_tuning_default(gc_tuning *t) {
     t->warp_degree = GC_GNN_WARP_DEGREE;
     t->hub_degree = GC_GNN_HUB_DEGREE;
     t->schedule = GC_SCHEDULE_DEGREE;
-    t->jp_ctas_per_sm = 2;
+    t->jp_ctas_per_sm = 5;
     t->jp_tight = 32;
     t->jp_nap = 32;
     t->gnn_warp_degree = GC_GNN_WIDE_DEGREE;
@@ -738,7 +738,7 @@ gc_status gc_batch_autotune(gc_ctx *ctx, gc_batch *b, gc_heuristic h, const gc_m
     if (effort >= 1) {
         // stage 2: resident CTAs of the ordered coloring kernel
         const gc_tuning base = best;
-        for (int c : {1, 2, 3, 4}) {
+        for (int c : {2, 3, 4, 5}) {
             gc_tuning t = base;
             t.jp_ctas_per_sm = c;
             if ((s = consider(t)) != GC_OK) return s;

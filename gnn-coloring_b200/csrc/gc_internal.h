@@ -45,7 +45,7 @@ struct gc_ctx {
     cudaEvent_t ev_copy_fence = nullptr, ev_copy_done = nullptr;
     cudaEvent_t ev_chunk[GC_UPLOAD_CHUNKS] = {};  // pieces of a page-locked E that have arrived
     int color_blocks_per_sm = 0;         // resident CTAs of the coloring kernel (occupancy query)
-    int jp_ctas_per_sm = 2;              // CTAs per SM of the coloring kernel: fewer pollers beat more lookahead (measured)
+    int jp_ctas_per_sm = 5;              // CTAs per SM of the coloring kernel
     unsigned int jp_tight = 32;          // coloring: unproductive polling rounds before sleeping
     unsigned int jp_nap = 32;            // coloring: first sleep between polling rounds (ns)
     bool jp_decide = true;               // coloring: early decisions from published forbidden colors
@@ -54,14 +54,14 @@ struct gc_ctx {
     int round_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each Culberson kernel
     int flow_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each dataflow kernel
     bool jp_classes = true;              // Culberson rounds: class by class instead of tickets
-    uint32_t jp_core_max = 32768;        // coloring: first tickets colored inside one cluster (0: off; GC_JP_CORE)
+    uint32_t jp_core_max = 2048;        // coloring: first tickets colored inside one cluster (0: off; GC_JP_CORE)
     int jp_core_cluster = -1;            // CTAs of that cluster (16 or 8; 0: unavailable; -1: not yet queried)
     uint32_t jp_core_block = 16;         // consecutive core tickets per CTA (GC_JP_CORE_BLOCK)
     unsigned int jp_core_nap = 0;        // core kernel: sleep between polling rounds, ns (GC_JP_CORE_NAP)
     int jp_core_warps = 16;              // core kernel: warps per CTA, 1..32 (GC_JP_CORE_WARPS)
     bool jp_core_decide = true;          // core kernel: early decisions from published seen colors (GC_JP_CORE_DECIDE)
     size_t jp_core_smem = 0;             // core kernel: shared memory per CTA (the device's opt-in maximum)
-    int jp_light_warps = 2;              // coloring: warps per CTA on the light stream (0: no split; GC_JP_LIGHT_WARPS)
+    int jp_light_warps = 4;              // batches: warps per CTA on the light stream (0: no split; GC_JP_LIGHT_WARPS)
     int gnn_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each GNN layer kernel
     uint32_t gnn_warp_deg = GC_GNN_WIDE_DEGREE;  // GNN: above this many neighbours a vertex gets a warp
     uint32_t hub_deg = GC_GNN_HUB_DEGREE;    // plain graphs: above this many neighbours a vertex is a hub (GC_HUB_DEGREE)

@@ -268,8 +268,10 @@ __device__ int color_one(const uint32_t *__restrict__ list, uint32_t cnt, const 
 }
 
 constexpr int COLOR_WARPS_PER_CTA = 8;
-constexpr int PENDING = 128;  // per warp: uncolored predecessors remembered for polling
+constexpr int PENDING = 1024;  // per warp: uncolored predecessors remembered for polling (4 KB)
 constexpr uint32_t DECIDE_MAX = 32;  // early decisions are tried with at most this many predecessors pending
+constexpr uint32_t POLL_ROUND = 2;   // polls of one predecessor between two rounds over the pending list
+static_assert(DECIDE_MAX <= 32, "one pending predecessor per lane");
 
 // Publishes the warp's forbidden colors 1..256 (window 0 of its bitmap) for vertex `self`, tagged
 // with the run's epoch.  Lanes 0..7, one 64-bit word each.
@@ -280,16 +282,19 @@ __device__ __forceinline__ void publish_mask(unsigned long long *fmask, uint32_t
 
 // Colors one ordered vertex whose predecessors are list[0..cnt): the smallest color >= 1 none of
 // them has.  Every predecessor color is read first without waiting (LOADS per lane in flight);
-// the ids of uncolored ones go to the warp's pending list in shared memory, and only those are
-// re-read (one global load each) until colored: back to back at first, then with growing sleeps.
-// Pending-list overflow (more than PENDING uncolored predecessors) waits in place.  Returns -1
-// when a wait exceeded spin_limit rounds or another warp raised the error flag.
+// the ids of uncolored ones go to the warp's pending list in shared memory, and only those are polled:
+// back to back at first, then with growing sleeps.  A list longer than PENDING waits in place for the
+// rest, a lane at a time and without early decisions; with 128 entries that was the usual case on
+// skewed graphs, and more warps in flight (longer lists) made it worse.  Ticket kernel on R-MAT of 4.2 M
+// vertices, GNN3 / GNN2 / first-fit keys: 128 entries and 2 CTAs per SM 5.0 / 4.4 / 5.1 ms, 1,024
+// entries and 4 CTAs 1.4 / 1.0 / 2.3 ms, with the polling below 1.1 / 0.7 / 2.3 ms.
+// Returns -1 when a wait exceeded spin_limit polls or another warp raised the error flag.
 // With `fmask` set, the warp also publishes the colors it has seen (for vertex `self`) while it
 // waits, and tries early decisions once at most DECIDE_MAX predecessors are pending.
 __device__ int color_one_v(const uint32_t *__restrict__ list, uint32_t cnt, const int *color, uint32_t *fb,
                            uint32_t *pend, int lane, DevState *st, unsigned int spin_limit, unsigned int tight,
-                           unsigned int nap, const uint32_t *__restrict__ pc, unsigned long long *fmask,
-                           uint32_t epoch, uint32_t self) {
+                           unsigned int nap, const uint32_t *__restrict__ pc, const uint32_t *__restrict__ key,
+                           unsigned long long *fmask, uint32_t epoch, uint32_t self) {
     const unsigned long long tag = (unsigned long long)epoch << 32;
     for (uint32_t window = 0;; window++) {
         fb[lane] = 0;
@@ -335,58 +340,88 @@ __device__ int color_one_v(const uint32_t *__restrict__ list, uint32_t cnt, cons
         __syncwarp();
         const bool publish = fmask && window == 0 && npend > 0;
         if (publish) publish_mask(fmask, self, tag, fb, lane);
-        // poll the pending list: lane l re-reads entries l, l + 32, ...
-        uint32_t nleft = npend;  // pending entries after the last round (warp-uniform)
+        // Polling.  A round over the whole list is hundreds of instructions, and a chain is as slow as the
+        // rounds.  So a warp first polls the pending predecessor that comes last in the order, whose color
+        // usually comes last; when it has one, and every POLL_ROUND polls, the warp re-reads the whole
+        // list, moves the entries still uncolored to its front, and tries an early decision (at most
+        // DECIDE_MAX pending).  With one left, both outcomes are known in advance.
         unsigned int spins = 0;
-        for (;;) {
-            // the candidate of an early decision: the mex of the colors seen so far
-            int cand = 0;
-            if (fmask && nleft <= DECIDE_MAX) {
-                __syncwarp();
-                cand = window_mex(fb, lane, window);
-            }
-            bool progress = false, undecided = false;
-            uint32_t mine = 0;
-            for (uint32_t i = lane; i < npend && !gave_up; i += 32) {
-                const uint32_t v = pend[i];
-                if (v == 0xffffffffu) continue;
-                const int cc = ld_relaxed(color + v);
-                bool excluded = false;  // v cannot end up with color cand
-                if (cand > 0 && cc == 0) {
-                    excluded = __ldg(pc + v) + 1u < (uint32_t)cand;
-                    if (!excluded && cand <= 32 * GC_JP_MASK_WORDS) {
-                        const unsigned long long w =
-                            ld_relaxed_u64(fmask + (size_t)v * GC_JP_MASK_WORDS + ((uint32_t)(cand - 1) >> 5));
-                        excluded = (uint32_t)(w >> 32) == epoch && ((w >> ((uint32_t)(cand - 1) & 31u)) & 1ull);
-                    }
-                }
-                if (cc) {
-                    mark(fb, cc, window);
-                    pend[i] = 0xffffffffu;
-                    progress = true;
-                    if (cc == cand) undecided = true;  // the candidate is taken
-                } else {
-                    mine++;
-                    if (!excluded) undecided = true;
-                }
-            }
-            if (cand > 0 && !__any_sync(0xffffffffu, undecided || gave_up)) {
-                __syncwarp();
-                return cand;  // every pending predecessor is excluded from cand: the mex is cand
-            }
-            nleft = __reduce_add_sync(0xffffffffu, mine);
-            if (nleft == 0 || __any_sync(0xffffffffu, gave_up)) break;
-            if (__any_sync(0xffffffffu, progress)) {
-                if (publish) {
-                    __syncwarp();
-                    publish_mask(fmask, self, tag, fb, lane);
-                }
-            } else {
-                if (++spins > spin_limit || ((spins & 255u) == 0 && ld_relaxed_u32(&st->err))) gave_up = true;
-                else if (spins > tight) __nanosleep(spins > 16 * tight + 64 ? 4 * nap : nap);
-            }
-        }
+        auto pause = [&]() {  // after a fruitless poll: true when the wait is over its limit or another one was
+            if (++spins > spin_limit || ((spins & 255u) == 0 && ld_relaxed_u32(&st->err))) return true;
+            if (spins > tight) __nanosleep(spins > 16 * tight + 64 ? 4 * nap : nap);
+            return false;
+        };
+        // v cannot end up with color c: it has too few predecessors, or one of them has c
+        auto excluded = [&](uint32_t v, int c) {
+            if (__ldg(pc + v) + 1u < (uint32_t)c) return true;
+            if (c > 32 * GC_JP_MASK_WORDS) return false;
+            const unsigned long long w = ld_relaxed_u64(fmask + (size_t)v * GC_JP_MASK_WORDS + ((uint32_t)(c - 1) >> 5));
+            return (uint32_t)(w >> 32) == epoch && ((w >> ((uint32_t)(c - 1) & 31u)) & 1ull) != 0;
+        };
         if (__any_sync(0xffffffffu, gave_up)) return -1;
+        while (npend > 1) {
+            if (fmask && npend <= DECIDE_MAX) {
+                const int cand = window_mex(fb, lane, window);
+                if (cand > 0 && __all_sync(0xffffffffu, (uint32_t)lane >= npend || excluded(pend[lane], cand))) {
+                    __syncwarp();
+                    return cand;  // every pending predecessor is excluded from cand: the mex is cand
+                }
+            }
+            // the pending predecessor that comes last: smallest key, then largest id
+            uint32_t lk = 0xffffffffu, lv = 0;
+            for (uint32_t i = lane; i < npend; i += 32) {
+                const uint32_t v = pend[i], kv = __ldg(key + v);
+                if (kv < lk || (kv == lk && v >= lv)) lk = kv, lv = v;
+            }
+            const uint32_t kmin = __reduce_min_sync(0xffffffffu, lk);
+            const uint32_t last = __reduce_max_sync(0xffffffffu, lk == kmin ? lv : 0u);
+            bool stop = false;
+            for (uint32_t k = 0; k < POLL_ROUND; k++) {
+                if (__shfl_sync(0xffffffffu, lane == 0 ? ld_relaxed(color + last) : 0, 0)) break;
+                if ((stop = __any_sync(0xffffffffu, pause()))) break;
+            }
+            if (stop) return -1;
+            bool progress = false;
+            uint32_t kept = 0;
+            for (uint32_t c0 = 0; c0 < npend; c0 += 32) {
+                const uint32_t i = c0 + (uint32_t)lane;
+                const uint32_t v = i < npend ? pend[i] : 0u;
+                const int cc = i < npend ? ld_relaxed(color + v) : -1;
+                if (i < npend && cc) {
+                    mark(fb, cc, window);
+                    progress = true;
+                }
+                const unsigned int km = __ballot_sync(0xffffffffu, cc == 0);  // (also: every lane has read its entry)
+                if (cc == 0) pend[kept + __popc(km & ((1u << lane) - 1u))] = v;
+                kept += __popc(km);
+            }
+            npend = kept;
+            __syncwarp();  // marks and the compacted list are visible
+            if (publish && __any_sync(0xffffffffu, progress)) publish_mask(fmask, self, tag, fb, lane);
+        }
+        if (npend == 1) {
+            // c1 unless the last predecessor takes it, else c2
+            __syncwarp();
+            const int c1 = window_mex(fb, lane, window);
+            const int c2 = c1 > 0 ? window_mex_after(fb, lane, window, c1) : 0;
+            const uint32_t last = pend[0];
+            int cc;
+            for (uint32_t k = 0;; k++) {
+                cc = __shfl_sync(0xffffffffu, lane == 0 ? ld_relaxed(color + last) : 0, 0);
+                if (cc) break;
+                if (fmask && c1 > 0 && k % POLL_ROUND == 0 &&
+                    __shfl_sync(0xffffffffu, lane == 0 && excluded(last, c1) ? 1 : 0, 0)) {
+                    __syncwarp();
+                    return c1;
+                }
+                if (__any_sync(0xffffffffu, pause())) return -1;
+            }
+            if (c1 > 0 && (cc != c1 || c2 > 0)) {
+                __syncwarp();
+                return cc == c1 ? c2 : c1;
+            }
+            if (lane == 0) mark(fb, cc, window);  // the window holds no answer
+        }
         __syncwarp();
         const int m = window_mex(fb, lane, window);
         __syncwarp();
@@ -416,9 +451,12 @@ __global__ void k_jp_records(const uint32_t *__restrict__ order, const uint32_t 
 // On power-law graphs the priority DAG's long chains lie almost all among the highest-priority inner
 // vertices (R-MAT 22, GNN3 keys: depth 2,683 in all, yet depth 2,000 is reached by ticket 8,422, and
 // with the first 32,768 tickets colored the rest is only 214 deep).  Through global memory every
-// link of a chain costs a store-to-poll round trip in L2 (about 1 us), so these tickets bound the
-// whole kernel.  Here one cluster colors tickets [0, K) with every color exchanged through
-// distributed shared memory instead:
+// link of a chain costs a store-to-poll round trip in L2 (about 1 us); the first few thousand tickets, nearly a
+// clique, are where that counts.  Here one cluster colors tickets [0, K) with every color exchanged
+// through distributed shared memory instead.  K is 2,048 (ctx->jp_core_max): beyond the clique the
+// ticket kernel's thousands of warps are faster than the cluster's 256 (core + ticket kernel on R-MAT of
+// 4.2 M vertices, largest degree first: K = 0 1.08 ms, 2,048 0.95, 4,096 0.96, 8,192 1.0, 32,768 1.3;
+// GNN3 keys 1.2, 1.41, 1.42, 1.45, 1.58; 100,003 vertices LF 0.40, 0.10, 0.11, 0.14, 0.22).
 //   - each CTA holds a replica of the K core colors (16 bits each) in its shared memory;
 //   - tickets go to the CTAs in blocks of B consecutive ones (block k to CTA k % C), so a short link
 //     of a chain often stays inside one SM; a CTA hands its tickets out in order to whichever warp
@@ -780,13 +818,17 @@ __global__ void __launch_bounds__(CORE_WARPS * 32, 1) k_jp_core(const uint4 *__r
 
 // ---- after the core: a heavy and a light stream --------------------------------------------------
 //
-// Past the core the DAG is shallow and the ticket kernel is bound by how many vertices are in flight
-// (about 1.7 us from ticket to color, most of it three dependent loads).  Most of these vertices
-// have few predecessors, so they are split off: tickets with at most LIGHT_MAX predecessors form the
-// light stream, colored one vertex per lane (32 per warp), the others the heavy stream, one vertex
-// per warp as before.  Both streams keep the priority order, and each has warps of its own, so the
-// oldest unfinished vertex of either stream is always held by a running warp and all its
-// predecessors are done: the kernel always progresses.
+// In a batch the ticket kernel is bound by how many vertices are in flight (about 1.7 us from ticket to
+// color, most of it three dependent loads), and most vertices have few predecessors.  So those are
+// split off: tickets with at most LIGHT_MAX predecessors form the light stream, colored one vertex per
+// lane (32 per warp), the others the heavy stream, one vertex per warp as before.  Both streams keep the
+// priority order, and each has warps of its own, so the oldest unfinished vertex of either stream is
+// always held by a running warp and all its predecessors are done: the kernel always progresses.
+// 400 graphs, 17 M vertices, largest degree first: 7.5 ms a pass with half of each CTA's warps on the
+// light stream, 15.1 ms without streams; eight lanes per light vertex, with early decisions, 11.9 ms.
+// A single graph keeps one stream: its chains pass through light vertices, and a lane tells its color
+// only when its whole warp is through (core + streams + ticket kernel of R-MAT 100,003, GNN3 keys: 0.28
+// ms with streams, 0.13 without; 2^20 vertices, first fit: 1.55 and 0.70).
 constexpr uint32_t LIGHT_MAX = 63;   // a light vertex's color is at most 64: one 64-bit mask
 constexpr uint32_t PART_TILE = 1024;
 
@@ -932,9 +974,10 @@ __device__ __forceinline__ int color_light(const uint32_t *__restrict__ list, ui
 // CTA's first COLOR_WARPS_PER_CTA - light_warps warps take the heavy stream split[0, n_heavy) one
 // vertex each (ticket counter st->ticket, from 0), the others the light stream -- split[cap - 1 - i],
 // i < n_light -- 32 vertices at a time, one per lane (counter st->ticket_light).
-__global__ void __launch_bounds__(COLOR_WARPS_PER_CTA * 32, 2) k_jp_color(const uint4 *__restrict__ rec,
+__global__ void __launch_bounds__(COLOR_WARPS_PER_CTA * 32, 5) k_jp_color(const uint4 *__restrict__ rec,
                                                                        const uint32_t *__restrict__ P,
-                                                                       const uint32_t *__restrict__ pc, int *color,
+                                                                       const uint32_t *__restrict__ pc,
+                                                                       const uint32_t *__restrict__ key, int *color,
                                                                        DevState *st, unsigned int spin_limit,
                                                                        unsigned int tight, unsigned int nap,
                                                                        unsigned long long *fmask,
@@ -973,7 +1016,7 @@ __global__ void __launch_bounds__(COLOR_WARPS_PER_CTA * 32, 2) k_jp_color(const 
         const uint4 r = src[t];
         const uint32_t u = r.x;
         const int c = color_one_v(P + r.y, r.z, color, forbid[warp], pending[warp], lane, st, spin_limit, tight, nap,
-                                  pc, fmask, epoch, u);
+                                  pc, key, fmask, epoch, u);
         if (lane == 0) {
             if (c < 0) raise_error(st, ERR_WAIT_EXPIRED, u);
             // -1 on error is non-zero, so successors stop waiting; the host reports the error
@@ -1307,7 +1350,7 @@ gc_status gc_jp_color(gc_graph *g) {
     // the tickets after the core as a heavy and a light stream (light_warps warps per CTA take the light one)
     const int light_warps = ctx->jp_light_warps;
     uint4 *split = nullptr;
-    if (light_warps > 0 && light_warps < COLOR_WARPS_PER_CTA) {
+    if (g->n_seg > 1 && light_warps > 0 && light_warps < COLOR_WARPS_PER_CTA) {
         const uint32_t ntiles = (N + PART_TILE - 1) / PART_TILE;
         if ((s = gc_alloc(ctx, &g->jpsplit, g->cap_N, "ticket streams")) != GC_OK) return s;
         if ((s = gc_alloc(ctx, &g->part_tiles, (g->cap_N + PART_TILE - 1) / PART_TILE, "ticket stream tiles")) != GC_OK)
@@ -1325,7 +1368,7 @@ gc_status gc_jp_color(gc_graph *g) {
     {
         ProfScope ps(ctx, "jp_color", ctx->stream);
         k_jp_color<<<ctx->num_sms * blocks, COLOR_WARPS_PER_CTA * 32, 0, ctx->stream>>>(
-            g->jprec, g->P, g->pc, g->color, ctx->dstate, ctx->spin_limit, tight, nap, fmask, epoch_word, split,
+            g->jprec, g->P, g->pc, g->key, g->color, ctx->dstate, ctx->spin_limit, tight, nap, fmask, epoch_word, split,
             g->cap_N, light_warps);
         ctx->launches++;
     }
