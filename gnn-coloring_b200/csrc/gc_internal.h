@@ -30,7 +30,11 @@ constexpr uint32_t GC_GNN_WARP_DEGREE = 256;
 // The GNN layers' own warp tier (degree schedule): a warp stages 32 rows through shared memory, which
 // costs about 2.5 L1 wavefronts per row against 1 for the four-lane tier, so only vertices whose lists
 // are long enough to need a warp's latency hiding get one (the split kernel keeps GC_GNN_WARP_DEGREE).
+// This and GC_GNN_HUB_DEGREE are the values of large graphs; smaller ones take lower ones (auto_degree).
 constexpr uint32_t GC_GNN_WIDE_DEGREE = 4096;
+// Up to this many neighbours the GNN takes 32 vertices per warp (R-MAT, layers of 1 M vertices: 429 us with 16,
+// 455 with 8, 462 with 32).
+constexpr uint32_t GC_GNN_THIN_DEGREE = 16;
 
 struct gc_ctx {
     int device = 0;
@@ -65,7 +69,7 @@ struct gc_ctx {
     int gnn_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each GNN layer kernel
     uint32_t gnn_warp_deg = GC_GNN_WIDE_DEGREE;  // GNN: above this many neighbours a vertex gets a warp
     uint32_t hub_deg = GC_GNN_HUB_DEGREE;    // plain graphs: above this many neighbours a vertex is a hub (GC_HUB_DEGREE)
-    uint32_t gnn_thin_deg = 16;          // GNN: vertices with at most this many neighbours get one lane each
+    uint32_t gnn_thin_deg = GC_GNN_THIN_DEGREE;  // GNN: vertices with at most this many neighbours go 32 per warp
     bool gnn_fuse_isolated = true;       // GNN: vertices without neighbours run all layers at once (GC_GNN_FUSE_ISOLATED)
     uint32_t gnn_grab = 2;               // GNN counter hand-out: items per grab (GC_GNN_GRAB; 1-2 best, 8 +4 %, 16 +17 %)
     uint32_t gnn_heavy = 16384;          // GNN counter hand-out: leading four-lane items taken singly (GC_GNN_HEAVY)
@@ -92,7 +96,7 @@ struct ProfScope {
     ~ProfScope();
 };
 
-// Hubs (more than GC_GNN_HUB_DEGREE neighbours) are split across several warps in the JP split
+// Hubs (more than GC_GNN_HUB_DEGREE neighbours, fewer in small graphs) are split across several warps in the JP split
 // pass, this many edges per warp task.
 constexpr uint32_t GC_SPLIT_CHUNK = 1024;  // edges per warp task (shared-memory buffer per warp)
 constexpr int GC_JP_MASK_WORDS = 8;        // published forbidden colors: 8 x 32 = colors 1..256
@@ -133,8 +137,9 @@ struct gc_graph {
     uint32_t *big = nullptr;         // split tasks of the hubs: (vertex, first edge) pairs
     uint32_t n_big_tasks = 0;
     size_t big_cap = 0;              // words allocated for `big`
-    uint32_t *hubs = nullptr;        // vertices with deg > GC_GNN_HUB_DEGREE, by descending degree
+    uint32_t *hubs = nullptr;        // the hubs; by descending degree once hubs_sorted
     uint32_t n_hubs = 0;
+    bool hubs_sorted = false;        // the hub list is in order and n_giant, giant_off describe it (gc_sort_hubs)
     uint32_t *hub_aux = nullptr;     // GNN: per hub 16 feature sums, then one completion counter each
     size_t hub_aux_cap = 0;
     uint32_t n_giant = 0;            // the leading hubs whose rows the GNN stages (see k_hub_stage)
@@ -148,7 +153,7 @@ struct gc_graph {
     uint32_t n_wide = 0;             // leading vorder entries with more than GC_GNN_WARP_DEGREE neighbours
     uint32_t n_wide_gnn = 0;         // leading vorder entries the GNN gives a warp (more than gnn_warp_deg)
     uint32_t gnn_warp_deg = GC_GNN_WIDE_DEGREE;
-    uint32_t n_thin = 0;             // trailing vorder entries with at most ctx->gnn_thin_deg neighbours
+    uint32_t n_thin = 0;             // trailing vorder entries that k_gnn_thin takes
     uint32_t n_iso = 0;              // of those, the trailing entries without neighbours (degree schedule only)
                                      // (degree schedule only; 0 with the graph-major schedule)
     // GNN scratch (allocated on first use).  Feature rows (x, y, t01) are stored in degree order:
@@ -230,6 +235,7 @@ inline void gc_dev_free(gc_ctx *ctx, void *p) {
 
 // ---- kernel drivers ----
 gc_status gc_graph_prepare(gc_graph *g);  // degree classes, max degree (k_graph.cu)
+gc_status gc_sort_hubs(gc_graph *g);      // the hub list by descending degree, and its giants: once per upload
 gc_status gc_priority_simple(gc_graph *g, gc_heuristic h);         // FF / LF / LLF (k_priority.cu)
 gc_status gc_priority_peel(gc_graph *g, bool log_thresholds);      // SL / SLL (k_priority.cu)
 gc_status gc_priority_gnn(gc_graph *g, const gc_model *m);         // GraphSAGE (k_gnn.cu)

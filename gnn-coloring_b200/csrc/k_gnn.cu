@@ -13,12 +13,13 @@
 //   ((t0+t1)+(t2+t3)) + ((t4+t5)+(t6+t7))                                  (dense_kernel_output)
 // and the key is that float's bit pattern (the sum is >= +0, so bit order = value order).
 //
-// Mapping, by degree (the degree order built at upload):
-//   - thin tier (at most 16 neighbours): one vertex per lane;
+// Mapping, by degree (the degree order built at upload; gc_graph_prepare sets the tiers' ends):
+//   - thin tier (at most GC_GNN_THIN_DEGREE neighbours): 32 vertices per warp, their rows gathered by
+//     quads, their dense parts one per lane;
 //   - quad tier: four lanes per vertex, a float4 of the row each, eight vertices per warp;
-//   - warp tier (more than GC_GNN_WIDE_DEGREE neighbours): a warp per vertex, rows staged in
-//     shared memory;
-//   - hubs (more than GC_GNN_HUB_DEGREE): a persistent kernel on a high-priority side stream; one
+//   - warp tier (more than 512 to GC_GNN_WIDE_DEGREE neighbours, by the graph's size): a warp per vertex,
+//     rows staged in shared memory;
+//   - hubs (more than 2,048 to GC_GNN_HUB_DEGREE, by the graph's size): a persistent kernel on a high-priority side stream; one
 //     item per hub gathers its neighbour rows into shared memory, 512 or 1,024 at a time, and one
 //     warp per feature evaluates the reference's sequential FP32 chain exactly, a step at a time
 //     (exact_step below); the rows of the largest hubs are staged feature-major by the whole GPU
@@ -443,63 +444,102 @@ __global__ void __launch_bounds__(ISO_THREADS) k_gnn_isolated(const uint32_t *__
     }
 }
 
-// ---- thin tier: one vertex per lane --------------------------------------------------------------
-
-// Vertices with at most ctx->gnn_thin_deg neighbours (the tail of the degree order, vorder[first,
-// n_vorder)): one per lane, 32 per warp, whose degrees are nearly equal because the order is sorted.
-// E holds the neighbours' feature rows; vorder[i]'s own row is row0 + i.
-// Each lane adds its vertex's neighbour rows in CSR order (the next row's loads in flight while the
-// current one is added; the 16 feature chains interleave) and runs the 32 x 16 dense part alone:
-// no lane sits idle on a short neighbour list, and no shuffles are needed.
+// ---- thin tier: 32 vertices per warp ---------------------------------------------------------------
+//
+// Vertices with few neighbours (the tail of the degree order, vorder[first, n_vorder)): 32 per warp, whose
+// degrees are nearly equal because the order is sorted.  E holds the neighbours' feature rows;
+// vorder[i]'s own row is row0 + i.
+//   - Neighbour sums by quads, as in the layer kernel: four lanes read a 64-byte row together (one L1
+//     wavefront; one vertex per lane took four), eight vertices at a time, eight rows each in flight.
+//     In the input layer the quads read the rows' float2 into shared memory, and each lane adds its own
+//     vertex's values in order.
+//   - The sums go through a 2 KB slab per warp, and each lane then runs the 32 x 16 dense part of its own
+//     vertex alone: no shuffles, and the weights are a kernel parameter.  Every lane reads the same
+//     weight at the same time, with compile-time indices, so each one is a constant-bank operand of
+//     its FMA; in shared memory each 16-byte weight load of the quads took four wavefronts, half of all
+//     that the layer kernel spent on a mesh (256^3 stencil: 24 of 48 per vertex, at 94 % of the pipe).
+//   - Own rows and outputs pass the slab as well, so that quads read and write them whole.
+// 3 layers over the 256^3 stencil 7,935 -> 5,500 us, Erdos-Renyi of 400,000 vertices 297 -> 186, random geometric
+// of 1 M 563 -> 368; of 8 M 5,273 -> 4,910 (its rows come from DRAM).
+// Slab layout: row v's 16-byte chunk c at chunk c ^ ((v >> 1) & 3) of its 64 bytes, which keeps both the
+// quads' and the lanes' accesses free of bank conflicts.
 constexpr int THIN_THREADS = 256;
+constexpr int THIN_CHUNK = 16;  // input layer: neighbours staged per vertex and step
 
-// One layer's 32 x 16 weights and 16 biases as a kernel parameter.  Every lane of the thin tier reads
-// the same weight at the same time, with compile-time indices, so each one is a constant-bank
-// operand of its FMA: no load through the L1 data pipe, which bounds this kernel (weights in shared
-// memory cost it 15 M of 53 M wavefronts per hidden layer on R-MAT 22).
 struct LayerArg {
     float w[LAYER_PARAMS];
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(THIN_THREADS, 3) k_gnn_thin(const uint2 *__restrict__ vrow, const uint32_t *__restrict__ E,
+__global__ void __launch_bounds__(THIN_THREADS, 4) k_gnn_thin(const uint2 *__restrict__ vrow, const uint32_t *__restrict__ E,
                                                               const uint32_t *__restrict__ vorder, uint32_t row0, uint32_t first,
                                                               uint32_t n_vorder, const float2 *__restrict__ t01,
                                                               const float *__restrict__ x, float *__restrict__ y,
                                                               uint32_t *__restrict__ key, const __grid_constant__ LayerArg P,
                                                               uint32_t *work_ctr, uint32_t grab) {
+    constexpr int SLAB = MODE == MODE_INPUT ? 32 * THIN_CHUNK * 2 : 32 * FEAT;  // floats per warp
+    __shared__ __align__(16) float slabs[THIN_THREADS / 32][SLAB];
     const float *W = P.w;  // row i of the weights: W[16 i .. 16 i + 15], biases W[512 ..]
     const float4 *X4 = reinterpret_cast<const float4 *>(x);
-    const int lane = threadIdx.x & 31;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    auto group = [&](uint32_t base) {  // the 32 vertices vorder[base, base + 32), one per lane
-        const uint32_t slot = base + lane;
+    const int lane = threadIdx.x & 31, q = lane & 3, qbase = lane & ~3;
+    float *slab = slabs[threadIdx.x >> 5];
+    float4 *slab4 = reinterpret_cast<float4 *>(slab);
+    const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto chunk = [](uint32_t v, uint32_t c) { return v * 4 + (c ^ ((v >> 1) & 3u)); };
+    const uint32_t n_groups = (n_vorder - first + 31) / 32;
+    uint32_t gi = 0, gend = 0;
+    for (;;) {
+        if (gi == gend) {
+            gi = grab_work(work_ctr, grab, lane);
+            if (gi >= n_groups) return;
+            gend = min(gi + grab, n_groups);
+        }
+        const uint32_t base = first + 32 * gi++;
+        const uint32_t slot = base + lane;  // this lane's vertex
         const bool valid = slot < n_vorder;
-        const uint32_t u = valid && MODE == MODE_OUTPUT ? vorder[slot] : 0u;  // the vertex (for its key)
-        const uint32_t r = row0 + slot;                                       // its feature row
-        const uint2 bd = valid ? vrow[r] : make_uint2(0u, 0u);
-        const uint32_t beg = bd.x, d = bd.y;
-        const uint32_t dmax = __reduce_max_sync(FULL, d);
-        const float fd = __uint2float_rn(d);
+        const uint2 bd = valid ? vrow[row0 + slot] : make_uint2(0u, 0u);
+        const float fd = __uint2float_rn(bd.y);
         float c[FEAT];
-#pragma unroll
-        for (int j = 0; j < FEAT; j++) c[j] = W[2 * FEAT * FEAT + j];
         if (MODE == MODE_INPUT) {
+            const uint32_t dmax = __reduce_max_sync(FULL, bd.y);
+            float2 *pairs = reinterpret_cast<float2 *>(slab);  // value k of vertex v at 32 k + (v ^ 8 (k & 3))
             float s0 = 0.0f, s1 = 0.0f;
-            float2 tn = d ? __ldg(t01 + __ldg(E + beg)) : make_float2(0.0f, 0.0f);
-            for (uint32_t k = 0; k < dmax; k++) {
-                const float2 t = tn;
-                if (k + 1 < d) tn = __ldg(t01 + __ldg(E + beg + k + 1));
-                if (k < d) {
-                    s0 = __fadd_rn(s0, t.x);
-                    s1 = __fadd_rn(s1, t.y);
+            for (uint32_t c0 = 0; c0 < dmax; c0 += THIN_CHUNK) {
+                uint32_t id[4][4];
+                uint32_t dq[4];
+#pragma unroll
+                for (int sub = 0; sub < 4; sub++) {
+                    const uint32_t beg = __shfl_sync(FULL, bd.x, 8 * sub + (lane >> 2)) + c0;
+                    const uint32_t d = __shfl_sync(FULL, bd.y, 8 * sub + (lane >> 2));
+                    dq[sub] = d > c0 ? d - c0 : 0u;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) id[sub][i] = 4u * i + q < dq[sub] ? ld_stream(E + beg + 4 * i + q) : 0u;
                 }
+#pragma unroll
+                for (int sub = 0; sub < 4; sub++) {
+                    const uint32_t v = 8u * sub + (lane >> 2);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (4u * i + q < dq[sub]) pairs[32 * (4 * i + q) + (v ^ (8u * q))] = __ldg(t01 + id[sub][i]);
+                }
+                __syncwarp();
+                const uint32_t n = min((uint32_t)THIN_CHUNK, bd.y > c0 ? bd.y - c0 : 0u);
+#pragma unroll
+                for (int k = 0; k < THIN_CHUNK; k++)
+                    if ((uint32_t)k < n) {
+                        const float2 t = pairs[32 * k + ((uint32_t)lane ^ (8u * (k & 3)))];
+                        s0 = __fadd_rn(s0, t.x);
+                        s1 = __fadd_rn(s1, t.y);
+                    }
+                __syncwarp();
             }
             if (fd > 0.0f) {
                 s0 = __fdiv_rn(s0, fd);
                 s1 = __fdiv_rn(s1, fd);
             }
-            const float2 self = valid ? t01[r] : make_float2(0.0f, 0.0f);
+            const float2 self = valid ? t01[row0 + slot] : make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int j = 0; j < FEAT; j++) c[j] = W[2 * FEAT * FEAT + j];
 #pragma unroll
             for (int i = 0; i < 32; i++) {
                 const float a = i < 8 ? s0 : (i < 16 ? s1 : (i < 24 ? self.x : self.y));
@@ -507,60 +547,66 @@ __global__ void __launch_bounds__(THIN_THREADS, 3) k_gnn_thin(const uint2 *__res
                 for (int j = 0; j < FEAT; j++) c[j] = __fmaf_rn(W[i * FEAT + j], a, c[j]);
             }
         } else {
-            float acc[FEAT];
+#pragma unroll 1
+            for (int sub = 0; sub < 4; sub++) {
+                const uint32_t v = 8u * sub + (lane >> 2);
+                const uint32_t beg = __shfl_sync(FULL, bd.x, (int)v), d = __shfl_sync(FULL, bd.y, (int)v);
+                const uint32_t dmax = __reduce_max_sync(FULL, d);
+                float4 s = zero4;
+                // neighbour ids one step ahead, so the row loads never wait for them
+                uint32_t n0 = q < d ? ld_stream(E + beg + q) : 0u;
+                uint32_t n1 = 4 + q < d ? ld_stream(E + beg + 4 + q) : 0u;
+                for (uint32_t c0 = 0; c0 < dmax; c0 += 8) {
+                    const uint32_t e0 = n0, e1 = n1;
+                    n0 = c0 + 8 + q < d ? ld_stream(E + beg + c0 + 8 + q) : 0u;
+                    n1 = c0 + 12 + q < d ? ld_stream(E + beg + c0 + 12 + q) : 0u;
+                    float4 r[8];
 #pragma unroll
-            for (int f = 0; f < FEAT; f++) acc[f] = 0.0f;
-            // ids two ahead, rows one ahead
-            uint32_t vnext = d > 1 ? __ldg(E + beg + 1) : 0u;
-            float4 rn[4];
-            {
-                const uint32_t v0 = d ? __ldg(E + beg) : 0u;
-#pragma unroll
-                for (int p = 0; p < 4; p++) rn[p] = d ? __ldg(X4 + (size_t)v0 * 4 + p) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-            for (uint32_t k = 0; k < dmax; k++) {
-                float4 r[4];
-#pragma unroll
-                for (int p = 0; p < 4; p++) r[p] = rn[p];
-                if (k + 1 < d) {
-                    const uint32_t v = vnext;
-                    vnext = k + 2 < d ? __ldg(E + beg + k + 2) : 0u;
-#pragma unroll
-                    for (int p = 0; p < 4; p++) rn[p] = __ldg(X4 + (size_t)v * 4 + p);
-                }
-                if (k < d) {
-#pragma unroll
-                    for (int p = 0; p < 4; p++) {
-                        acc[4 * p + 0] = __fadd_rn(acc[4 * p + 0], r[p].x);
-                        acc[4 * p + 1] = __fadd_rn(acc[4 * p + 1], r[p].y);
-                        acc[4 * p + 2] = __fadd_rn(acc[4 * p + 2], r[p].z);
-                        acc[4 * p + 3] = __fadd_rn(acc[4 * p + 3], r[p].w);
+                    for (int k = 0; k < 8; k++) {
+                        const uint32_t e = __shfl_sync(FULL, k < 4 ? e0 : e1, qbase + (k & 3));
+                        r[k] = c0 + k < d ? __ldg(X4 + (size_t)e * 4 + q) : zero4;
                     }
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        if (c0 + k < d) s = add4(s, r[k]);
                 }
+                slab4[chunk(v, q)] = s;
             }
-            if (fd > 0.0f) {
+            __syncwarp();
 #pragma unroll
-                for (int f = 0; f < FEAT; f++) acc[f] = __fdiv_rn(acc[f], fd);
-            }
-            float self[FEAT];
-#pragma unroll
-            for (int p = 0; p < 4; p++) {
-                const float4 s4 = valid ? __ldg(X4 + (size_t)r * 4 + p) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                self[4 * p + 0] = s4.x;
-                self[4 * p + 1] = s4.y;
-                self[4 * p + 2] = s4.z;
-                self[4 * p + 3] = s4.w;
-            }
-#pragma unroll
-            for (int i = 0; i < 32; i++) {
-                const float a = i < FEAT ? acc[i] : self[i - FEAT];
+            for (int j = 0; j < FEAT; j++) c[j] = W[2 * FEAT * FEAT + j];
+            auto dense = [&](int i, float a) {
 #pragma unroll
                 for (int j = 0; j < FEAT; j++) c[j] = __fmaf_rn(W[i * FEAT + j], a, c[j]);
+            };
+#pragma unroll
+            for (int p = 0; p < 4; p++) {  // the mean
+                float4 a = slab4[chunk(lane, p)];
+                if (fd > 0.0f) a = make_float4(__fdiv_rn(a.x, fd), __fdiv_rn(a.y, fd), __fdiv_rn(a.z, fd), __fdiv_rn(a.w, fd));
+                dense(4 * p + 0, a.x);
+                dense(4 * p + 1, a.y);
+                dense(4 * p + 2, a.z);
+                dense(4 * p + 3, a.w);
             }
+            __syncwarp();
+#pragma unroll
+            for (int sub = 0; sub < 4; sub++) {  // own rows, whole
+                const uint32_t v = 8u * sub + (lane >> 2);
+                slab4[chunk(v, q)] = base + v < n_vorder ? __ldg(X4 + (size_t)(row0 + base + v) * 4 + q) : zero4;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                const float4 a = slab4[chunk(lane, p)];
+                dense(FEAT + 4 * p + 0, a.x);
+                dense(FEAT + 4 * p + 1, a.y);
+                dense(FEAT + 4 * p + 2, a.z);
+                dense(FEAT + 4 * p + 3, a.w);
+            }
+            __syncwarp();
         }
 #pragma unroll
         for (int j = 0; j < FEAT; j++) c[j] = relu(c[j]);
-        if (!valid) return;
         if (MODE == MODE_OUTPUT) {
             // t_k = o_k + o_{k+8}, then ((t0+t1)+(t2+t3)) + ((t4+t5)+(t6+t7))  (dense_kernel_output)
             float t[8];
@@ -568,30 +614,18 @@ __global__ void __launch_bounds__(THIN_THREADS, 3) k_gnn_thin(const uint2 *__res
             for (int k = 0; k < 8; k++) t[k] = __fadd_rn(c[k], c[k + 8]);
             const float sum = __fadd_rn(__fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3])),
                                         __fadd_rn(__fadd_rn(t[4], t[5]), __fadd_rn(t[6], t[7])));
-            key[u] = __float_as_uint(sum);
+            if (valid) key[vorder[slot]] = __float_as_uint(sum);
         } else {
-            float4 *Y4 = reinterpret_cast<float4 *>(y) + (size_t)r * 4;
 #pragma unroll
-            for (int p = 0; p < 4; p++) Y4[p] = make_float4(c[4 * p], c[4 * p + 1], c[4 * p + 2], c[4 * p + 3]);
-        }
-    };
-    // one call site, so the group body is inlined once
-    const uint32_t n_groups = (n_vorder - first + 31) / 32;
-    uint32_t base = first + blockIdx.x * blockDim.x + (threadIdx.x & ~31u), gi = 0, gend = 0;
-    for (;;) {
-        if (work_ctr) {
-            if (gi == gend) {
-                gi = grab_work(work_ctr, grab, lane);
-                if (gi >= n_groups) break;
-                gend = min(gi + grab, n_groups);
+            for (int p = 0; p < 4; p++) slab4[chunk(lane, p)] = make_float4(c[4 * p], c[4 * p + 1], c[4 * p + 2], c[4 * p + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int sub = 0; sub < 4; sub++) {
+                const uint32_t v = 8u * sub + (lane >> 2);
+                if (base + v < n_vorder) reinterpret_cast<float4 *>(y)[(size_t)(row0 + base + v) * 4 + q] = slab4[chunk(v, q)];
             }
-            base = first + gi * 32;
-            gi++;
-        } else if (base >= n_vorder) {
-            break;
+            __syncwarp();
         }
-        group(base);
-        if (!work_ctr) base += stride;
     }
 }
 
@@ -1284,7 +1318,7 @@ gc_status launch_layer(gc_graph *g, const float *Wb, const float *Wh, const floa
         }
         const uint32_t end_thin = g->n_vorder - n_iso;
         if (end_thin > first_thin) {
-            const uint32_t grid = std::min<uint32_t>((uint32_t)ctx->num_sms * 3,
+            const uint32_t grid = std::min<uint32_t>((uint32_t)ctx->num_sms * 4,
                                                      (end_thin - first_thin + THIN_THREADS - 1) / THIN_THREADS);
             LayerArg la;
             memcpy(la.w, Wh, sizeof(la.w));
@@ -1312,6 +1346,7 @@ gc_status gc_gnn_rows_begin(gc_graph *g) {
     if ((s = gc_alloc(ctx, &g->Er, (size_t)g->cap_M, "neighbour rows")) != GC_OK) return s;
     if ((s = gc_alloc(ctx, &g->vrow, rows, "row offsets")) != GC_OK) return s;
     if (g->N == 0) return GC_OK;
+    if ((s = gc_sort_hubs(g)) != GC_OK) return s;  // hub h takes row h
     k_gnn_rows<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(g->V, g->hubs, g->n_hubs, g->vorder, g->n_vorder, g->row_of,
                                                            g->vrow);
     ctx->launches++;
@@ -1332,6 +1367,7 @@ gc_status gc_priority_gnn(gc_graph *g, const gc_model *m) {
     gc_status s;
     if (!m || m->layers < 2) return gc_fail(ctx, GC_ERR_INVALID, "GNN needs a model with at least 2 layers");
     if (g->N == 0) return GC_OK;
+    if ((s = gc_sort_hubs(g)) != GC_OK) return s;
     const size_t rows = (size_t)g->cap_N;
     if ((s = gc_alloc(ctx, &g->x, rows * FEAT, "gnn features")) != GC_OK) return s;
     if ((s = gc_alloc(ctx, &g->y, rows * FEAT, "gnn features")) != GC_OK) return s;
