@@ -829,6 +829,9 @@ __global__ void __launch_bounds__(CORE_WARPS * 32, 1) k_jp_core(const uint4 *__r
 // A single graph keeps one stream: its chains pass through light vertices, and a lane tells its color
 // only when its whole warp is through (core + streams + ticket kernel of R-MAT 100,003, GNN3 keys: 0.28
 // ms with streams, 0.13 without; 2^20 vertices, first fit: 1.55 and 0.70).
+// So does a batch of up to jp_light_min vertices, few of which wait for a warp (passes with / without: 4 graphs,
+// 20,000 vertices, largest degree first 196 / 156 us; 8 of 418,000, first fit 1,042 / 486; 96 of 622,000, 715
+// / 991; 64 of 2.2 M, largest degree first 1,121 / 1,527).
 constexpr uint32_t LIGHT_MAX = 63;   // a light vertex's color is at most 64: one 64-bit mask
 constexpr uint32_t PART_TILE = 1024;
 
@@ -1350,7 +1353,7 @@ gc_status gc_jp_color(gc_graph *g) {
     // the tickets after the core as a heavy and a light stream (light_warps warps per CTA take the light one)
     const int light_warps = ctx->jp_light_warps;
     uint4 *split = nullptr;
-    if (g->n_seg > 1 && light_warps > 0 && light_warps < COLOR_WARPS_PER_CTA) {
+    if (g->n_seg > 1 && N > ctx->jp_light_min && light_warps > 0 && light_warps < COLOR_WARPS_PER_CTA) {
         const uint32_t ntiles = (N + PART_TILE - 1) / PART_TILE;
         if ((s = gc_alloc(ctx, &g->jpsplit, g->cap_N, "ticket streams")) != GC_OK) return s;
         if ((s = gc_alloc(ctx, &g->part_tiles, (g->cap_N + PART_TILE - 1) / PART_TILE, "ticket stream tiles")) != GC_OK)
