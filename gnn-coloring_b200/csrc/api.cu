@@ -298,6 +298,17 @@ gc_status color_by_tickets(gc_ctx *ctx, gc_graph *g) {
 // when it is asked for.  The last coloring's errors, stall flag and statistics come back in one read.
 gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *colors_used) {
     gc_status s;
+    if ((first || rounds > 0) && gc_small_eligible(g, rounds)) {
+        if (!first) {
+            if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
+            g->has_keys = true;
+        }
+        if ((s = gc_small_color(g, first ? rounds : rounds - 1, colors_used != nullptr)) != GC_OK) return s;
+        if (!ctx->hstate->flow_stall) {
+            if (colors_used) g->colors_used = *colors_used = gc_colors_of_state(g);
+            return GC_OK;
+        }
+    }
     if ((s = gc_reset_state(ctx)) != GC_OK) return s;
     bool unread = false;  // a dataflow coloring whose stall flag has not been read
     if (first && (s = color_by_keys(ctx, g, &unread)) != GC_OK) return s;
@@ -376,6 +387,7 @@ gc_status gc_ctx_create(int device, gc_ctx **out) {
     if (const char *e = getenv("GC_JP_TIGHT")) ctx->jp_tight = (unsigned int)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_FLOW")) ctx->flow_max_deg = (uint32_t)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_FLOW_CTAS")) ctx->flow_ctas_per_sm = std::max(1, atoi(e));
+    if (const char *e = getenv("GC_JP_SMALL")) ctx->small_max = (uint32_t)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_CLASSES")) ctx->jp_classes = atoi(e) != 0;
     if (const char *e = getenv("GC_JP_DECIDE")) ctx->jp_decide = atoi(e) != 0;
     if (const char *e = getenv("GC_JP_LIGHT_WARPS")) ctx->jp_light_warps = atoi(e);

@@ -36,6 +36,8 @@ constexpr uint32_t GC_GNN_WIDE_DEGREE = 4096;
 // 455 with 8, 462 with 32).
 constexpr uint32_t GC_GNN_THIN_DEGREE = 16;
 
+constexpr uint32_t GC_SMALL_AUTO = ~0u;
+
 struct gc_ctx {
     int device = 0;
     int num_sms = 0;
@@ -55,6 +57,8 @@ struct gc_ctx {
     bool jp_decide = true;               // coloring: early decisions from published forbidden colors
     uint32_t flow_max_deg = 128;         // coloring: graphs with a smaller maximum degree go by dataflow (0: none; GC_JP_FLOW)
     int flow_ctas_per_sm = 8;            // dataflow kernel: CTAs per SM at most (GC_JP_FLOW_CTAS)
+    uint32_t small_max = GC_SMALL_AUTO;  // coloring: graphs of up to this many vertices that fit go in one CTA (0: none; GC_JP_SMALL)
+    bool small_ready = false;            // that kernel's shared-memory limit is set
     int round_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each Culberson kernel
     int flow_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each dataflow kernel
     bool jp_classes = true;              // Culberson rounds: class by class instead of tickets
@@ -252,6 +256,11 @@ gc_status gc_jp_color(gc_graph *g);                                // JP by curr
 bool gc_flow_eligible(const gc_graph *g);
 gc_status gc_jp_flow(gc_graph *g);
 gc_status gc_keys_from_colors(gc_graph *g);                        // Culberson step (k_jp.cu)
+// JP by current keys, `rounds` Culberson rounds and (stats) the color count of a small graph in one CTA
+// (k_small.cu).  Waits; a set flow_stall means that nothing was written and the others must color it.
+bool gc_small_eligible(const gc_graph *g, int rounds);
+gc_status gc_small_color(gc_graph *g, int rounds, bool stats);
+
 // Culberson rounds on the library's own colors, class by class (k_round.cu); queued only.  `colors`: at
 // least the number of colors now (gc_queue_max_color leaves it in the state's first_colors).
 bool gc_rounds_eligible(const gc_graph *g);

@@ -45,14 +45,16 @@ GRAPHS = {
 
 @pytest.fixture(scope="module")
 def contexts():
-    """A context with the dataflow kernels and one without."""
+    """A context with the dataflow kernels and one without; small graphs have no kernel of their own."""
     device = int(os.environ.get("GC_DEVICE", "0"))
-    flow = gcn.Context(device)
-    os.environ["GC_JP_FLOW"] = "0"
+    os.environ["GC_JP_SMALL"] = "0"
     try:
+        flow = gcn.Context(device)
+        os.environ["GC_JP_FLOW"] = "0"
         tickets = gcn.Context(device)
     finally:
-        del os.environ["GC_JP_FLOW"]
+        os.environ.pop("GC_JP_FLOW", None)
+        del os.environ["GC_JP_SMALL"]
     models = [gcn.Model(c, *gcn.synthetic_model(3, 1003)) for c in (flow, tickets)]
     yield list(zip((flow, tickets), models))
     for m in models:

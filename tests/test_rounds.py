@@ -49,6 +49,18 @@ GRAPHS = {
 }
 
 
+@pytest.fixture(scope="module")
+def gpu_ctx():
+    """A context in which small graphs have no kernel of their own."""
+    os.environ["GC_JP_SMALL"] = "0"
+    try:
+        ctx = gcn.Context(int(os.environ.get("GC_DEVICE", "0")))
+    finally:
+        del os.environ["GC_JP_SMALL"]
+    yield ctx
+    ctx.close()
+
+
 @pytest.mark.parametrize("name", list(GRAPHS))
 def test_rounds_match_oracle(gpu_ctx, name):
     N, V, E = GRAPHS[name]()
