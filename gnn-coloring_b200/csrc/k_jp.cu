@@ -1076,6 +1076,12 @@ __global__ void __launch_bounds__(COLOR_THREADS, 6) k_jp_big_leaves(const uint32
 // (GC_SPLIT_CHUNK edges), the warp-tier vertices (vorder[0, n_wide)), then blocks of 32
 // consecutive vertices, which a warp takes 8 at a time with 4 lanes per vertex.  Vertices above
 // warp_deg have their edges checked by the first two kinds of item only.
+//
+// What bounds it: a gathered entry is an L1 tag look-up of its own, one a clock and SM (R-MAT of 123 M entries
+// with their lists 0.55 ms), once enough are in flight: 256^3 stencil 918 -> 712 us with eight per lane instead
+// of the row's end one at a time, R-MAT 2^22 706 -> 615, random geometric 2^23 617 -> 532, Erdos-Renyi 2 M x 16
+// 198 -> 160.  Gathering bytes instead of words (by id, or by degree for R-MAT) does not change the number of
+// look-ups and was slower: 1,031, 761, 590 and 186 us.
 __device__ __forceinline__ void stats_record(int *stat, DevState *st, uint32_t nseg, uint32_t s, int cmax, bool bad) {
     if (nseg) {
         atomicMax(stat + 2 * s, cmax);
@@ -1085,6 +1091,8 @@ __device__ __forceinline__ void stats_record(int *stat, DevState *st, uint32_t n
         if (bad) atomicOr(&st->invalid, 1u);
     }
 }
+
+constexpr int STATS_LOADS = 4;
 
 __global__ void __launch_bounds__(256) k_color_stats(const uint32_t *__restrict__ V, const uint32_t *__restrict__ E,
                                                      const int *__restrict__ color, const uint32_t *__restrict__ vorder,
@@ -1111,7 +1119,16 @@ __global__ void __launch_bounds__(256) k_color_stats(const uint32_t *__restrict_
             }
             const int cu = color[u];
             bool hit = false;
-            for (uint32_t j = b + lane; j < e; j += 32) hit |= color[ld_stream(E + j)] == cu;
+            for (uint32_t j = b + lane; j < e; j += 32 * STATS_LOADS) {
+                uint32_t v[STATS_LOADS];
+                int c[STATS_LOADS];
+#pragma unroll
+                for (int k = 0; k < STATS_LOADS; k++) v[k] = j + 32 * k < e ? ld_stream(E + j + 32 * k) : 0u;
+#pragma unroll
+                for (int k = 0; k < STATS_LOADS; k++) c[k] = j + 32 * k < e ? color[v[k]] : -1;
+#pragma unroll
+                for (int k = 0; k < STATS_LOADS; k++) hit |= j + 32 * k < e && c[k] == cu;
+            }
             if (__any_sync(0xffffffffu, hit) && lane == 0)
                 stats_record(stat, st, nseg, nseg ? seg_of(voff, nseg, u) : 0u, 0, true);
             continue;
@@ -1123,30 +1140,50 @@ __global__ void __launch_bounds__(256) k_color_stats(const uint32_t *__restrict_
         int bmax = 0;
         bool bbad = false;
 #pragma unroll 1
-        for (int sub = 0; sub < 4; sub++) {
-            const uint32_t u = base + 8 * sub + (lane >> 2);
-            const bool valid = u < N;
-            const uint32_t b = valid ? V[u] : 0u, e = valid ? V[u + 1] : 0u;
-            const int cu = valid ? color[u] : 0;
-            bool bad = valid && cu <= 0;
-            if (valid && e - b <= warp_deg) {
-                uint32_t j = b + q;
-                for (; j + 12 < e; j += 16) {
-                    const uint32_t v0 = ld_stream(E + j), v1 = ld_stream(E + j + 4);
-                    const uint32_t v2 = ld_stream(E + j + 8), v3 = ld_stream(E + j + 12);
-                    bad |= (color[v0] == cu) | (color[v1] == cu) | (color[v2] == cu) | (color[v3] == cu);
-                }
-                for (; j < e; j += 4) bad |= color[ld_stream(E + j)] == cu;
+        for (int sub = 0; sub < 4; sub += 2) {  // two vertices per quad at a time: 2 x STATS_LOADS entries in flight per lane
+            uint32_t u[2], b[2], d[2];
+            int cu[2];
+            bool bad[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                u[h] = base + 8 * (sub + h) + (lane >> 2);
+                const bool valid = u[h] < N;
+                b[h] = valid ? V[u[h]] : 0u;
+                d[h] = valid ? V[u[h] + 1] - b[h] : 0u;
+                cu[h] = valid ? color[u[h]] : 0;
+                bad[h] = valid && cu[h] <= 0;
+                if (d[h] > warp_deg) d[h] = 0;  // (a warp or task of its own, above)
             }
-            if (uniform) {
-                bmax = max(bmax, cu);
-                bbad |= bad;
-            } else {
-                const uint32_t s = valid ? seg_of(voff, nseg, u) : 0xffffffffu;
-                const unsigned int peers = __match_any_sync(0xffffffffu, s);
-                const int m = __reduce_max_sync(peers, cu);
-                const unsigned int anybad = __reduce_or_sync(peers, bad ? 1u : 0u);
-                if (valid && lane == __ffs(peers) - 1) stats_record(stat, st, nseg, s, m, anybad != 0);
+            const uint32_t dmax = __reduce_max_sync(0xffffffffu, max(d[0], d[1]));
+            for (uint32_t j = q; j < dmax; j += 4 * STATS_LOADS) {
+                uint32_t v[2][STATS_LOADS];
+                int c[2][STATS_LOADS];
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int k = 0; k < STATS_LOADS; k++) v[h][k] = j + 4 * k < d[h] ? ld_stream(E + b[h] + j + 4 * k) : 0u;
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int k = 0; k < STATS_LOADS; k++) c[h][k] = j + 4 * k < d[h] ? color[v[h][k]] : -1;
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int k = 0; k < STATS_LOADS; k++) bad[h] |= j + 4 * k < d[h] && c[h][k] == cu[h];
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (uniform) {
+                    bmax = max(bmax, cu[h]);
+                    bbad |= bad[h];
+                } else {
+                    const bool valid = u[h] < N;
+                    const uint32_t s = valid ? seg_of(voff, nseg, u[h]) : 0xffffffffu;
+                    const unsigned int peers = __match_any_sync(0xffffffffu, s);
+                    const int m = __reduce_max_sync(peers, cu[h]);
+                    const unsigned int anybad = __reduce_or_sync(peers, bad[h] ? 1u : 0u);
+                    if (valid && lane == __ffs(peers) - 1) stats_record(stat, st, nseg, s, m, anybad != 0);
+                }
             }
         }
         if (uniform) {
