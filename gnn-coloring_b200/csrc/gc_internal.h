@@ -36,7 +36,7 @@ constexpr uint32_t GC_GNN_WIDE_DEGREE = 4096;
 // 455 with 8, 462 with 32).
 constexpr uint32_t GC_GNN_THIN_DEGREE = 16;
 
-constexpr uint32_t GC_SMALL_AUTO = ~0u;
+constexpr uint32_t GC_SMALL_AUTO = ~0u, GC_CORE_AUTO = ~0u;
 
 struct gc_ctx {
     int device = 0;
@@ -62,7 +62,7 @@ struct gc_ctx {
     int round_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each Culberson kernel
     int flow_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each dataflow kernel
     bool jp_classes = true;              // Culberson rounds: class by class instead of tickets
-    uint32_t jp_core_max = 2048;        // coloring: first tickets colored inside one cluster (0: off; GC_JP_CORE)
+    uint32_t jp_core_max = GC_CORE_AUTO;  // coloring: first tickets colored inside one cluster (0: off; GC_JP_CORE)
     int jp_core_cluster = -1;            // CTAs of that cluster (16 or 8; 0: unavailable; -1: not yet queried)
     uint32_t jp_core_block = 16;         // consecutive core tickets per CTA (GC_JP_CORE_BLOCK)
     unsigned int jp_core_nap = 0;        // core kernel: sleep between polling rounds, ns (GC_JP_CORE_NAP)

@@ -283,11 +283,11 @@ __device__ __forceinline__ void publish_mask(unsigned long long *fmask, uint32_t
 // Colors one ordered vertex whose predecessors are list[0..cnt): the smallest color >= 1 none of
 // them has.  Every predecessor color is read first without waiting (LOADS per lane in flight);
 // the ids of uncolored ones go to the warp's pending list in shared memory, and only those are polled:
-// back to back at first, then with growing sleeps.  A list longer than PENDING waits in place for the
-// rest, a lane at a time and without early decisions; with 128 entries that was the usual case on
-// skewed graphs, and more warps in flight (longer lists) made it worse.  Ticket kernel on R-MAT of 4.2 M
-// vertices, GNN3 / GNN2 / first-fit keys: 128 entries and 2 CTAs per SM 5.0 / 4.4 / 5.1 ms, 1,024
-// entries and 4 CTAs 1.4 / 1.0 / 2.3 ms, with the polling below 1.1 / 0.7 / 2.3 ms.
+// back to back at first, then with growing sleeps.  Where the pending list is full, the rest of the
+// predecessors is read when there is room again.  Ticket kernel on R-MAT of 4.2 M vertices, GNN3 / GNN2 /
+// first-fit keys, waiting in place for what did not fit (a lane at a time): 128 entries and 2 CTAs per SM
+// 5.0 / 4.4 / 5.1 ms, 1,024 entries and 4 CTAs 1.4 / 1.0 / 2.3 ms, with the polling below 1.1 / 0.7 / 2.3 ms;
+// GNN4 keys, whose hubs come late, 18 ms so and 2.0 ms reading on later.
 // Returns -1 when a wait exceeded spin_limit polls or another warp raised the error flag.
 // With `fmask` set, the warp also publishes the colors it has seen (for vertex `self`) while it
 // waits, and tries early decisions once at most DECIDE_MAX predecessors are pending.
@@ -299,45 +299,30 @@ __device__ int color_one_v(const uint32_t *__restrict__ list, uint32_t cnt, cons
     for (uint32_t window = 0;; window++) {
         fb[lane] = 0;
         __syncwarp();
-        uint32_t npend = 0;  // warp-uniform
-        bool gave_up = false;
-        for (uint32_t j0 = 0; j0 < cnt; j0 += 32 * LOADS) {
-            uint32_t v[LOADS];
-            int c[LOADS];
+        uint32_t npend = 0, at = 0;  // warp-uniform; entries before `at` have been read
+        // reads on while the pending list has room for all that may be uncolored
+        auto read_list = [&]() {
+            for (; at < cnt && npend + 32 * LOADS <= PENDING; at += 32 * LOADS) {
+                uint32_t v[LOADS];
+                int c[LOADS];
 #pragma unroll
-            for (int q = 0; q < LOADS; q++) {
-                const uint32_t j = j0 + q * 32 + lane;
-                v[q] = j < cnt ? __ldg(list + j) : 0xffffffffu;
-            }
+                for (int q = 0; q < LOADS; q++) {
+                    const uint32_t j = at + q * 32 + lane;
+                    v[q] = j < cnt ? __ldg(list + j) : 0xffffffffu;
+                }
 #pragma unroll
-            for (int q = 0; q < LOADS; q++) c[q] = v[q] != 0xffffffffu ? ld_relaxed(color + v[q]) : -1;
+                for (int q = 0; q < LOADS; q++) c[q] = v[q] != 0xffffffffu ? ld_relaxed(color + v[q]) : -1;
 #pragma unroll
-            for (int q = 0; q < LOADS; q++) {
-                if (c[q] > 0) mark(fb, c[q], window);
-                const unsigned int zero = __ballot_sync(0xffffffffu, c[q] == 0);
-                if (zero) {
-                    const uint32_t slot = npend + __popc(zero & ((1u << lane) - 1u));
-                    if (c[q] == 0) {
-                        if (slot < PENDING) {
-                            pend[slot] = v[q];
-                        } else {  // list full: wait in place
-                            unsigned int spins = 0;
-                            int cc;
-                            while ((cc = ld_relaxed(color + v[q])) == 0) {
-                                if (++spins > spin_limit || ((spins & 255u) == 0 && ld_relaxed_u32(&st->err))) {
-                                    gave_up = true;
-                                    break;
-                                }
-                                __nanosleep(64);
-                            }
-                            if (!gave_up) mark(fb, cc, window);
-                        }
-                    }
-                    npend = min((uint32_t)PENDING, npend + __popc(zero));
+                for (int q = 0; q < LOADS; q++) {
+                    if (c[q] > 0) mark(fb, c[q], window);
+                    const unsigned int zero = __ballot_sync(0xffffffffu, c[q] == 0);
+                    if (c[q] == 0) pend[npend + __popc(zero & ((1u << lane) - 1u))] = v[q];
+                    npend += __popc(zero);
                 }
             }
-        }
-        __syncwarp();
+            __syncwarp();
+        };
+        read_list();
         const bool publish = fmask && window == 0 && npend > 0;
         if (publish) publish_mask(fmask, self, tag, fb, lane);
         // Polling.  A round over the whole list is hundreds of instructions, and a chain is as slow as the
@@ -358,9 +343,12 @@ __device__ int color_one_v(const uint32_t *__restrict__ list, uint32_t cnt, cons
             const unsigned long long w = ld_relaxed_u64(fmask + (size_t)v * GC_JP_MASK_WORDS + ((uint32_t)(c - 1) >> 5));
             return (uint32_t)(w >> 32) == epoch && ((w >> ((uint32_t)(c - 1) & 31u)) & 1ull) != 0;
         };
-        if (__any_sync(0xffffffffu, gave_up)) return -1;
-        while (npend > 1) {
-            if (fmask && npend <= DECIDE_MAX) {
+        while (npend > 1 || at < cnt) {
+            if (at < cnt && npend + 32 * LOADS <= PENDING) {
+                read_list();
+                continue;
+            }
+            if (fmask && npend <= DECIDE_MAX) {  // (all read)
                 const int cand = window_mex(fb, lane, window);
                 if (cand > 0 && __all_sync(0xffffffffu, (uint32_t)lane >= npend || excluded(pend[lane], cand))) {
                     __syncwarp();
@@ -453,10 +441,10 @@ __global__ void k_jp_records(const uint32_t *__restrict__ order, const uint32_t 
 // with the first 32,768 tickets colored the rest is only 214 deep).  Through global memory every
 // link of a chain costs a store-to-poll round trip in L2 (about 1 us); the first few thousand tickets, nearly a
 // clique, are where that counts.  Here one cluster colors tickets [0, K) with every color exchanged
-// through distributed shared memory instead.  K is 2,048 (ctx->jp_core_max): beyond the clique the
+// through distributed shared memory instead.  K is 2,048 (CORE_DEFAULT): beyond the clique the
 // ticket kernel's thousands of warps are faster than the cluster's 256 (core + ticket kernel on R-MAT of
-// 4.2 M vertices, largest degree first: K = 0 1.08 ms, 2,048 0.95, 4,096 0.96, 8,192 1.0, 32,768 1.3;
-// GNN3 keys 1.2, 1.41, 1.42, 1.45, 1.58; 100,003 vertices LF 0.40, 0.10, 0.11, 0.14, 0.22).
+// 4.2 M vertices, largest degree first: K = 0 1.25 ms, 1,024 1.03, 2,048 0.97, 4,096 0.95, 8,192 0.99, 32,768
+// 1.30; 100,003 vertices 0.11, 0.09, 0.10, 0.11, 0.14, 0.22).  core_tickets says where there is none.
 //   - each CTA holds a replica of the K core colors (16 bits each) in its shared memory;
 //   - tickets go to the CTAs in blocks of B consecutive ones (block k to CTA k % C), so a short link
 //     of a chain often stays inside one SM; a CTA hands its tickets out in order to whichever warp
@@ -1260,6 +1248,21 @@ gc_status core_cluster_config(gc_ctx *ctx) {
     return GC_OK;
 }
 
+// Core tickets wanted for a coloring.  The clique of hubs must come first in the ticket order and be large:
+// none up to 65,536 vertices (sort to leaves, without / with a core: R-MAT 50,000 x 10 LF 134 / 149 us, FF 124 /
+// 146, 20,000 x 24 146 / 151, 131 / 149; 100,003 x 16 217 / 178, 171 / 181; 300,007 x 32 358 / 257, 336 / 302; 2^22
+// x 32 1,515 / 1,167, 2,870 / 2,575; batches of 8,000 vertices 123 / 149, 132 / 159) and none by GNN keys, which
+// spread the hubs' order over chains that the ticket kernel follows as fast beside all else (GNN3, same graphs
+// 189 / 208, 194 / 211, 230 / 254, 362 / 391, 1,550 / 1,691; GNN2 100,003 246 / 233, 2^22 1,248 / 1,280).  A
+// large batch is quicker with one under every heuristic (64 graphs, 2.2 M vertices, GNN2 2,250 / 2,200).
+constexpr uint32_t CORE_DEFAULT = 2048, CORE_MIN_N = 65536;
+
+uint32_t core_tickets(const gc_graph *g) {
+    const uint32_t most = g->ctx->jp_core_max;
+    if (most != GC_CORE_AUTO) return most;
+    return g->N > CORE_MIN_N && (g->n_seg || g->key_kind != GC_GNN) ? CORE_DEFAULT : 0u;
+}
+
 // The most core tickets, up to kmax, whose replicas and published sets fit the core kernel's shared
 // memory on a cluster of the configured size.
 uint32_t core_fit(const gc_ctx *ctx, uint32_t kmax) {
@@ -1360,7 +1363,8 @@ gc_status gc_jp_color(gc_graph *g) {
 
     if ((s = gc_alloc(ctx, &g->jprec, g->cap_N, "ticket records")) != GC_OK) return s;
     uint32_t core = 0;  // core tickets colored in one cluster (at most)
-    if (ctx->jp_core_max && (s = core_cluster_config(ctx)) == GC_OK && ctx->jp_core_cluster > 0) core = core_fit(ctx, ctx->jp_core_max);
+    const uint32_t wanted = core_tickets(g);
+    if (wanted && (s = core_cluster_config(ctx)) == GC_OK && ctx->jp_core_cluster > 0) core = core_fit(ctx, wanted);
     if (s != GC_OK) return s;
     if (core && (s = gc_alloc(ctx, &g->rank, g->cap_N, "core ranks")) != GC_OK) return s;
     k_jp_records<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(g->order, g->V, g->pc, ctx->dstate, g->jprec,
