@@ -52,6 +52,7 @@ constexpr uint32_t FLOW_PAD = 32;  // words between counters: one 128-byte line 
 constexpr uint32_t FLOW_CTA = 3 * FLOW_QUEUES * FLOW_PAD;  // the CTAs' start counter
 constexpr uint32_t FLOW_SLOTS = FLOW_CTA + FLOW_PAD;       // first queue slot
 constexpr int FLOW_THREADS = 256;
+constexpr uint32_t FLOW_FEW_N = 1u << 18;
 
 // A vertex's counter word: rem in bits 48..63, the degree in bits 32..47, the first CSR entry below.
 // The subtraction that makes a successor ready so returns where its neighbour list is, and the list is
@@ -311,8 +312,12 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
     }
     {
         ProfScope ps(ctx, "jp_flow", ctx->stream);
-        // at least four CTAs (a warp for every array); a warp per four vertices at most
-        const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)std::min(occ, ctx->flow_ctas_per_sm);
+        // at least four CTAs (a warp for every array); a warp per four vertices at most; up to FLOW_FEW_N
+        // vertices half of what fits, since the chains are then all there is and idle warps' polls slow them
+        // (8 / 4 per SM: Erdos-Renyi 65,536 LF 113 / 102 us, GNN3 128 / 115, random geometric 200,000 108 / 99;
+        // 500,000 149 / 195, Erdos-Renyi 600,000 226 / 279)
+        const int per_sm = std::min(occ, N <= FLOW_FEW_N ? std::max(1, ctx->flow_ctas_per_sm / 2) : ctx->flow_ctas_per_sm);
+        const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)per_sm;
         const uint32_t blocks = std::max<uint32_t>(4u, std::min<uint32_t>(most, (N + 31) / 32));
         k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->color, g->flow_q, N, stride,
                                                                ctx->dstate, std::min<uint32_t>(ctx->spin_limit, 1u << 16));
