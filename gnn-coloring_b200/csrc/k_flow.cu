@@ -32,14 +32,20 @@
 // DevState::flow_stall and every warp leaves.  The host then runs the ticket kernels, whose waits
 // only follow each vertex's own list.
 //
-// What bounds it: on a wavefront the chain of hops, each a counter atomic, then the neighbour ids, then
-// the next atomic (about 1.7 us); elsewhere the vertices in flight (one per warp, 2 to 3 us each).
+// What bounds it: on a wavefront the chain of hops.  A hop to the successor a warp goes on with takes 0.63 us
+// (its counter's atomic, then its neighbour ids); one through a queue adds the tail's atomic, the slot's
+// store and poll, so a slot holds where the list begins as well: fetched after the counter word, stencils
+// took up to 15 % longer (256^3 GNN4 10.5 -> 9.0 ms, Erdos-Renyi 400,000 GNN3 229 -> 184 us, 65,536 LF 112 ->
+// 96).  Elsewhere the vertices in flight (one per warp, 2 to 3 us each; 256^3 first fit 6).
 // Measured on a B200, coloring kernels of one job, tickets (sort, cluster core, streams, ticket kernel,
-// leaves) -> dataflow: 256^3 stencil with GNN4 keys 272 -> 11 ms, 97 x 61 x 113 stencil first fit
-// 8.9 -> 1.1 ms, random geometric 2^23 GNN4 4.0 -> 2.7 ms, Erdos-Renyi 65,536 LF 0.36 -> 0.13 ms.
+// leaves) -> dataflow: 256^3 stencil with GNN4 keys 272 -> 9.6 ms, 97 x 61 x 113 stencil first fit
+// 8.9 -> 1.1 ms, random geometric 2^23 GNN4 4.0 -> 2.7 ms, Erdos-Renyi 65,536 LF 0.36 -> 0.11 ms.
 // Measured and not kept: eight lanes per vertex and four vertices per warp (hops of 3.3 us: the longer
 // code path of a lane is on the chain), a separate 16-byte record (hops of 1.9 us), a slot taken
-// before the color is stored, four slots taken at once under backlog.
+// before the color is stored, four slots taken at once under backlog; ready vertices handed to waiting
+// warps of the same CTA through shared memory (97 x 61 x 113 first fit 1.1 -> 1.4 ms and more: the atomics
+// of many vertices in one SM are slower); lists fetched into L2 when one predecessor is left to start
+// (stencils 5 % faster, the others 1 to 5 % slower).
 #include <algorithm>
 
 #include "gc_internal.h"
@@ -86,11 +92,16 @@ __device__ __forceinline__ uint32_t *flow_head(uint32_t *fq, uint32_t k) { retur
 __device__ __forceinline__ uint32_t *flow_tail(uint32_t *fq, uint32_t k) { return fq + (FLOW_QUEUES + k) * FLOW_PAD; }
 __device__ __forceinline__ uint32_t *flow_skip(uint32_t *fq, uint32_t k) { return fq + (2 * FLOW_QUEUES + k) * FLOW_PAD; }
 
-// Queues vertex v: slots hold v + 1, so that the zeroed buffer reads as empty.
-__device__ __forceinline__ void flow_push(uint32_t *fq, uint32_t stride, uint32_t v) {
+__device__ __forceinline__ unsigned long long *flow_slots(uint32_t *fq) {
+    return reinterpret_cast<unsigned long long *>(fq + FLOW_SLOTS);
+}
+
+// Queues vertex v, whose list begins at `beg`: slots hold v + 1 and beg, so that the zeroed buffer reads as
+// empty and the list can be fetched along with the counter word.
+__device__ __forceinline__ void flow_push(uint32_t *fq, uint32_t stride, uint32_t v, uint32_t beg) {
     const uint32_t k = v % FLOW_QUEUES;
     const uint32_t at = atomicAdd(flow_tail(fq, k), 1u);
-    if (at < stride) st_relaxed_u32(fq + FLOW_SLOTS + (size_t)k * stride + at, v + 1u);
+    if (at < stride) st_relaxed_u64(flow_slots(fq) + (size_t)k * stride + at, (unsigned long long)beg << 32 | (v + 1u));
 }
 
 // Four lanes per vertex, vertices in id order (records, CSR offsets and rows stream).
@@ -136,7 +147,7 @@ __global__ void __launch_bounds__(FLOW_THREADS) k_flow_init(const uint32_t *__re
             word[u] = (unsigned long long)cnt * FLOW_ONE | (unsigned long long)d << 32 | beg;
             mask[u] = FlowMask<W>::put(m);
             color[u] = cnt == 0 ? 1 : 0;
-            if (cnt == 0) flow_push(fq, stride, u);
+            if (cnt == 0) flow_push(fq, stride, u, beg);
         }
     }
 }
@@ -170,7 +181,7 @@ struct FlowWait {
 template <int W>
 __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsigned long long *word,
                                                           const typename FlowMask<W>::T *__restrict__ mask,
-                                                          const uint32_t *__restrict__ E, int *color, uint32_t *fq,
+                                                          const uint32_t *__restrict__ E, uint32_t M, int *color, uint32_t *fq,
                                                           uint32_t N, uint32_t stride, DevState *st, uint32_t check) {
     constexpr unsigned int FULL = 0xffffffffu;
     __shared__ uint32_t cta_s;
@@ -180,7 +191,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsign
     const uint32_t k = (cta_s * (FLOW_THREADS / 32) + (threadIdx.x >> 5)) % FLOW_QUEUES;
     const uint32_t nk = k < N ? (N - k + FLOW_QUEUES - 1) / FLOW_QUEUES : 0u;  // vertices of this array
     uint32_t *head = flow_head(fq, k), *skip = flow_skip(fq, k);
-    const uint32_t *slots = fq + FLOW_SLOTS + (size_t)k * stride;
+    const unsigned long long *slots = flow_slots(fq) + (size_t)k * stride;
     FlowWait fw;
     uint32_t u, d, v[W];  // the vertex, its degree, and this lane's neighbours (entries 32 w + lane)
     typename FlowMask<W>::T mt;
@@ -193,21 +204,26 @@ __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsign
     for (;;) {
         // a queued vertex: take a slot and wait until it is filled, or can no longer be (vertices that a
         // warp went on with leave that many slots at the array's end unfilled)
-        uint32_t slot = 0, u1 = 0;
+        uint32_t slot = 0;
+        unsigned long long u1 = 0;
         if (lane == 0) slot = atomicAdd(head, 1u);
         slot = __shfl_sync(FULL, slot, 0);
         if (slot >= nk) return;
         for (;;) {
-            u1 = __shfl_sync(FULL, lane == 0 ? ld_relaxed_u32(slots + slot) : 0u, 0);
+            u1 = __shfl_sync(FULL, lane == 0 ? ld_relaxed_u64(slots + slot) : 0ull, 0);
             if (u1) break;
             if ((fw.spins & 7u) == 7u && slot + min(nk, __shfl_sync(FULL, lane == 0 ? ld_relaxed_u32(skip) : 0u, 0)) >= nk) return;
             if (fw.give_up(fq, st, check, lane)) return;
         }
         fw.spins = 0;
-        u = u1 - 1u;
-        {
-            const unsigned long long wu = __ldcg(word + u);
-            fetch((uint32_t)wu, (uint32_t)(wu >> 32));
+        u = (uint32_t)u1 - 1u;
+        {   // the list's first 32 entries are fetched before its length is known
+            const uint32_t lo = (uint32_t)(u1 >> 32);
+            mt = __ldg(mask + u);
+            v[0] = lane < M - lo ? ld_stream(E + lo + lane) : 0u;
+            d = (uint32_t)(__ldcg(word + u) >> 32) & 0xffffu;
+#pragma unroll
+            for (int w = 1; w < W; w++) v[w] = 32u * w + lane < d ? ld_stream(E + lo + 32 * w + lane) : 0u;
         }
         for (;;) {  // u, then a successor that u made ready, and so on
             uint32_t m[W], wait = 0;  // wait, bit w: entry 32 w + lane is a predecessor without a color
@@ -250,7 +266,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsign
                         atomicAdd(flow_skip(fq, u % FLOW_QUEUES), 1u);
                     }
                 }
-                if (ready) flow_push(fq, stride, keep[w]);
+                if (ready) flow_push(fq, stride, keep[w], (uint32_t)old[w]);
             }
             uint32_t used[W];
 #pragma unroll
@@ -300,7 +316,7 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
             return s;
         if (occ < 1) occ = 1;
     }
-    if ((s = gc_check_cuda(ctx, cudaMemsetAsync(g->flow_q, 0, 4 * ((size_t)FLOW_SLOTS + (size_t)FLOW_QUEUES * stride),
+    if ((s = gc_check_cuda(ctx, cudaMemsetAsync(g->flow_q, 0, 4 * ((size_t)FLOW_SLOTS + 2 * (size_t)FLOW_QUEUES * stride),
                                                 ctx->stream), "flow queues")) != GC_OK)
         return s;
     const uint32_t N = g->N;
@@ -314,12 +330,12 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
         ProfScope ps(ctx, "jp_flow", ctx->stream);
         // at least four CTAs (a warp for every array); a warp per four vertices at most; up to FLOW_FEW_N
         // vertices half of what fits, since the chains are then all there is and idle warps' polls slow them
-        // (8 / 4 per SM: Erdos-Renyi 65,536 LF 113 / 102 us, GNN3 128 / 115, random geometric 200,000 108 / 99;
-        // 500,000 149 / 195, Erdos-Renyi 600,000 226 / 279)
+        // (8 / 4 per SM, one slot's list fetched later: Erdos-Renyi 65,536 LF 113 / 102 us, GNN3 128 / 115, random
+        // geometric 200,000 108 / 99; 500,000 149 / 195, Erdos-Renyi 600,000 226 / 279)
         const int per_sm = std::min(occ, N <= FLOW_FEW_N ? std::max(1, ctx->flow_ctas_per_sm / 2) : ctx->flow_ctas_per_sm);
         const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)per_sm;
         const uint32_t blocks = std::max<uint32_t>(4u, std::min<uint32_t>(most, (N + 31) / 32));
-        k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->color, g->flow_q, N, stride,
+        k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->M, g->color, g->flow_q, N, stride,
                                                                ctx->dstate, std::min<uint32_t>(ctx->spin_limit, 1u << 16));
     }
     ctx->launches += 2;
@@ -348,6 +364,6 @@ gc_status gc_jp_flow(gc_graph *g) {
     const uint32_t stride = (g->N + FLOW_QUEUES - 1) / FLOW_QUEUES;
     if ((s = gc_alloc(ctx, &g->jprec, g->cap_N, "vertex records")) != GC_OK) return s;
     if (wide && (s = gc_alloc(ctx, &g->jpsplit, g->cap_N, "vertex records")) != GC_OK) return s;
-    if ((s = gc_alloc(ctx, &g->flow_q, (size_t)g->cap_N + FLOW_QUEUES + FLOW_SLOTS, "flow queues")) != GC_OK) return s;
+    if ((s = gc_alloc(ctx, &g->flow_q, 2 * ((size_t)g->cap_N + FLOW_QUEUES) + FLOW_SLOTS, "flow queues")) != GC_OK) return s;
     return wide ? flow_run<FLOW_WIDE>(g, stride) : g->max_deg >= 32 ? flow_run<2>(g, stride) : flow_run<1>(g, stride);
 }
