@@ -37,31 +37,33 @@ __global__ void k_simple_keys(const uint32_t *__restrict__ V, uint32_t N, int h,
 // delta + 1.  Removal within a round depends only on the degrees at the round's start and the
 // decrements commute, so the keys equal the reference's at any thread count.
 //
-// All rounds run in one cooperative kernel, a CTA of 1,024 threads per SM: filter, barrier, decrement,
-// barrier.  A power-law graph has hundreds of rounds, most of which remove a few vertices, so a round
-// is bound by its latencies: two grid barriers and a few dependent loads.
-//   - Once the remaining vertices fit the threads (four each), every thread keeps its own: the filter
-//     reads their degrees, and the warp that finds removed vertices of up to PEEL_WARP_DEG neighbours
-//     decrements them itself after the barrier, eight lanes each; larger ones go to a list whose
-//     vertices share all threads evenly.  Before that (large graphs, the
-//     first rounds), the filter scans a list of the remaining vertices and puts all removed ones on lists.
+// All rounds run in one cooperative kernel, a CTA of 1,024 threads per SM.  A power-law graph has hundreds
+// of rounds, most of which remove a few vertices, so a round is bound by its latencies: a grid barrier (1.9
+// us) and a few dependent loads.
+//   - While the remaining vertices are more than the threads can keep (four each), a round is filter, barrier,
+//     decrement, barrier: the filter scans a list of them and puts the removed ones on lists.
+//   - After that every thread keeps its own vertices and their degrees in registers, and a round has one
+//     barrier.  Round r counts neighbours down in array r mod 2, and in round r + 1 the owner of a vertex
+//     takes what that array has lost since it last looked off the vertex's degree.  So nobody reads what
+//     others are counting down, and a removed vertex's neighbours are counted down at once: lists of up to
+//     PEEL_WARP_DEG by its warp, eight lanes each, longer ones by its CTA.
 //   - The decrements go to every neighbour without asking whether it is still there (nothing reads a
 //     removed vertex's degree again), so nothing waits for their results.
 //   - SL tries delta + 1 first; only when that removes nothing does it look for the smallest remaining
 //     degree (one more barrier).
-//   - When no vertex remains, the last round's decrements are left out.
-//   - The barrier's counter and the round's counts are one 16-byte word, polled together by one thread
+//   - The barrier's counter and the round's count are one 16-byte word, polled together by one thread
 //     per CTA.
 // Measured (B200), three launches per round queued in batches -> this: SL on R-MAT of 2^20 vertices and
-// edge factor 16 (217 rounds) 8.2 -> 1.9 ms, on Erdos-Renyi 65,536 (16 rounds) 0.41 -> 0.10 ms.  A round
-// of the former takes about 5.5 us when it removes little (the barriers 3.8 of them) and 10 us when it
-// removes thousands (decrements of the same hubs, one at a time).  All removed vertices on lists: 2.2 ms;
-// a whole warp for every kept one: 2.3 ms.
+// edge factor 16 (217 rounds) 8.2 -> 1.6 ms, on Erdos-Renyi 65,536 (16 rounds) 0.41 -> 0.09 ms.  With two
+// barriers in every round and long lists shared by the grid: 1.9 and 0.10.  Rounds that remove thousands
+// take longer (decrements of the same hubs, one at a time).  All removed vertices on lists: 2.2 ms; a whole
+// warp for every kept one: 2.3 ms.
 constexpr uint32_t GONE = 0xffffffffu;
 constexpr uint32_t NO_DEGREE = 0xffffffffu;
 constexpr int PEEL_THREADS = 1024;
 constexpr int PEEL_ITEMS = 4;              // vertices a thread keeps
 constexpr uint32_t PEEL_WARP_DEG = 64;
+constexpr uint32_t PEEL_WIDE = 512;
 constexpr unsigned int PEEL_WAIT_LIMIT = 1u << 24;  // polls of one barrier
 
 struct PeelState {
@@ -167,6 +169,8 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
     constexpr int ITEMS = PEEL_ITEMS;
     __shared__ unsigned int cta_min;
     __shared__ uint2 own[PEEL_THREADS / 32][32 * ITEMS];  // per warp: the lists it decrements
+    __shared__ uint2 wide[PEEL_WIDE];                     // long lists that the CTA shares
+    __shared__ unsigned int wide_n[2];                    // their number, by the round's parity
     const int lane = threadIdx.x & 31;
     const unsigned int lt = (1u << lane) - 1u;
     const uint32_t tid = blockIdx.x * PEEL_THREADS + threadIdx.x, threads = gridDim.x * PEEL_THREADS;
@@ -305,66 +309,59 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
         }
         if (!round_end()) return;
     }
-    // ---- each thread keeps its vertices (neighbouring list entries in different warps: the list is close to
-    // id order, and vertices that leave together are often neighbours in it)
+    // ---- each thread keeps its vertices and their degrees (neighbouring list entries in different warps: the
+    // list is close to id order, and vertices that leave together are often neighbours in it)
+    uint32_t seen[ITEMS], seen_next[ITEMS];  // a kept vertex's counters when they were last read
     if (!done) {
         const uint32_t slot0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = threads >> 5;
+        const uint32_t *past = (r & 1) ? deg : other, *next = (r & 1) ? other : deg;
 #pragma unroll
         for (int k = 0; k < ITEMS; k++) {
             const uint32_t i = ((uint32_t)k * 32u + lane) * warps + slot0;
             u[k] = i < len ? __ldcg(cur + i) : GONE;
-            beg[k] = end[k] = 0;
+            beg[k] = end[k] = d[k] = seen[k] = seen_next[k] = 0;
             if (u[k] != GONE) {
                 beg[k] = V[u[k]];
                 end[k] = V[u[k] + 1];
+                d[k] = __ldcg(deg + u[k]);
+                seen[k] = __ldcg(past + u[k]);
+                seen_next[k] = __ldcg(next + u[k]);
             }
         }
+        if (threadIdx.x < 2) wide_n[threadIdx.x] = 0;
+        if (!peel_barrier(ps, target, nullptr, value)) return;  // (nothing is counted down before all have read)
     }
     for (; !done; r++) {
         uint4 *sl = &ps->slot[r % 3];
         const uint32_t thr = threshold();
+        const uint32_t *past = (r & 1) ? deg : other;
+        uint32_t *count = (r & 1) ? other : deg;
         low = NO_DEGREE;
-        // rm, bit k: vertex k leaves now and this warp decrements its neighbours; bit 4 + k: it goes on the list
-        uint32_t rm = 0, cnt = 0, longs = 0;
+        uint32_t rm = 0, cnt = 0, out_n = 0;  // rm, bit k: vertex k leaves and this warp counts its neighbours down
+        uint32_t x[ITEMS];
 #pragma unroll
-        for (int k = 0; k < ITEMS; k++) d[k] = u[k] != GONE ? __ldcg(deg + u[k]) : NO_DEGREE;
+        for (int k = 0; k < ITEMS; k++) x[k] = u[k] != GONE ? __ldcg(past + u[k]) : 0u;
 #pragma unroll
         for (int k = 0; k < ITEMS; k++) {
-            const bool there = u[k] != GONE, out = there && d[k] <= thr;
-            const bool is_long = out && end[k] - beg[k] > PEEL_WARP_DEG;
+            const bool there = u[k] != GONE;
+            d[k] -= seen[k] - x[k];
+            seen[k] = seen_next[k];
+            seen_next[k] = x[k];
+            const bool out = there && d[k] <= thr;
             if (out) {
                 key[u[k]] = delta;
-                rm |= (is_long ? 16u : 1u) << k;
+                u[k] = GONE;
+                uint32_t at = PEEL_WIDE;
+                if (end[k] - beg[k] > PEEL_WARP_DEG) at = atomicAdd(&wide_n[r & 1], 1u);
+                if (at < PEEL_WIDE) wide[at] = make_uint2(beg[k], end[k]);
+                else rm |= 1u << k;
             } else if (there) {
                 low = min(low, d[k]);
             }
-            cnt += __popc(__ballot_sync(FULL, out && !is_long));
-            longs += __popc(__ballot_sync(FULL, is_long));
+            out_n += __popc(__ballot_sync(FULL, out));
+            cnt += __popc(__ballot_sync(FULL, (rm >> k) & 1u));
         }
-        if (lane == 0 && cnt) atomicAdd(&sl->y, cnt);
-        if (longs) {
-            uint32_t at = 0;
-            if (lane == 0) at = atomicAdd(&sl->z, longs);
-            at = __shfl_sync(FULL, at, 0);
-#pragma unroll
-            for (int k = 0; k < ITEMS; k++) {
-                const bool is_long = (rm >> k) & 16u;
-                const unsigned int ml = __ballot_sync(FULL, is_long);
-                if (is_long) removed[N - 1u - (at + __popc(ml & lt))] = u[k];
-                at += __popc(ml);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < ITEMS; k++)
-            if ((rm >> k) & 17u) u[k] = GONE;
-        if (!peel_slot_barrier(ps, sl, got)) return;
-        const uint32_t ns = got.y, nl = got.z;
-        alive -= ns + nl;
-        if (alive == 0) {
-            r++;
-            break;
-        }
-        if (nl) decrement(removed + (N - 1u), -1, nl, 32u);
+        if (lane == 0 && out_n) atomicAdd(&sl->y, out_n);
         if (cnt) {  // the warp's own: their lists packed, eight lanes each
             uint2 *mine = own[threadIdx.x >> 5];
             uint32_t at = 0;
@@ -376,16 +373,32 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
                 at += __popc(mk);
             }
             __syncwarp();
-            for (uint32_t i = lane >> 3; i < cnt; i += 4) peel_neighbours(E, mine[i].x + (lane & 7), mine[i].y, 8u, deg);
+            for (uint32_t i = lane >> 3; i < cnt; i += 4) peel_neighbours(E, mine[i].x + (lane & 7), mine[i].y, 8u, count);
             __syncwarp();
         }
-        if (ns + nl == 0 && !log_mode) {
+        __syncthreads();
+        if (const uint32_t n = min(wide_n[r & 1], PEEL_WIDE)) {  // the CTA's long lists, a power of two of lanes each
+            const uint32_t most = PEEL_THREADS / n, lanes = most <= 32 ? 32u : 1u << (31 - __clz(most));
+            for (uint32_t i = threadIdx.x / lanes; i < n; i += PEEL_THREADS / lanes)
+                peel_neighbours(E, wide[i].x + (threadIdx.x & (lanes - 1u)), wide[i].y, lanes, count);
+        }
+        if (threadIdx.x == 0) wide_n[(r + 1) & 1] = 0;
+        if (tid == 0) {  // the next round's slot: every CTA has left the barrier of the round before last
+            ps->slot[(r + 1) % 3] = make_uint4(0u, 0u, 0u, 0u);
+            ps->min_deg[(r + 1) % 3] = NO_DEGREE;
+        }
+        if (!peel_slot_barrier(ps, sl, got)) return;
+        alive -= got.y;
+        if (alive == 0) {
+            r++;
+            break;
+        }
+        if (got.y == 0 && !log_mode) {
             if (!grid_min(low, &ps->min_deg[r % 3])) return;
             delta = max(delta, value);
         } else {
             delta++;
         }
-        if (!round_end()) return;
     }
     if (tid == 0) ps->rounds = r ? r : 1u;
 }
