@@ -29,6 +29,7 @@ struct DevState {
     unsigned int n_light;       // coloring: tickets of the light stream (after the core)
     unsigned int isolated;      // preparation: vertices without neighbours (outside the hub list)
     unsigned int first_colors;  // Culberson rounds: colors of the coloring they start from
+    unsigned int core_pred;     // coloring: predecessors of the core's tickets
     unsigned int flow_stall;    // coloring: the dataflow kernel stopped before every vertex was queued
 };
 

@@ -155,7 +155,9 @@ __global__ void __launch_bounds__(SPLIT_WARPS * 32) k_jp_split_big(const uint32_
 }
 
 // Sources (no predecessor) take color 1 now; everything else starts uncolored.
-__global__ void k_jp_init_colors(const uint32_t *__restrict__ pc, uint32_t N, int *__restrict__ color) {
+__global__ void k_jp_init_colors(const uint32_t *__restrict__ pc, uint32_t N, int *__restrict__ color, DevState *st,
+                                 uint32_t core_pred) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->core_pred = core_pred;
     for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < N; u += gridDim.x * blockDim.x)
         color[u] = pc[u] == 0 ? 1 : 0;
 }
@@ -422,15 +424,19 @@ __device__ int color_one_v(const uint32_t *__restrict__ list, uint32_t cnt, cons
 // or done, so the oldest unfinished ticket always progresses.
 // Ticket records: rec[t] = (vertex, first CSR entry, predecessor count) of ticket t, so that a
 // warp needs one 16-byte load per ticket instead of the order -> V, pc chain.
-// With `rank` set, the tickets below kmax (the cluster-colored core) also record rank[u] = t.
+// With `rank` set, the tickets below kmax (the cluster-colored core) also record rank[u] = t and add up
+// their predecessors.
 __global__ void k_jp_records(const uint32_t *__restrict__ order, const uint32_t *__restrict__ V,
-                             const uint32_t *__restrict__ pc, const DevState *st, uint4 *__restrict__ rec,
+                             const uint32_t *__restrict__ pc, DevState *st, uint4 *__restrict__ rec,
                              uint32_t *__restrict__ rank, uint32_t kmax) {
     const uint32_t n = st->ordered;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const uint32_t u = order[t];
-        rec[t] = make_uint4(u, V[u], pc[u], 0u);
-        if (rank && t < kmax) rank[u] = t;
+        const uint32_t u = order[t], cnt = pc[u];
+        rec[t] = make_uint4(u, V[u], cnt, 0u);
+        if (rank && t < kmax) {
+            rank[u] = t;
+            atomicAdd(&st->core_pred, min(cnt, kmax));
+        }
     }
 }
 
@@ -464,6 +470,8 @@ __global__ void k_jp_records(const uint32_t *__restrict__ order, const uint32_t 
 // Waits are bounded (spin_limit polls; on expiry the error is raised and the warp publishes
 // 0xffff, which releases its successors).  A cluster barrier before exit keeps every CTA's shared
 // memory alive while others may still store into it.
+constexpr uint32_t CORE_FORCED = 1u << 31;     // in DevState::core_pred: take the core whatever its density
+constexpr uint32_t CORE_DENSE = 28;
 constexpr int CORE_WARPS = 32;                 // most warps per CTA (the launch takes ctx->jp_core_warps)
 constexpr int CORE_PEND = 256;                 // per warp: uncolored predecessors remembered for polling
 constexpr uint32_t CORE_MAX = 32768;           // most core tickets (16-bit ranks, 64 KB replica)
@@ -471,6 +479,12 @@ constexpr int CORE_LOADS = 8;                  // per lane: predecessor ranks in
 constexpr int CORE_PUB = 8;                    // published seen colors per core ticket: 8 words, colors 1..256
 constexpr uint32_t CORE_DECIDE = 32;           // at most this many pending: one per lane, early decisions tried
 static_assert(CORE_DECIDE <= 32, "one pending predecessor per lane");
+
+// The core's tickets: the first kmax, where they are a dense set (the rule beside core_tickets), else none.
+__device__ __forceinline__ uint32_t core_size(const DevState *st, uint32_t kmax) {
+    const uint32_t K = min(st->ordered, kmax), pred = st->core_pred;
+    return (pred & CORE_FORCED) || (unsigned long long)pred * CORE_DENSE >= (unsigned long long)K * K ? K : 0u;
+}
 
 // Tickets one CTA of a C-CTA cluster owns, for K core tickets in blocks of B (an upper bound).
 __host__ __device__ __forceinline__ uint32_t core_owned(uint32_t K, uint32_t B, uint32_t C) {
@@ -529,7 +543,7 @@ __device__ __forceinline__ void core_st_remote(const unsigned short *p, unsigned
 __global__ void __launch_bounds__(256) k_jp_core_lists(uint4 *__restrict__ rec, uint32_t *__restrict__ P,
                                                        const uint32_t *__restrict__ rank, const int *__restrict__ color,
                                                        const DevState *st, uint32_t kmax) {
-    const uint32_t K = min(st->ordered, kmax);
+    const uint32_t K = core_size(st, kmax);
     const int lane = threadIdx.x & 31;
     const unsigned int lt = (1u << lane) - 1u;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -577,7 +591,7 @@ __global__ void __launch_bounds__(CORE_WARPS * 32, 1) k_jp_core(const uint4 *__r
     const uint32_t npub = core_owned(kmax, B, C);
     uint32_t *fb_all = pub + (size_t)npub * CORE_PUB;                         // W x 32
     unsigned short *pend_all = reinterpret_cast<unsigned short *>(fb_all + CORE_WARPS * 32);  // W x CORE_PEND
-    const uint32_t K = min(ld_relaxed_u32(&st->ordered), kmax);
+    const uint32_t K = core_size(st, kmax);
     for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) {
         replica[i] = 0;
         cpc[i] = (unsigned short)(rec[i].w >> 1);
@@ -827,7 +841,7 @@ constexpr uint32_t PART_TILE = 1024;
 __global__ void __launch_bounds__(PART_TILE) k_jp_part_count(const uint4 *__restrict__ rec, const DevState *st,
                                                              uint32_t core, uint32_t *__restrict__ tile_heavy) {
     __shared__ uint32_t warp_cnt[PART_TILE / 32];
-    const uint32_t n = st->ordered, first = min(n, core);
+    const uint32_t n = st->ordered, first = core_size(st, core);
     const uint32_t t = first + blockIdx.x * PART_TILE + threadIdx.x;
     const bool heavy = t < n && rec[t].z > LIGHT_MAX;
     const unsigned int m = __ballot_sync(0xffffffffu, heavy);
@@ -876,7 +890,7 @@ __global__ void __launch_bounds__(1024) k_jp_part_scan(uint32_t *__restrict__ ti
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        const uint32_t n = st->ordered, first = min(n, core);
+        const uint32_t n = st->ordered, first = core_size(st, core);
         st->n_heavy = carry;
         st->n_light = n - first - carry;
         st->ticket_light = 0;
@@ -889,7 +903,7 @@ __global__ void __launch_bounds__(PART_TILE) k_jp_part_scatter(const uint4 *__re
                                                                uint32_t core, const uint32_t *__restrict__ tile_heavy,
                                                                uint4 *__restrict__ out, uint32_t cap) {
     __shared__ uint32_t warp_off[PART_TILE / 32];
-    const uint32_t n = st->ordered, first = min(n, core);
+    const uint32_t n = st->ordered, first = core_size(st, core);
     const uint32_t tile0 = first + blockIdx.x * PART_TILE;
     const uint32_t t = tile0 + threadIdx.x;
     const bool valid = t < n;
@@ -1188,10 +1202,10 @@ __global__ void k_keys_from_colors(const int *__restrict__ color, uint32_t N, ui
 }
 
 // Also advances the epoch of the published forbidden colors (never 0: the buffer starts zeroed).
-// The ordered kernel's first ticket: past the core tickets the cluster colored (first_cap of them
-// at most), else 0.
-__global__ void k_reset_ticket(DevState *st, unsigned long long *epoch_word, uint32_t first_cap = 0) {
-    st->ticket = min(st->ordered, first_cap);
+// The ordered kernel's first ticket: past the core tickets the cluster colored, of kmax (0: none, or
+// streams without them).
+__global__ void k_reset_ticket(DevState *st, unsigned long long *epoch_word, uint32_t kmax = 0) {
+    st->ticket = core_size(st, kmax);
     st->big_leaves = 0;
     if (epoch_word) {
         const unsigned long long e = (*epoch_word + 1) & 0xffffffffull;
@@ -1248,19 +1262,24 @@ gc_status core_cluster_config(gc_ctx *ctx) {
     return GC_OK;
 }
 
-// Core tickets wanted for a coloring.  The clique of hubs must come first in the ticket order and be large:
-// none up to 65,536 vertices (sort to leaves, without / with a core: R-MAT 50,000 x 10 LF 134 / 149 us, FF 124 /
-// 146, 20,000 x 24 146 / 151, 131 / 149; 100,003 x 16 217 / 178, 171 / 181; 300,007 x 32 358 / 257, 336 / 302; 2^22
-// x 32 1,515 / 1,167, 2,870 / 2,575; batches of 8,000 vertices 123 / 149, 132 / 159) and none by GNN keys, which
-// spread the hubs' order over chains that the ticket kernel follows as fast beside all else (GNN3, same graphs
-// 189 / 208, 194 / 211, 230 / 254, 362 / 391, 1,550 / 1,691; GNN2 100,003 246 / 233, 2^22 1,248 / 1,280).  A
-// large batch is quicker with one under every heuristic (64 graphs, 2.2 M vertices, GNN2 2,250 / 2,200).
-constexpr uint32_t CORE_DEFAULT = 2048, CORE_MIN_N = 65536;
+// Core tickets wanted for a coloring.  None up to 65,536 vertices, whose clique of hubs is small (sort to
+// leaves, without / with a core: R-MAT 50,000 x 10 LF 129 / 148 us, FF 118 / 141, 20,000 x 24 141 / 149, 132 / 148;
+// 100,003 x 16 179 / 179, 157 / 180; 300,007 x 32 LF 342 / 264; 2^22 x 32 1,517 / 1,188; batches of 8,000 vertices
+// 123 / 149, 132 / 159).
+// Above that the device decides (core_size): the hubs must come first in the ticket order.  Then the first
+// 2,048 tickets hold a good part of the K^2 / 2 predecessors that a clique would have: R-MAT of 131,072 / 2^20
+// vertices by LF, SL and LLF 0.10 / 0.34, likewise by the weights of a trained GNN (R-MAT 2^11: as LF to 1 %).  By FF
+// it is 0.02 / 0.03, by random GNN weights or random priorities 0.001 to 0.004, and then the ticket kernel
+// follows their chains as fast beside all else (FF 300,007 269 / 310, 2^22 2,545 / 2,600; GNN3 369 / 410, 1,521
+// / 1,681; the empty core kernels cost 15).  The line is 2 / CORE_DENSE.  Batches always have a core above
+// 2^19 vertices and none below (without / with: 20 graphs, 163,000 vertices, LF 249 / 283, GNN2 434 / 453; 64 graphs,
+// 2.2 M, LF 1,172 / 1,110, GNN2 2,287 / 2,245).
+constexpr uint32_t CORE_DEFAULT = 2048, CORE_MIN_N = 65536, CORE_MIN_BATCH = 1u << 19;
 
 uint32_t core_tickets(const gc_graph *g) {
     const uint32_t most = g->ctx->jp_core_max;
     if (most != GC_CORE_AUTO) return most;
-    return g->N > CORE_MIN_N && (g->n_seg || g->key_kind != GC_GNN) ? CORE_DEFAULT : 0u;
+    return g->N > (g->n_seg ? CORE_MIN_BATCH : CORE_MIN_N) ? CORE_DEFAULT : 0u;
 }
 
 // The most core tickets, up to kmax, whose replicas and published sets fit the core kernel's shared
@@ -1348,7 +1367,8 @@ gc_status gc_jp_color(gc_graph *g) {
                                                                       g->pc);
             ctx->launches += 2;
         }
-        k_jp_init_colors<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(g->pc, N, g->color);
+        k_jp_init_colors<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(g->pc, N, g->color, ctx->dstate,
+                                                                ctx->jp_core_max != GC_CORE_AUTO || g->n_seg ? CORE_FORCED : 0u);
         ctx->launches++;
     }
     if ((s = gc_check_launch(ctx, "jp split")) != GC_OK) return s;
