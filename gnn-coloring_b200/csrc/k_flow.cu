@@ -20,11 +20,14 @@
 //
 // The queue is FLOW_QUEUES arrays, vertex v in array v mod FLOW_QUEUES, each with its own head and tail
 // counter: a single counter serves an atomic every 0.7 ns, which alone would cost 10 ms for 16.8 M
-// vertices.  FLOW_QUEUES is odd so that the regular strides of a mesh spread over the arrays.  Every
-// vertex is either queued in its array once or gone on with once (the array's skip counter), so an
-// array is done after as many vertices as it has, and warps take its slots in order: a slot below the
+// vertices.  The powers of two have 36 different remainders modulo 37, so the strides of a mesh spread over
+// the arrays (modulo 31 they have five, and the 256^3 stencil took 10.5 ms first fit, now 5.1).  Hundreds of
+// warps wait at an array's end, each for a slot of its own, so consecutive slots lie in different lines: side
+// by side, their polls and stores met in a few lines (256^3 GNN4 9.0 -> 7.5 ms, Erdos-Renyi 400,000 GNN3 184 ->
+// 134 us, 65,536 LF 96 -> 86).  Every vertex is either queued in its array once or gone on with once (the
+// array's skip counter), so an array is done after as many vertices as it has, and warps take its slots in order: a slot below the
 // tail always belongs to a running warp.  Arrays are served by the warps whose number (in the order in
-// which the CTAs start) has that remainder: the first four CTAs that run serve them all, so the kernel
+// which the CTAs start) has that remainder: the first five CTAs that run serve them all, so the kernel
 // advances whatever else occupies the GPU.
 //
 // A CSR that is not symmetric (a caller's mistake that the upload does not check) can leave vertices
@@ -35,17 +38,19 @@
 // What bounds it: on a wavefront the chain of hops.  A hop to the successor a warp goes on with takes 0.63 us
 // (its counter's atomic, then its neighbour ids); one through a queue adds the tail's atomic, the slot's
 // store and poll, so a slot holds where the list begins as well: fetched after the counter word, stencils
-// took up to 15 % longer (256^3 GNN4 10.5 -> 9.0 ms, Erdos-Renyi 400,000 GNN3 229 -> 184 us, 65,536 LF 112 ->
-// 96).  Elsewhere the vertices in flight (one per warp, 2 to 3 us each; 256^3 first fit 6).
+// took up to 15 % longer (256^3 GNN4 10.5 -> 9.0 ms, Erdos-Renyi 400,000 GNN3 229 -> 184 us).
+// Elsewhere the vertices in flight (one per warp, 2 to 3 us each).
 // Measured on a B200, coloring kernels of one job, tickets (sort, cluster core, streams, ticket kernel,
-// leaves) -> dataflow: 256^3 stencil with GNN4 keys 272 -> 9.6 ms, 97 x 61 x 113 stencil first fit
-// 8.9 -> 1.1 ms, random geometric 2^23 GNN4 4.0 -> 2.7 ms, Erdos-Renyi 65,536 LF 0.36 -> 0.11 ms.
+// leaves) -> dataflow: 256^3 stencil with GNN4 keys 272 -> 8.1 ms, 97 x 61 x 113 stencil first fit
+// 8.9 -> 1.1 ms, random geometric 2^23 GNN4 4.0 -> 2.6 ms, Erdos-Renyi 65,536 LF 0.36 -> 0.10 ms.
 // Measured and not kept: eight lanes per vertex and four vertices per warp (hops of 3.3 us: the longer
 // code path of a lane is on the chain), a separate 16-byte record (hops of 1.9 us), a slot taken
 // before the color is stored, four slots taken at once under backlog; ready vertices handed to waiting
 // warps of the same CTA through shared memory (97 x 61 x 113 first fit 1.1 -> 1.4 ms and more: the atomics
 // of many vertices in one SM are slower); lists fetched into L2 when one predecessor is left to start
-// (stencils 5 % faster, the others 1 to 5 % slower).
+// (stencils 5 % faster, the others 1 to 5 % slower); fewer instructions per poll, that is more polls (97 x 61
+// x 113 first fit 1.04 -> 1.31 ms), or sleeps between them (1.7 ms); arrays by a hash of the id (300,000 x 32
+// 9 % slower).
 #include <algorithm>
 
 #include "gc_internal.h"
@@ -53,7 +58,8 @@
 namespace {
 using namespace gc;
 
-constexpr uint32_t FLOW_QUEUES = 31;
+constexpr uint32_t FLOW_QUEUES = 37;
+constexpr uint32_t FLOW_MIN_CTAS = 5;  // a warp for every array
 constexpr uint32_t FLOW_PAD = 32;  // words between counters: one 128-byte line each
 constexpr uint32_t FLOW_CTA = 3 * FLOW_QUEUES * FLOW_PAD;  // the CTAs' start counter
 constexpr uint32_t FLOW_SLOTS = FLOW_CTA + FLOW_PAD;       // first queue slot
@@ -96,12 +102,17 @@ __device__ __forceinline__ unsigned long long *flow_slots(uint32_t *fq) {
     return reinterpret_cast<unsigned long long *>(fq + FLOW_SLOTS);
 }
 
+// Slots that are filled one after the other lie in different lines, since as many warps poll them.
+__device__ __forceinline__ uint32_t flow_place(uint32_t at) {
+    return (at & ~1023u) | (at & 63u) << 4 | (at >> 6 & 15u);
+}
+
 // Queues vertex v, whose list begins at `beg`: slots hold v + 1 and beg, so that the zeroed buffer reads as
 // empty and the list can be fetched along with the counter word.
 __device__ __forceinline__ void flow_push(uint32_t *fq, uint32_t stride, uint32_t v, uint32_t beg) {
     const uint32_t k = v % FLOW_QUEUES;
     const uint32_t at = atomicAdd(flow_tail(fq, k), 1u);
-    if (at < stride) st_relaxed_u64(flow_slots(fq) + (size_t)k * stride + at, (unsigned long long)beg << 32 | (v + 1u));
+    if (at < stride) st_relaxed_u64(flow_slots(fq) + (size_t)k * stride + flow_place(at), (unsigned long long)beg << 32 | (v + 1u));
 }
 
 // Four lanes per vertex, vertices in id order (records, CSR offsets and rows stream).
@@ -154,9 +165,9 @@ __global__ void __launch_bounds__(FLOW_THREADS) k_flow_init(const uint32_t *__re
 
 // Vertices started or queued so far; every lane gets it.
 __device__ __forceinline__ uint32_t flow_progress(uint32_t *fq, int lane) {
-    return __reduce_add_sync(0xffffffffu, lane < (int)FLOW_QUEUES ? ld_relaxed_u32(flow_tail(fq, lane)) +
-                                                                        ld_relaxed_u32(flow_skip(fq, lane))
-                                                                  : 0u);
+    uint32_t n = 0;
+    for (uint32_t k = lane; k < FLOW_QUEUES; k += 32) n += ld_relaxed_u32(flow_tail(fq, k)) + ld_relaxed_u32(flow_skip(fq, k));
+    return __reduce_add_sync(0xffffffffu, n);
 }
 
 // One more fruitless poll of a warp: true when the warp must leave.  After `check` polls the warp
@@ -210,7 +221,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsign
         slot = __shfl_sync(FULL, slot, 0);
         if (slot >= nk) return;
         for (;;) {
-            u1 = __shfl_sync(FULL, lane == 0 ? ld_relaxed_u64(slots + slot) : 0ull, 0);
+            u1 = __shfl_sync(FULL, lane == 0 ? ld_relaxed_u64(slots + flow_place(slot)) : 0ull, 0);
             if (u1) break;
             if ((fw.spins & 7u) == 7u && slot + min(nk, __shfl_sync(FULL, lane == 0 ? ld_relaxed_u32(skip) : 0u, 0)) >= nk) return;
             if (fw.give_up(fq, st, check, lane)) return;
@@ -328,13 +339,13 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
     }
     {
         ProfScope ps(ctx, "jp_flow", ctx->stream);
-        // at least four CTAs (a warp for every array); a warp per four vertices at most; up to FLOW_FEW_N
+        // at least FLOW_MIN_CTAS; a warp per four vertices at most; up to FLOW_FEW_N
         // vertices half of what fits, since the chains are then all there is and idle warps' polls slow them
         // (8 / 4 per SM, one slot's list fetched later: Erdos-Renyi 65,536 LF 113 / 102 us, GNN3 128 / 115, random
         // geometric 200,000 108 / 99; 500,000 149 / 195, Erdos-Renyi 600,000 226 / 279)
         const int per_sm = std::min(occ, N <= FLOW_FEW_N ? std::max(1, ctx->flow_ctas_per_sm / 2) : ctx->flow_ctas_per_sm);
         const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)per_sm;
-        const uint32_t blocks = std::max<uint32_t>(4u, std::min<uint32_t>(most, (N + 31) / 32));
+        const uint32_t blocks = std::max<uint32_t>(FLOW_MIN_CTAS, std::min<uint32_t>(most, (N + 31) / 32));
         k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->M, g->color, g->flow_q, N, stride,
                                                                ctx->dstate, std::min<uint32_t>(ctx->spin_limit, 1u << 16));
     }
@@ -361,9 +372,9 @@ gc_status gc_jp_flow(gc_graph *g) {
     gc_ctx *ctx = g->ctx;
     gc_status s;
     const bool wide = g->max_deg >= 64;
-    const uint32_t stride = (g->N + FLOW_QUEUES - 1) / FLOW_QUEUES;
+    const uint32_t stride = ((g->N + FLOW_QUEUES - 1) / FLOW_QUEUES + 1023u) & ~1023u;
     if ((s = gc_alloc(ctx, &g->jprec, g->cap_N, "vertex records")) != GC_OK) return s;
     if (wide && (s = gc_alloc(ctx, &g->jpsplit, g->cap_N, "vertex records")) != GC_OK) return s;
-    if ((s = gc_alloc(ctx, &g->flow_q, 2 * ((size_t)g->cap_N + FLOW_QUEUES) + FLOW_SLOTS, "flow queues")) != GC_OK) return s;
+    if ((s = gc_alloc(ctx, &g->flow_q, 2 * ((size_t)g->cap_N + 1024 * FLOW_QUEUES) + FLOW_SLOTS, "flow queues")) != GC_OK) return s;
     return wide ? flow_run<FLOW_WIDE>(g, stride) : g->max_deg >= 32 ? flow_run<2>(g, stride) : flow_run<1>(g, stride);
 }
