@@ -355,13 +355,13 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
 
 }  // namespace
 
-// Which graphs go by dataflow: a maximum degree below 64 always (Erdos-Renyi of mean degree 16 to 24 and
-// 0.2 to 4 M vertices, whole call: 0.20 to 1.74 ms against 0.44 to 2.01 with tickets); below 128 up to
-// FLOW_WIDE_MAX_N vertices, since the wide kernel keeps half as many vertices in flight (mean degree
-// 32, 0.5 M vertices: 0.59 against 0.71 ms; 1 M: 1.15 against 1.02).  Larger degrees would put long
+// Which graphs go by dataflow: a maximum degree below 64 always (whole calls, largest degree first, dataflow /
+// tickets: Erdos-Renyi 200,000 x 16 167 / 281 us, 1 M x 24 545 / 1,038, 4 M x 16 1,607 / 3,459); below 128 up to
+// FLOW_WIDE_MAX_N vertices, the largest size measured, since the wide kernel keeps half as many vertices in
+// flight (250,000 x 40 363 / 397, 500,000 x 34 461 / 639, 1 M x 34 939 / 1,185).  Larger degrees would put long
 // lists on the chain, and power-law graphs have their chains colored inside one cluster (k_jp_core).
 // Plain graphs only: a batch is captured, and the stall flag needs the host.
-constexpr uint32_t FLOW_WIDE_MAX_N = 1u << 19;
+constexpr uint32_t FLOW_WIDE_MAX_N = 1u << 20;
 
 bool gc_flow_eligible(const gc_graph *g) {
     const uint32_t widest = g->N <= FLOW_WIDE_MAX_N ? 32u * FLOW_WIDE : 64u;

@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__re
 // Graphs whose CSR and working arrays fit one SM's shared memory, up to the sizes at which one SM's
 // instruction rate costs more than the other kernels' latency.  Against the dataflow kernel that is a matter
 // of vertices (calls with first fit or largest degree first, other kernels / this one: Erdos-Renyi 1,000 x 16
-// 94 / 53 us, 2,000 x 16 97 / 67, 3,000 x 24 126 / 113, 4,096 x 12 83 / 92, 8,192 x 7 75 / 98; with two rounds
-// 211 / 85, 214 / 113, 270 / 204, 221 / 175, 202 / 207), against the ticket kernels, whose graphs have long lists
+// 88 / 55 us, 2,000 x 16 90 / 71, 3,000 x 24 119 / 109, 4,000 x 12 79 / 87, 6,000 x 8 68 / 93; with two rounds
+// 201 / 89, 208 / 120, 264 / 200, 210 / 168, 203 / 186), against the ticket kernels, whose graphs have long lists
 // and many levels, one of entries (R-MAT 1,000 x 16, 12,000 entries 125 / 86, 1,000 x 32, 21,000 128 / 119, 1,400
 // x 32, 28,000 124 / 145; with two rounds 274 / 164, 320 / 223, 312 / 278, 4,000 x 16, 52,000 371 / 447).
 bool gc_small_eligible(const gc_graph *g, int rounds) {
