@@ -387,6 +387,7 @@ gc_status gc_ctx_create(int device, gc_ctx **out) {
     if (const char *e = getenv("GC_JP_TIGHT")) ctx->jp_tight = (unsigned int)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_FLOW")) ctx->flow_max_deg = (uint32_t)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_FLOW_CTAS")) ctx->flow_ctas_per_sm = std::max(1, atoi(e));
+    if (const char *e = getenv("GC_JP_FLOW_LIMIT")) ctx->flow_limit = (unsigned int)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_SMALL")) ctx->small_max = (uint32_t)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_CLASSES")) ctx->jp_classes = atoi(e) != 0;
     if (const char *e = getenv("GC_JP_DECIDE")) ctx->jp_decide = atoi(e) != 0;

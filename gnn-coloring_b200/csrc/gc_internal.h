@@ -57,6 +57,7 @@ struct gc_ctx {
     bool jp_decide = true;               // coloring: early decisions from published forbidden colors
     uint32_t flow_max_deg = 128;         // coloring: graphs with a smaller maximum degree go by dataflow (0: none; GC_JP_FLOW)
     int flow_ctas_per_sm = 8;            // dataflow kernel: CTAs per SM at most (GC_JP_FLOW_CTAS)
+    unsigned int flow_limit = 1u << 16;  // dataflow kernel: fruitless polls before a warp looks whether anything moves (GC_JP_FLOW_LIMIT)
     uint32_t small_max = GC_SMALL_AUTO;  // coloring: graphs of up to this many vertices that fit go in one CTA (0: none; GC_JP_SMALL)
     bool small_ready = false;            // that kernel's shared-memory limit is set
     int round_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each Culberson kernel

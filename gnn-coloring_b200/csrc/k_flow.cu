@@ -347,7 +347,7 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
         const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)per_sm;
         const uint32_t blocks = std::max<uint32_t>(FLOW_MIN_CTAS, std::min<uint32_t>(most, (N + 31) / 32));
         k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->M, g->color, g->flow_q, N, stride,
-                                                               ctx->dstate, std::min<uint32_t>(ctx->spin_limit, 1u << 16));
+                                                               ctx->dstate, std::min(ctx->spin_limit, ctx->flow_limit));
     }
     ctx->launches += 2;
     return gc_check_launch(ctx, "jp flow");
