@@ -13,6 +13,11 @@
 // Eight lanes per vertex; 32 in levels of up to 32 vertices and for more than HEAVY neighbours, which are
 // queued from the other end of q.
 //
+// That reading of "colored" needs a symmetric CSR: with one-sided entries a vertex could start before a
+// predecessor, and its color would follow the warps' timing.  So the first counting pass also adds up a hash of
+// every entry (u, v) that is the negative of (v, u)'s.  The sum of a symmetric CSR is zero; any other graph's is
+// not (but for a chance of 2^-32), and the other kernels, which ask each entry who precedes, color it.
+//
 // What bounds it: a level's serial chain, about 1,400 cycles (barrier, queue, list, colors, two shared atomics),
 // and in wide levels the SM's instruction rate.  Erdos-Renyi 1,000 x 16 first fit (36 levels): 71,000 cycles,
 // 4,800 of them loading, 54,500 levels; the call 94 -> 53 us.  512 threads 59 us, 256 threads 65.  Eight lanes
@@ -134,10 +139,19 @@ __device__ __forceinline__ void color_vertex(const Small &s, uint32_t u, bool va
     if (valid && gl == 0) s.a(u) = (uint16_t)c;
 }
 
+// A hash of the entry (u, v), the negative of that of (v, u): the pair by multiplicative hashing (Knuth, The
+// Art of Computer Programming 3, 6.4) twice, signed by its order.  A self-loop counts as symmetric.
+__device__ __forceinline__ uint32_t entry_hash(uint32_t u, uint32_t v) {
+    uint32_t h = (min(u, v) << 16 | max(u, v)) * 0x9e3779b9u;
+    h = (h ^ h >> 15) * 0x9e3779b9u;
+    h ^= h >> 16;
+    return u < v ? h : u > v ? 0u - h : 0u;
+}
+
 __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__restrict__ V, const uint32_t *__restrict__ E,
                                                             uint32_t *key, uint32_t N, uint32_t M, int rounds, bool stats,
                                                             int *__restrict__ color, DevState *state) {
-    __shared__ uint32_t invalid, top;
+    __shared__ uint32_t invalid, top, sides;  // sides: the entries' hashes, zero for a symmetric CSR
     Small s;
     s.N = N;
     s.rem_ = HEAD + N + 1;
@@ -158,17 +172,28 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__re
             if (i + k * blockDim.x < M) s.ids(i + k * blockDim.x) = (uint16_t)v[k];
     }
     if (t < 3) s.light(t) = s.heavy(t) = 0;
-    if (t == 0) invalid = top = 0;
+    if (t == 0) invalid = top = sides = 0;
     bool done = true;
+    uint32_t hashes = 0;
     for (int it = 0; it <= rounds; it++) {
         __syncthreads();
         auto found = [&](uint32_t u, uint32_t cnt, bool big) {
             s.rem(u) = cnt | (big ? BIG : 0u);
             if (cnt == 0) push(s, u, big, 0, 0, 0);
         };
-        if (it == 0) for_vertices(s, [&](uint32_t u, uint32_t v) { return precedes(ks[v], v, ks[u], u) ? 1u : 0u; }, found);
-        else for_vertices(s, [&](uint32_t u, uint32_t v) { return precedes(s.b(v), v, s.b(u), u) ? 1u : 0u; }, found);
+        if (it == 0) {
+            for_vertices(s, [&](uint32_t u, uint32_t v) {
+                hashes += entry_hash(u, v);
+                return precedes(ks[v], v, ks[u], u) ? 1u : 0u;
+            }, found);
+            hashes = __reduce_add_sync(FULL, hashes);
+            if (lane == 0) atomicAdd(&sides, hashes);
+        } else for_vertices(s, [&](uint32_t u, uint32_t v) { return precedes(s.b(v), v, s.b(u), u) ? 1u : 0u; }, found);
         __syncthreads();
+        if (sides) {
+            done = false;
+            break;
+        }
         if (it == 0)
             for (uint32_t i = t; i < N; i += blockDim.x) ks[i] = 0;  // (both color arrays)
         uint32_t la = 0, ha = 0;

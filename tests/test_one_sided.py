@@ -1,0 +1,68 @@
+"""CSRs that are not symmetric, against the library's contract: where a call succeeds all the same, each vertex has the
+smallest color that no neighbour of its own list that precedes it has, whichever kernel colored it."""
+import os
+
+import numpy as np
+import pytest
+
+import gnn_coloring as gcn
+
+pytestmark = pytest.mark.gpu
+
+
+def _csr(lists):
+    V = np.concatenate([[0], np.cumsum([len(x) for x in lists])]).astype(np.uint32)
+    return len(lists), V, np.concatenate([np.sort(np.asarray(x, np.uint32)) for x in lists]).astype(np.uint32)
+
+
+def _colors_by_own_lists(N, V, E, p):
+    color = np.zeros(N, np.int64)
+    for u in np.lexsort((np.arange(N), -p)):
+        v = E[V[u]:V[u + 1]].astype(np.int64)
+        before = v[(p[v] > p[u]) | ((p[v] == p[u]) & (v < u))]
+        taken = set(color[before].tolist())
+        color[u] = next(c for c in range(1, N + 2) if c not in taken)
+    return color
+
+
+def _lists(N, V, E):
+    return [E[V[u]:V[u + 1]].tolist() for u in range(N)]
+
+
+def test_a_vertex_named_by_one_that_it_does_not_name():
+    """Vertex 41 ends a path and waits for it; vertex 42 names 41 and precedes it, one-sidedly."""
+    lists = [[v for v in (u - 1, u + 1) if 0 <= v < 42] for u in range(42)] + [[41]] + [[] for _ in range(21)]
+    N, V, E = _csr(lists)
+    p = np.arange(N, 0, -1).astype(np.float64)
+    p[42] = 100.0
+    want = _colors_by_own_lists(N, V, E, p)
+    ctx = gcn.Context(int(os.environ.get("GC_DEVICE", "0")))
+    g = gcn.Graph(ctx, N, V, E)
+    for _ in range(3):
+        g.set_priority(p)
+        g.color(count=False)
+        assert np.array_equal(g.colors(), want)
+    g.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_entries_added_on_one_side(seed):
+    """Extra entries from vertices to later ones: nobody's own predecessors change."""
+    N, V, E = gcn.gen_er(900, 900 * (2 + seed), 10 + seed)
+    lists, rng = _lists(N, V, E), np.random.default_rng(seed)
+    for u, v in rng.integers(0, N, (1 << seed, 2)):
+        u, v = min(u, v), max(u, v)
+        if u != v and int(v) not in lists[u]:
+            lists[u].append(int(v))
+    N, V, E = _csr(lists)
+    p = np.arange(N, 0, -1).astype(np.float64)  # first fit: smaller ids precede
+    want = _colors_by_own_lists(N, V, E, p)
+    ctx = gcn.Context(int(os.environ.get("GC_DEVICE", "0")))
+    g = gcn.Graph(ctx, N, V, E)
+    for _ in range(2):
+        g.priority("FF")
+        g.color(count=False)
+        assert np.array_equal(g.colors(), want)
+    g.close()
+    ctx.close()
