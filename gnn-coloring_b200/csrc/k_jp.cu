@@ -539,10 +539,12 @@ __device__ __forceinline__ void core_st_remote(const unsigned short *p, unsigned
 // Pre-pass, one warp per core ticket t < K: the predecessor list P[first, first + count) becomes the
 // ranks of its inner predecessors (compacted in place, CSR order kept), rec[t].z their number and
 // rec[t].w = (all predecessors, at most 65,535) << 1 | (1 when a source, color 1 from the split, is
-// among them).
+// among them).  A predecessor that is neither a source nor an earlier ticket (a leaf, which precedes nobody in a
+// symmetric CSR) has no rank: rank[] then holds anything, so a rank counts only when that ticket is the
+// predecessor's, and the coloring ends with an error otherwise.
 __global__ void __launch_bounds__(256) k_jp_core_lists(uint4 *__restrict__ rec, uint32_t *__restrict__ P,
                                                        const uint32_t *__restrict__ rank, const int *__restrict__ color,
-                                                       const DevState *st, uint32_t kmax) {
+                                                       DevState *st, uint32_t kmax) {
     const uint32_t K = core_size(st, kmax);
     const int lane = threadIdx.x & 31;
     const unsigned int lt = (1u << lane) - 1u;
@@ -558,7 +560,8 @@ __global__ void __launch_bounds__(256) k_jp_core_lists(uint4 *__restrict__ rec, 
             if (j < r.z) {
                 const uint32_t v = P[r.y + j];
                 if (color[v] == 1) source = true;
-                else inner = true, rk = rank[v];
+                else if ((rk = rank[v]) < t && rec[rk].x == v) inner = true;
+                else raise_error(st, ERR_ORDER, r.x);
             }
             const unsigned int m = __ballot_sync(0xffffffffu, inner);
             __syncwarp();  // every lane has read its entry before any is overwritten

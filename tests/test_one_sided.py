@@ -66,3 +66,33 @@ def test_entries_added_on_one_side(seed):
         assert np.array_equal(g.colors(), want)
     g.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("core", ["8", "64", "32768"])
+def test_core_ticket_that_waits_for_a_leaf(core):
+    """Vertex 1 of a path names vertex 50, which precedes it but names only vertex 60: a leaf, without a ticket.  The
+    coloring fails with a status, and the context stays usable."""
+    lists = [[v for v in (u - 1, u + 1) if 0 <= v < 40] for u in range(40)] + [[] for _ in range(60)]
+    lists[1].append(50)
+    lists[50], lists[60] = [60], [50]
+    N, V, E = _csr(lists)
+    p = np.arange(N, 0, -1).astype(np.float64)
+    p[60], p[50] = 300.0, 200.0
+    env = dict(GC_JP_SMALL="0", GC_JP_FLOW="0", GC_JP_CORE=core, GC_SPIN_LIMIT="1000")
+    os.environ.update(env)
+    ctx = gcn.Context(int(os.environ.get("GC_DEVICE", "0")))
+    for k in env:
+        del os.environ[k]
+    g = gcn.Graph(ctx, N, V, E)
+    g.set_priority(p)
+    with pytest.raises(gcn.GCError) as e:
+        g.color()
+    assert e.value.name == "GC_ERR_DEVICE"
+    g.close()
+    N, V, E = gcn.gen_er(500, 2000, 1)
+    g = gcn.Graph(ctx, N, V, E)
+    g.priority("LF")
+    g.color()
+    assert np.array_equal(g.colors(), _colors_by_own_lists(N, V, E, g.priorities()))
+    g.close()
+    ctx.close()
