@@ -69,8 +69,11 @@ constexpr uint32_t FLOW_FEW_N = 1u << 18;
 // A vertex's counter word: rem in bits 48..63, the degree in bits 32..47, the first CSR entry below.
 // The subtraction that makes a successor ready so returns where its neighbour list is, and the list is
 // on its way one load earlier.  rem is the top field: one subtraction too many (a self-loop, a CSR that
-// is not symmetric) wraps there and leaves the others alone.
+// is not symmetric) wraps there and leaves the others alone.  A vertex that thousands name one-sidedly would become
+// ready a second time, take another's place in its array, and leave that one without a color: the subtraction
+// that finds FLOW_ASKEW in rem stops the kernel long before.
 constexpr unsigned long long FLOW_ONE = 1ull << 48;
+constexpr uint32_t FLOW_ASKEW = 0x8000u;
 // W words of 32 mask bits per vertex (bit j of word w: neighbour 32 w + j precedes).
 constexpr int FLOW_WIDE = 4;
 template <int W>
@@ -262,7 +265,9 @@ __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsign
             bool more = false;
 #pragma unroll
             for (int w = 0; w < W; w++) {
-                bool ready = (uint32_t)(old[w] >> 48) == 1u;
+                const uint32_t left = (uint32_t)(old[w] >> 48);
+                bool ready = left == 1u;
+                if (left == FLOW_ASKEW) st_relaxed_u32(&st->flow_stall, 1u);
                 const unsigned int rm = __ballot_sync(FULL, ready);
                 if (!rm) continue;
                 if (!more) {

@@ -68,6 +68,34 @@ def test_entries_added_on_one_side(seed):
     ctx.close()
 
 
+def test_a_vertex_named_by_more_than_its_counter_holds():
+    """70,000 vertices name vertex 0, which names one of them; the end of a path makes the last vertex of 0's queue
+    array ready once everything else is done."""
+    n, chain = 70000, 3000
+    lists = [[0] for _ in range(n)]
+    a = n - 1
+    lists[0] = [a]
+    ids = [u for u in range(1, n - 1) if u % 37][:chain]  # the path, outside 0's array
+    w, z = 37 * ((n - 200) // 37), n - 3
+    on = next(u for u in range(w - 1, 0, -1) if u % 37)
+    for k, u in enumerate(ids):
+        lists[u] = ids[max(0, k - 1):k] + ids[k + 1:k + 2]
+    lists[ids[-1]] += [on, w]
+    lists[on], lists[w], lists[z] = [ids[-1]], [ids[-1], z], []
+    N, V, E = _csr(lists)
+    p = np.full(N, 2.0)
+    p[ids] = np.arange(chain, 0, -1) + 10.0
+    p[[0, on, w, z]] = 1.0, 1.5, 1.5, 1.0
+    want = _colors_by_own_lists(N, V, E, p)
+    ctx = gcn.Context(int(os.environ.get("GC_DEVICE", "0")))
+    g = gcn.Graph(ctx, N, V, E)
+    g.set_priority(p)
+    g.color(count=False)
+    assert np.array_equal(g.colors(), want)
+    g.close()
+    ctx.close()
+
+
 @pytest.mark.parametrize("core", ["8", "64", "32768"])
 def test_core_ticket_that_waits_for_a_leaf(core):
     """Vertex 1 of a path names vertex 50, which precedes it but names only vertex 60: a leaf, without a ticket.  The
