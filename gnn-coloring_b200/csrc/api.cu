@@ -284,7 +284,7 @@ gc_status color_by_keys(gc_ctx *ctx, gc_graph *g, bool *unread) {
     if (!*unread) return gc_jp_color(g);
     gc_status s = gc_jp_flow(g);
     if (s != GC_OK) return s;
-    g->has_colors = true;
+    g->has_colors = false;  // (until the state has been read)
     g->colors_ours = true;
     return GC_OK;
 }
@@ -339,8 +339,15 @@ gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *co
         if ((s = color_by_tickets(ctx, g)) != GC_OK) return s;
         unread = false;
     }
+    g->has_colors = true;
     if (colors_used) g->colors_used = *colors_used = gc_colors_of_state(g);
     return GC_OK;
+}
+
+// A coloring that a device error ended is no coloring.
+gc_status checked(gc_graph *g, gc_status s) {
+    if (s == GC_ERR_DEVICE || s == GC_ERR_CUDA) g->has_colors = false;
+    return s;
 }
 
 }  // namespace
@@ -748,14 +755,14 @@ gc_status gc_color(gc_ctx *ctx, gc_graph *g, int recolor, int *colors_used) {
     if (!ctx || !g || g->ctx != ctx || recolor < 0) return GC_ERR_INVALID;
     if (!g->has_keys) return gc_fail(ctx, GC_ERR_STATE, "no priorities: call gc_priority or gc_priority_set first");
     DeviceGuard dg(ctx);
-    return color_rounds(ctx, g, true, recolor, colors_used);
+    return checked(g, color_rounds(ctx, g, true, recolor, colors_used));
 }
 
 gc_status gc_recolor(gc_ctx *ctx, gc_graph *g, int iters, int *colors_used) {
     if (!ctx || !g || g->ctx != ctx || iters < 0) return GC_ERR_INVALID;
     if (!g->has_colors) return gc_fail(ctx, GC_ERR_STATE, "no coloring to recolor");
     DeviceGuard dg(ctx);
-    return color_rounds(ctx, g, false, iters, colors_used);
+    return checked(g, color_rounds(ctx, g, false, iters, colors_used));
 }
 
 gc_status gc_validate(gc_ctx *ctx, gc_graph *g, int *max_color) {

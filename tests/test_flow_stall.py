@@ -70,3 +70,19 @@ def test_stopped_dataflow_is_colored_by_tickets(name, classes):
     g.close()
     ctx.close()
 
+
+def test_failed_coloring_leaves_no_colors(monkeypatch):
+    """Dataflow and tickets both give up (wait limit 0): the colors written so far are not a coloring."""
+    monkeypatch.setenv("GC_SPIN_LIMIT", "0")
+    ctx = _context()
+    N, V, E = _path(200000)
+    g = gcn.Graph(ctx, N, V, E)
+    g.priority("FF")
+    with pytest.raises(gcn.GCError) as e:
+        g.color()
+    assert e.value.name == "GC_ERR_DEVICE"
+    with pytest.raises(gcn.GCError) as e:
+        g.colors()
+    assert e.value.name == "GC_ERR_STATE"
+    g.close()
+    ctx.close()
