@@ -51,8 +51,8 @@ __global__ void k_simple_keys(const uint32_t *__restrict__ V, uint32_t N, int h,
 //     removed vertex's degree again), so nothing waits for their results.
 //   - SL tries delta + 1 first; only when that removes nothing does it look for the smallest remaining
 //     degree (one more barrier).
-//   - The barrier's counter and the round's count are one 16-byte word, polled together by one thread
-//     per CTA.
+//   - The barrier's counter and the round's count are one 64-bit word, polled by one thread per CTA: a scalar
+//     that only atomics change, so whoever reads the last arrival reads the final count.
 // Measured (B200), three launches per round queued in batches -> this: SL on R-MAT of 2^20 vertices and
 // edge factor 16 (217 rounds) 8.2 -> 1.6 ms, on Erdos-Renyi 65,536 (16 rounds) 0.41 -> 0.09 ms.  With two
 // barriers in every round and long lists shared by the grid: 1.9 and 0.10.  Rounds that remove thousands
@@ -66,9 +66,15 @@ constexpr uint32_t PEEL_WARP_DEG = 64;
 constexpr uint32_t PEEL_WIDE = 512;
 constexpr unsigned int PEEL_WAIT_LIMIT = 1u << 24;  // polls of one barrier
 
+struct PeelSlot {
+    unsigned long long word;  // arrivals at the filter's barrier; above bit 32 the removed vertices on the short
+                              // list (or kept by their warps)
+    unsigned int longs;       // removed vertices on the long list
+    unsigned int packed;      // remaining vertices on the next list
+};
+
 struct PeelState {
-    uint4 slot[3];         // round r in slot r mod 3, cleared a round ahead: arrivals at the filter's barrier,
-                           // removed vertices on the short list (or kept by their warps), on the long list, packed
+    PeelSlot slot[3];      // round r in slot r mod 3, cleared a round ahead
     unsigned int pad0[20];
     unsigned int arrived;  // arrivals at the other barriers so far
     unsigned int pad1[31];
@@ -86,13 +92,8 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ uint4 ld_relaxed_v4(const uint4 *p) {
-    uint4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p)
-                 : "memory");
-    return v;
+__device__ __forceinline__ void red_release_u64(unsigned long long *p) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(p) : "memory");
 }
 __device__ __forceinline__ bool peel_expired(PeelState *ps, unsigned int &spins) {
     return ++spins > PEEL_WAIT_LIMIT || ((spins & 255u) == 0 && gc::ld_relaxed_u32(&ps->failed));
@@ -100,27 +101,33 @@ __device__ __forceinline__ bool peel_expired(PeelState *ps, unsigned int &spins)
 
 // Grid barriers: every CTA's earlier writes are visible to all after them.  False when the wait expired
 // (in some CTA).  One thread per CTA polls (thousands of warps asking one address would queue for
-// microseconds).  The first kind arrives at a round's slot and returns it: its counts are complete when
-// all CTAs have arrived, since each adds to them before it arrives.
-__device__ __forceinline__ bool peel_slot_barrier(PeelState *ps, uint4 *slot, uint4 &got) {
+// microseconds).  The first kind arrives at a round's slot and returns its counts, which are complete when
+// all CTAs have arrived, since each adds to them before it arrives; those of the lists are read on request.
+struct PeelCounts {
+    uint32_t removed, longs, packed;
+};
+
+template <bool LISTS>
+__device__ __forceinline__ bool peel_slot_barrier(PeelState *ps, PeelSlot *slot, PeelCounts &got) {
     __shared__ uint4 got_s;
     __syncthreads();
     if (threadIdx.x == 0) {
-        red_release(&slot->x);
-        unsigned int spins = 0;
-        uint4 v;
-        while ((v = ld_relaxed_v4(slot)).x != gridDim.x)
+        red_release_u64(&slot->word);
+        unsigned int spins = 0, good = 1;
+        unsigned long long v;
+        while ((uint32_t)(v = gc::ld_relaxed_u64(&slot->word)) != gridDim.x)
             if (peel_expired(ps, spins)) {
                 gc::st_relaxed_u32(&ps->failed, 1u);
-                v.x = 0;
+                good = 0;
                 break;
             }
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        got_s = v;
+        got_s = make_uint4(good, (uint32_t)(v >> 32), LISTS ? gc::ld_relaxed_u32(&slot->longs) : 0u,
+                           LISTS ? gc::ld_relaxed_u32(&slot->packed) : 0u);
     }
     __syncthreads();
-    got = got_s;
-    return got.x != 0;
+    got = PeelCounts{got_s.y, got_s.z, got_s.w};
+    return got_s.x != 0;
 }
 // `read`: a word to return in `value` (may be null).
 __device__ __forceinline__ bool peel_barrier(PeelState *ps, unsigned int &target, const unsigned int *read, unsigned int &value) {
@@ -201,11 +208,11 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
     uint32_t alive = N, len = N, r = 0;
     uint32_t *cur = list0, *other = list1;
     uint32_t u[ITEMS], d[ITEMS], beg[ITEMS], end[ITEMS];
-    uint4 got;
+    PeelCounts got;
     bool done = false;
     auto round_end = [&]() {  // once the decrements are out; the slots of the round after next are free
         if (tid == 0) {
-            ps->slot[(r + 2) % 3] = make_uint4(0u, 0u, 0u, 0u);
+            ps->slot[(r + 2) % 3] = PeelSlot{0ull, 0u, 0u};
             ps->min_deg[(r + 2) % 3] = NO_DEGREE;
         }
         return peel_barrier(ps, target, nullptr, value);
@@ -224,7 +231,7 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
     };
     // ---- the remaining vertices on a list
     for (bool pack = false; len > threads * ITEMS; r++) {
-        uint4 *sl = &ps->slot[r % 3];
+        PeelSlot *sl = &ps->slot[r % 3];
         const uint32_t thr = threshold();
         // short: at most 16 neighbours for each of the lanes a vertex is sure to get in the decrement (a
         // removed vertex has about as many neighbours as the threshold)
@@ -259,8 +266,8 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
             }
             if (shorts | longs) {
                 uint32_t at = 0;
-                if (lane == 0 && shorts) at = atomicAdd(&sl->y, shorts);
-                if (lane == 1 && longs) at = atomicAdd(&sl->z, longs);
+                if (lane == 0 && shorts) at = (uint32_t)(atomicAdd(&sl->word, (unsigned long long)shorts << 32) >> 32);
+                if (lane == 1 && longs) at = atomicAdd(&sl->longs, longs);
                 uint32_t as = __shfl_sync(FULL, at, 0), al = __shfl_sync(FULL, at, 1);
 #pragma unroll
                 for (int k = 0; k < ITEMS; k++) {
@@ -274,7 +281,7 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
             }
             if (pack && kept) {
                 uint32_t at = 0;
-                if (lane == 0) at = atomicAdd(&sl->w, kept);
+                if (lane == 0) at = atomicAdd(&sl->packed, kept);
                 at = __shfl_sync(FULL, at, 0);
 #pragma unroll
                 for (int k = 0; k < ITEMS; k++) {
@@ -285,10 +292,10 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
                 }
             }
         }
-        if (!peel_slot_barrier(ps, sl, got)) return;
-        const uint32_t ns = got.y, nl = got.z;
+        if (!peel_slot_barrier<true>(ps, sl, got)) return;
+        const uint32_t ns = got.removed, nl = got.longs;
         if (pack) {
-            len = got.w;
+            len = got.packed;
             uint32_t *t = cur;
             cur = other;
             other = t;
@@ -332,7 +339,7 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
         if (!peel_barrier(ps, target, nullptr, value)) return;  // (nothing is counted down before all have read)
     }
     for (; !done; r++) {
-        uint4 *sl = &ps->slot[r % 3];
+        PeelSlot *sl = &ps->slot[r % 3];
         const uint32_t thr = threshold();
         const uint32_t *past = (r & 1) ? deg : other;
         uint32_t *count = (r & 1) ? other : deg;
@@ -361,7 +368,7 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
             out_n += __popc(__ballot_sync(FULL, out));
             cnt += __popc(__ballot_sync(FULL, (rm >> k) & 1u));
         }
-        if (lane == 0 && out_n) atomicAdd(&sl->y, out_n);
+        if (lane == 0 && out_n) atomicAdd(&sl->word, (unsigned long long)out_n << 32);
         if (cnt) {  // the warp's own: their lists packed, eight lanes each
             uint2 *mine = own[threadIdx.x >> 5];
             uint32_t at = 0;
@@ -384,16 +391,16 @@ __global__ void __launch_bounds__(PEEL_THREADS, 1) k_peel(const uint32_t *__rest
         }
         if (threadIdx.x == 0) wide_n[(r + 1) & 1] = 0;
         if (tid == 0) {  // the next round's slot: every CTA has left the barrier of the round before last
-            ps->slot[(r + 1) % 3] = make_uint4(0u, 0u, 0u, 0u);
+            ps->slot[(r + 1) % 3] = PeelSlot{0ull, 0u, 0u};
             ps->min_deg[(r + 1) % 3] = NO_DEGREE;
         }
-        if (!peel_slot_barrier(ps, sl, got)) return;
-        alive -= got.y;
+        if (!peel_slot_barrier<false>(ps, sl, got)) return;
+        alive -= got.removed;
         if (alive == 0) {
             r++;
             break;
         }
-        if (got.y == 0 && !log_mode) {
+        if (got.removed == 0 && !log_mode) {
             if (!grid_min(low, &ps->min_deg[r % 3])) return;
             delta = max(delta, value);
         } else {
