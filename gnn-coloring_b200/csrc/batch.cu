@@ -106,6 +106,7 @@ struct gc_batch {
     int32_t *h_stat = nullptr;      // pinned copy of the per-graph statistics (2 * cap_G)
     std::vector<BatchCapture> caps;
     gc_tuning tuning{};
+    bool hub_auto = true, gnn_warp_auto = true;  // those two by the batch's size, until a tuning sets them
 };
 
 namespace {
@@ -193,6 +194,8 @@ gc_status finish_batch_upload(gc_batch *b, uint32_t G, const uint32_t *voff_host
     g->warp_deg = b->tuning.warp_degree;
     g->gnn_warp_deg = b->tuning.gnn_warp_degree;
     g->hub_deg = b->tuning.hub_degree;
+    g->gnn_warp_auto = b->gnn_warp_auto;
+    g->hub_auto = b->hub_auto;
     g->sched = b->tuning.schedule;
     g->jp_ctas = b->tuning.jp_ctas_per_sm;
     g->jp_tight = b->tuning.jp_tight;
@@ -359,11 +362,21 @@ gc_status capture(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor, B
     return s;
 }
 
-gc_status apply_tuning(gc_batch *b, const gc_tuning &t) {
+// A tuning, and which of its thresholds the batch's size decides instead.
+struct Candidate {
+    gc_tuning t;
+    bool hub_auto, gnn_warp_auto;
+};
+
+gc_status apply_tuning(gc_batch *b, const Candidate &c) {
     gc_graph *g = b->g;
-    const bool reprepare = t.warp_degree != g->warp_deg || t.hub_degree != g->hub_deg || t.schedule != g->sched ||
-                           t.gnn_warp_degree != g->gnn_warp_deg;
+    const gc_tuning &t = c.t;
+    const bool reprepare = t.warp_degree != g->warp_deg || t.schedule != g->sched ||
+                           (c.hub_auto ? !g->hub_auto : t.hub_degree != g->hub_now) ||
+                           (c.gnn_warp_auto ? !g->gnn_warp_auto : t.gnn_warp_degree != g->gnn_warp_now);
     b->tuning = t;
+    b->hub_auto = g->hub_auto = c.hub_auto;
+    b->gnn_warp_auto = g->gnn_warp_auto = c.gnn_warp_auto;
     drop_captures(b);
     g->warp_deg = t.warp_degree;
     g->gnn_warp_deg = t.gnn_warp_degree;
@@ -658,12 +671,14 @@ gc_status gc_batch_set_tuning(gc_ctx *ctx, gc_batch *b, const gc_tuning *t) {
     if (!ctx || !b || b->ctx != ctx || !t) return GC_ERR_INVALID;
     if (!tuning_valid(*t)) return gc_fail(ctx, GC_ERR_INVALID, "invalid tuning");
     DeviceGuard dg(ctx);
-    return apply_tuning(b, *t);
+    return apply_tuning(b, Candidate{*t, false, false});
 }
 
 gc_status gc_batch_get_tuning(const gc_batch *b, gc_tuning *t) {
     if (!b || !t) return GC_ERR_INVALID;
     *t = b->tuning;
+    if (b->hub_auto) t->hub_degree = b->g->hub_now;
+    if (b->gnn_warp_auto) t->gnn_warp_degree = b->g->gnn_warp_now;
     return GC_OK;
 }
 
@@ -673,10 +688,10 @@ gc_status gc_batch_autotune(gc_ctx *ctx, gc_batch *b, gc_heuristic h, const gc_m
     DeviceGuard dg(ctx);
     gc_status s = check_heuristic(ctx, h, m);
     if (s != GC_OK) return s;
-    gc_tuning best = b->tuning;
+    Candidate best{b->tuning, b->hub_auto, b->gnn_warp_auto};
     double best_ms = INFINITY;
     // one warm pass, then the faster of two timed passes
-    auto measure = [&](const gc_tuning &t, double *ms) -> gc_status {
+    auto measure = [&](const Candidate &t, double *ms) -> gc_status {
         gc_status st = apply_tuning(b, t);
         if (st != GC_OK) return st;
         if ((st = direct_pass(b, h, m, recolor, nullptr, nullptr)) != GC_OK) return st;
@@ -686,11 +701,12 @@ gc_status gc_batch_autotune(gc_ctx *ctx, gc_batch *b, gc_heuristic h, const gc_m
         *ms = std::min(a, c);
         return GC_OK;
     };
-    std::vector<gc_tuning> seen;
-    auto consider = [&](const gc_tuning &t) -> gc_status {
-        if (!tuning_valid(t)) return GC_OK;
-        for (const gc_tuning &o : seen)
-            if (!memcmp(&o, &t, sizeof t)) return GC_OK;
+    std::vector<Candidate> seen;
+    auto consider = [&](const Candidate &t) -> gc_status {
+        if (!tuning_valid(t.t)) return GC_OK;
+        for (const Candidate &o : seen)
+            if (!memcmp(&o.t, &t.t, sizeof t.t) && o.hub_auto == t.hub_auto && o.gnn_warp_auto == t.gnn_warp_auto)
+                return GC_OK;
         seen.push_back(t);
         double ms = 0;
         gc_status st = measure(t, &ms);
@@ -702,59 +718,60 @@ gc_status gc_batch_autotune(gc_ctx *ctx, gc_batch *b, gc_heuristic h, const gc_m
         return GC_OK;
     };
     if (b->g->N == 0) {
-        if (best_out) *best_out = best;
+        if (best_out) gc_batch_get_tuning(b, best_out);
         if (best_ms_out) *best_ms_out = 0.0;
         return GC_OK;
     }
     if ((s = consider(best)) != GC_OK) return s;
     std::vector<uint32_t> warp_degs = {64, 128, 256, 512};
     if (effort >= 2) warp_degs = {16, 32, 64, 128, 256, 512, 1024, 4096};
-    std::vector<uint32_t> hub_degs = {best.hub_degree};
-    if (effort >= 2) hub_degs = {4096, 16384, 65536};
-    std::vector<int> scheds = {best.schedule};
+    std::vector<uint32_t> hub_degs = {0};  // 0: as it is (set, or by the batch's size)
+    if (effort >= 2) hub_degs = {0, 4096, 16384, 65536};
+    std::vector<int> scheds = {best.t.schedule};
     if (effort >= 1 && b->G > 1) scheds = {GC_SCHEDULE_DEGREE, GC_SCHEDULE_SEGMENT};
     // stage 1: vertex-to-thread mapping (tier thresholds) and schedule
     {
-        const gc_tuning base = best;
+        const Candidate base = best;
         for (int sc : scheds)
             for (uint32_t hd : hub_degs)
                 for (uint32_t wd : warp_degs) {
-                    gc_tuning t = base;
-                    t.schedule = sc;
-                    t.hub_degree = hd;
-                    t.warp_degree = wd;
-                    if ((s = consider(t)) != GC_OK) return s;
+                    Candidate c = base;
+                    c.t.schedule = sc;
+                    if (hd) c.t.hub_degree = hd, c.hub_auto = false;
+                    c.t.warp_degree = wd;
+                    if ((s = consider(c)) != GC_OK) return s;
                 }
     }
-    if (effort >= 1 && (h == GC_GNN) && best.schedule == GC_SCHEDULE_DEGREE) {
+    if (effort >= 1 && (h == GC_GNN) && best.t.schedule == GC_SCHEDULE_DEGREE) {
         // stage 1b: the GNN layers' own warp tier
-        const gc_tuning base = best;
+        const Candidate base = best;
         for (uint32_t gw : {256u, 1024u, 4096u}) {
-            gc_tuning t = base;
-            t.gnn_warp_degree = gw;
-            if ((s = consider(t)) != GC_OK) return s;
+            Candidate c = base;
+            c.t.gnn_warp_degree = gw;
+            c.gnn_warp_auto = false;
+            if ((s = consider(c)) != GC_OK) return s;
         }
     }
     if (effort >= 1) {
         // stage 2: resident CTAs of the ordered coloring kernel
-        const gc_tuning base = best;
-        for (int c : {2, 3, 4, 5}) {
-            gc_tuning t = base;
-            t.jp_ctas_per_sm = c;
-            if ((s = consider(t)) != GC_OK) return s;
+        const Candidate base = best;
+        for (int ctas : {2, 3, 4, 5}) {
+            Candidate c = base;
+            c.t.jp_ctas_per_sm = ctas;
+            if ((s = consider(c)) != GC_OK) return s;
         }
         // stage 3: its polling rhythm
-        const gc_tuning base2 = best;
+        const Candidate base2 = best;
         const unsigned int polls[][2] = {{32, 32}, {8, 32}, {128, 32}, {32, 128}, {4, 8}};
         for (auto &p : polls) {
-            gc_tuning t = base2;
-            t.jp_tight = p[0];
-            t.jp_nap = p[1];
-            if ((s = consider(t)) != GC_OK) return s;
+            Candidate c = base2;
+            c.t.jp_tight = p[0];
+            c.t.jp_nap = p[1];
+            if ((s = consider(c)) != GC_OK) return s;
         }
     }
     if ((s = apply_tuning(b, best)) != GC_OK) return s;
-    if (best_out) *best_out = best;
+    if (best_out) gc_batch_get_tuning(b, best_out);
     if (best_ms_out) *best_ms_out = best_ms;
     return GC_OK;
 }

@@ -30,7 +30,8 @@ constexpr uint32_t GC_GNN_WARP_DEGREE = 256;
 // The GNN layers' own warp tier (degree schedule): a warp stages 32 rows through shared memory, which
 // costs about 2.5 L1 wavefronts per row against 1 for the four-lane tier, so only vertices whose lists
 // are long enough to need a warp's latency hiding get one (the split kernel keeps GC_GNN_WARP_DEGREE).
-// This and GC_GNN_HUB_DEGREE are the values of large graphs; smaller ones take lower ones (auto_degree).
+// This and GC_GNN_HUB_DEGREE are the values of large graphs; smaller ones take lower ones (auto_degree), as long as
+// nobody has set a value: one that was set is taken as it is, these two included.
 constexpr uint32_t GC_GNN_WIDE_DEGREE = 4096;
 // Up to this many neighbours the GNN takes 32 vertices per warp (R-MAT, layers of 1 M vertices: 429 us with 16,
 // 455 with 8, 462 with 32).
@@ -73,9 +74,10 @@ struct gc_ctx {
     int jp_light_warps = 4;              // batches: warps per CTA on the light stream (0: no split; GC_JP_LIGHT_WARPS)
     uint32_t jp_light_min = 1u << 19;    // batches of more vertices than this have a light stream (GC_JP_LIGHT_MIN)
     int gnn_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each GNN layer kernel
-    uint32_t gnn_warp_deg = GC_GNN_WIDE_DEGREE;  // GNN: above this many neighbours a vertex gets a warp
+    uint32_t gnn_warp_deg = GC_GNN_WIDE_DEGREE;  // GNN: above this many neighbours a vertex gets a warp (GC_GNN_WARP_DEGREE)
     uint32_t hub_deg = GC_GNN_HUB_DEGREE;    // plain graphs: above this many neighbours a vertex is a hub (GC_HUB_DEGREE)
-    uint32_t gnn_thin_deg = GC_GNN_THIN_DEGREE;  // GNN: vertices with at most this many neighbours go 32 per warp
+    uint32_t gnn_thin_deg = GC_GNN_THIN_DEGREE;  // GNN: vertices with at most this many neighbours go 32 per warp (GC_GNN_THIN_DEGREE)
+    bool gnn_warp_auto = true, hub_auto = true, gnn_thin_auto = true;  // not set: chosen by the graph's size
     bool gnn_fuse_isolated = true;       // GNN: vertices without neighbours run all layers at once (GC_GNN_FUSE_ISOLATED)
     uint32_t gnn_grab = 2;               // GNN counter hand-out: items per grab (GC_GNN_GRAB; 1-2 best, 8 +4 %, 16 +17 %)
     uint32_t gnn_heavy = 16384;          // GNN counter hand-out: leading four-lane items taken singly (GC_GNN_HEAVY)
@@ -159,6 +161,8 @@ struct gc_graph {
     uint32_t n_wide = 0;             // leading vorder entries with more than GC_GNN_WARP_DEGREE neighbours
     uint32_t n_wide_gnn = 0;         // leading vorder entries the GNN gives a warp (more than gnn_warp_deg)
     uint32_t gnn_warp_deg = GC_GNN_WIDE_DEGREE;
+    bool gnn_warp_auto = true, hub_auto = true;  // chosen by the graph's size, not set
+    uint32_t gnn_warp_now = GC_GNN_WIDE_DEGREE, hub_now = GC_GNN_HUB_DEGREE;  // in force (gc_graph_prepare)
     uint32_t n_thin = 0;             // trailing vorder entries that k_gnn_thin takes
     uint32_t n_iso = 0;              // of those, the trailing entries without neighbours (degree schedule only)
                                      // (degree schedule only; 0 with the graph-major schedule)

@@ -85,7 +85,7 @@ __global__ void k_hub_degrees(const uint32_t *__restrict__ V, const uint32_t *__
 
 constexpr uint32_t THIN_WHOLE = 128, THIN_MIN_PER_SM = 1024;  // (32 resident warps of 32 vertices)
 
-// Degree thresholds of a graph of M directed edges, where the caller left the defaults.  A vertex's FP32
+// Degree thresholds of a graph of M directed edges, where nobody has set them.  A vertex's FP32
 // sums are serial: about 0.03 us a neighbour in the GNN's warp tier and 0.12 us in its four-lane tier,
 // so its longest list bounds a layer of a graph that takes 5.4 ps an edge; the hub kernel evaluates
 // a list 16 times faster, but at three times the SM time per row.  So the tiers end lower on smaller
@@ -158,6 +158,11 @@ gc_status gc_graph_prepare(gc_graph *g) {
     gc_ctx *ctx = g->ctx;
     gc_status s;
     g->rows_ready = false;  // the GNN's feature-row order follows the hub list and the degree order
+    const bool by_degree = g->sched == GC_SCHEDULE_DEGREE;
+    const uint32_t hub_deg = by_degree && g->hub_auto ? auto_degree(g->M, 8192, 2048, GC_GNN_HUB_DEGREE) : g->hub_deg;
+    const uint32_t wide_deg = g->gnn_warp_auto ? auto_degree(g->M, 20000, 512, GC_GNN_WIDE_DEGREE) : g->gnn_warp_deg;
+    g->hub_now = hub_deg;
+    g->gnn_warp_now = wide_deg;
     if (g->N == 0) {
         g->max_deg = 0;
         g->n_big_tasks = 0;
@@ -173,11 +178,6 @@ gc_status gc_graph_prepare(gc_graph *g) {
     int grid = ctx->num_sms * 8;
     // the GNN keeps its own warp tier only with the degree schedule (the graph-major order puts the
     // split's warp tier first, so there the two tiers coincide)
-    const bool by_degree = g->sched == GC_SCHEDULE_DEGREE;
-    const uint32_t hub_deg = by_degree && g->hub_deg == GC_GNN_HUB_DEGREE ? auto_degree(g->M, 8192, 2048, GC_GNN_HUB_DEGREE)
-                                                                         : g->hub_deg;
-    const uint32_t wide_deg = g->gnn_warp_deg == GC_GNN_WIDE_DEGREE ? auto_degree(g->M, 20000, 512, GC_GNN_WIDE_DEGREE)
-                                                                    : g->gnn_warp_deg;
     const uint32_t gnn_wd = by_degree ? std::max(wide_deg, g->warp_deg) : g->warp_deg;
     // pass 1: counts
     if ((s = gc_reset_state(ctx)) != GC_OK) return s;
@@ -196,10 +196,10 @@ gc_status gc_graph_prepare(gc_graph *g) {
     // Below one group for each resident warp the chip is half idle and a vertex's own chain is what
     // counts, which the quad tier keeps shorter: Erdos-Renyi 65,536 90 us here, 80 there; 150,000
     // 136 and 123; 200,000 144 and 139; 400,000 186 and 233; R-MAT 100,003 193 and 183, 1 M 429 and 551.
-    const bool whole = g->max_deg <= THIN_WHOLE && ctx->gnn_thin_deg == GC_GNN_THIN_DEGREE;
+    const bool whole = g->max_deg <= THIN_WHOLE && ctx->gnn_thin_auto;
     g->n_iso = by_degree ? ctx->hstate->isolated : 0u;  // the last entries of the degree order
     g->n_thin = !by_degree ? 0u : whole ? g->N - n_hubs : ctx->hstate->thin;
-    if (ctx->gnn_thin_deg == GC_GNN_THIN_DEGREE && g->n_thin < (uint32_t)ctx->num_sms * THIN_MIN_PER_SM)
+    if (ctx->gnn_thin_auto && g->n_thin < (uint32_t)ctx->num_sms * THIN_MIN_PER_SM)
         g->n_thin = g->n_iso;
     g->n_wide_gnn = g->sched == GC_SCHEDULE_DEGREE ? ctx->hstate->gnn_wide : g->n_wide;
     // lists: the hub list and the degree order fit in cap_N; the task list grows when needed

@@ -179,7 +179,9 @@ typedef enum gc_schedule {
     GC_SCHEDULE_SEGMENT = 1  /* graph by graph, by degree class inside: one graph's rows stay in L2 */
 } gc_schedule;
 
-/* What an autotuner may change; none of it changes a single color or priority bit. */
+/* What an autotuner may change; none of it changes a single color or priority bit.  A batch chooses hub_degree and
+ * gnn_warp_degree by its number of edges (from 2048 and 512 up to the defaults below) until a tuning sets them;
+ * values that were set are taken as they are. */
 typedef struct gc_tuning {
     uint32_t warp_degree;   /* above this many neighbours a vertex gets a whole warp (else 4 lanes) */
     uint32_t hub_degree;    /* above this many neighbours a vertex gets a whole CTA (GNN) or split tasks */
@@ -243,8 +245,9 @@ gc_status gc_batch_download_colors(gc_ctx *ctx, gc_batch *b, int32_t *color);
 gc_status gc_batch_autotune(gc_ctx *ctx, gc_batch *b, gc_heuristic h, const gc_model *model, int recolor,
                             int effort, gc_tuning *best, double *best_ms);
 gc_status gc_batch_set_tuning(gc_ctx *ctx, gc_batch *b, const gc_tuning *t);
+/* The tuning in force: with thresholds that the batch chose by its size, those values. */
 gc_status gc_batch_get_tuning(const gc_batch *b, gc_tuning *t);
-/* The library's default tuning. */
+/* The library's default tuning (its thresholds are those of large batches). */
 void gc_tuning_default(gc_tuning *t);
 
 /* ---- serving: a request loop with continuous batching ----------------------------------------- */
