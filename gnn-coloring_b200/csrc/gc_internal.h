@@ -140,7 +140,6 @@ struct gc_graph {
     unsigned long long *fmask = nullptr;
     uint32_t *sort_buf = nullptr;  // radix sort ping-pong (keys and values), 4 * cap_N words
     uint32_t *sort_hist = nullptr;
-    uint32_t sort_hist_cap = 0;
     // degree classes (depend on the graph only; rebuilt on upload)
     uint32_t *big = nullptr;         // split tasks of the hubs: (vertex, first edge) pairs
     uint32_t n_big_tasks = 0;

@@ -359,15 +359,12 @@ gc_status gc_sort_vertices(gc_graph *g, const uint32_t *keys, int key_bits, int 
     if ((s = gc_alloc(ctx, &g->sort_buf, 4 * (size_t)g->cap_N, "sort buffers")) != GC_OK) return s;
     const int passes = key_bits <= 0 ? 1 : (key_bits + 7) / 8;
     const uint32_t ntiles = (N + SORT_TILE - 1) / SORT_TILE;
-    // digit totals and bases (4 passes at most), tile counters, then the tiles' status words per pass
+    // digit totals and bases (4 passes at most), tile counters, then the tiles' status words per pass.  Allocated
+    // once for the most passes and the graph's capacity (half a byte per vertex): captured passes hold the address
     const size_t head = 2 * 4 * RADIX + 4;
     const size_t words = head + (size_t)passes * ntiles * RADIX;
-    if (g->sort_hist_cap < words) {
-        gc_dev_free(ctx, g->sort_hist);
-        g->sort_hist = nullptr;
-        if ((s = gc_alloc(ctx, &g->sort_hist, words, "sort histogram")) != GC_OK) return s;
-        g->sort_hist_cap = (uint32_t)words;
-    }
+    const size_t most = head + 4 * (size_t)((g->cap_N + SORT_TILE - 1) / SORT_TILE) * RADIX;
+    if ((s = gc_alloc(ctx, &g->sort_hist, most, "sort histogram")) != GC_OK) return s;
     uint32_t *totals = g->sort_hist, *bases = totals + 4 * RADIX, *tile_ctr = bases + 4 * RADIX;
     uint32_t *status = g->sort_hist + head;
     ProfScope ps(ctx, "sort", ctx->stream);
