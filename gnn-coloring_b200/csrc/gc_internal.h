@@ -133,12 +133,11 @@ struct gc_graph {
     uint4 *jpsplit = nullptr;       // the tickets after the core: heavy stream from the front, light from the back
     uint32_t *part_tiles = nullptr; // heavy tickets per tile of the split (prefix)
     uint32_t *round_ctr = nullptr;    // Culberson rounds: work counters (k_round.cu)
-    uint32_t *flow_q = nullptr;       // dataflow coloring: queue counters and slots (k_flow.cu)
     // forbidden colors 1..256 published by waiting vertices of the ordered coloring kernel:
     // GC_JP_MASK_WORDS words per vertex, each (epoch << 32 | 32 color bits); the word after the
     // last vertex's holds the epoch counter, advanced once per coloring run
     unsigned long long *fmask = nullptr;
-    uint32_t *sort_buf = nullptr;  // radix sort ping-pong (keys and values), 4 * cap_N words
+    uint32_t *sort_buf = nullptr;  // radix sort ping-pong (keys and values), 4 * cap_N words; the dataflow's queues
     uint32_t *sort_hist = nullptr;
     // degree classes (depend on the graph only; rebuilt on upload)
     uint32_t *big = nullptr;         // split tasks of the hubs: (vertex, first edge) pairs
@@ -259,6 +258,7 @@ gc_status gc_jp_color(gc_graph *g);                                // JP by curr
 // run instead.
 bool gc_flow_eligible(const gc_graph *g);
 gc_status gc_jp_flow(gc_graph *g);
+size_t gc_flow_queue_words(uint32_t cap_N);
 gc_status gc_keys_from_colors(gc_graph *g);                        // Culberson step (k_jp.cu)
 // JP by current keys, `rounds` Culberson rounds and (stats) the color count of a small graph in one CTA
 // (k_small.cu).  Waits; a set flow_stall means that nothing was written and the others must color it.
@@ -277,6 +277,7 @@ int gc_colors_of_state(const gc_graph *g);    // its result once the state has b
 enum { SORT_KEEP_ALL = 0, SORT_KEEP_INNER = 1, SORT_KEEP_DEG_AT_MOST = 2 };
 gc_status gc_sort_vertices(gc_graph *g, const uint32_t *keys, int key_bits, int filter, uint32_t max_deg,
                            uint32_t *out, uint32_t *d_count);
+gc_status gc_sort_scratch(gc_graph *g);  // allocates sort_buf, for the sorts and the dataflow's queues
 gc_status gc_sort_order_bits(gc_graph *g, int key_bits, bool filter, uint32_t *d_count);
 // Stable sort of n (key, value) pairs by ascending key into (kout, vout); kbuf, vbuf: n-word
 // scratch; hist: gc_sort_pairs_hist_words(n) words (k_sort.cu).

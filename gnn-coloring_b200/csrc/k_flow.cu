@@ -323,6 +323,7 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
     // counter words in the first half of the ticket records' buffer; masks in the second half (up to 8
     // bytes per vertex), else in the ticket streams' buffer
     unsigned long long *word = reinterpret_cast<unsigned long long *>(g->jprec);
+    uint32_t *fq = g->sort_buf;
     using MaskT = typename FlowMask<W>::T;
     MaskT *mask = W <= 2 ? reinterpret_cast<MaskT *>(word + g->cap_N) : reinterpret_cast<MaskT *>(g->jpsplit);
     int &occ = ctx->flow_blocks_per_sm[W == FLOW_WIDE ? 2 : W - 1];
@@ -332,14 +333,14 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
             return s;
         if (occ < 1) occ = 1;
     }
-    if ((s = gc_check_cuda(ctx, cudaMemsetAsync(g->flow_q, 0, 4 * ((size_t)FLOW_SLOTS + 2 * (size_t)FLOW_QUEUES * stride),
+    if ((s = gc_check_cuda(ctx, cudaMemsetAsync(fq, 0, 4 * ((size_t)FLOW_SLOTS + 2 * (size_t)FLOW_QUEUES * stride),
                                                 ctx->stream), "flow queues")) != GC_OK)
         return s;
     const uint32_t N = g->N;
     {
         ProfScope ps(ctx, "flow_init", ctx->stream);
         const uint32_t blocks = std::min<uint32_t>((uint32_t)ctx->num_sms * 8, (N + 63) / 64);
-        k_flow_init<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(g->V, g->E, g->key, N, word, mask, g->color, g->flow_q,
+        k_flow_init<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(g->V, g->E, g->key, N, word, mask, g->color, fq,
                                                                  stride);
     }
     {
@@ -351,7 +352,7 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
         const int per_sm = std::min(occ, N <= FLOW_FEW_N ? std::max(1, ctx->flow_ctas_per_sm / 2) : ctx->flow_ctas_per_sm);
         const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)per_sm;
         const uint32_t blocks = std::max<uint32_t>(FLOW_MIN_CTAS, std::min<uint32_t>(most, (N + 31) / 32));
-        k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->M, g->color, g->flow_q, N, stride,
+        k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->M, g->color, fq, N, stride,
                                                                ctx->dstate, std::min(ctx->spin_limit, ctx->flow_limit));
     }
     ctx->launches += 2;
@@ -373,6 +374,12 @@ bool gc_flow_eligible(const gc_graph *g) {
     return g->n_seg == 0 && g->N > 0 && g->max_deg < std::min(g->ctx->flow_max_deg, widest);
 }
 
+// Counters and slots (two words each).  They share the sort's scratch, so that a graph which the tickets color after
+// all holds no more than they need.
+size_t gc_flow_queue_words(uint32_t cap_N) {
+    return 2 * ((size_t)cap_N + 1024 * FLOW_QUEUES) + FLOW_SLOTS;
+}
+
 gc_status gc_jp_flow(gc_graph *g) {
     gc_ctx *ctx = g->ctx;
     gc_status s;
@@ -380,6 +387,6 @@ gc_status gc_jp_flow(gc_graph *g) {
     const uint32_t stride = ((g->N + FLOW_QUEUES - 1) / FLOW_QUEUES + 1023u) & ~1023u;
     if ((s = gc_alloc(ctx, &g->jprec, g->cap_N, "vertex records")) != GC_OK) return s;
     if (wide && (s = gc_alloc(ctx, &g->jpsplit, g->cap_N, "vertex records")) != GC_OK) return s;
-    if ((s = gc_alloc(ctx, &g->flow_q, 2 * ((size_t)g->cap_N + 1024 * FLOW_QUEUES) + FLOW_SLOTS, "flow queues")) != GC_OK) return s;
+    if ((s = gc_sort_scratch(g)) != GC_OK) return s;
     return wide ? flow_run<FLOW_WIDE>(g, stride) : g->max_deg >= 32 ? flow_run<2>(g, stride) : flow_run<1>(g, stride);
 }

@@ -107,7 +107,7 @@ gc_status gc_sort_hubs(gc_graph *g) {
     if (g->hubs_sorted || !n_hubs) return GC_OK;
     // (vertex, degree) pairs of the hubs, sorted on the host by descending degree, so the longest FP32 add
     // chains start first
-    if ((s = gc_alloc(ctx, &g->sort_buf, 4 * (size_t)g->cap_N, "sort buffers")) != GC_OK) return s;
+    if ((s = gc_sort_scratch(g)) != GC_OK) return s;
     k_hub_degrees<<<ctx->num_sms, 256, 0, ctx->stream>>>(g->V, g->hubs, n_hubs, g->sort_buf);
     ctx->launches++;
     std::vector<uint32_t> hp(2 * (size_t)n_hubs), h(n_hubs);

@@ -347,6 +347,10 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_sweep(SortIn in, int shif
 
 }  // namespace
 
+gc_status gc_sort_scratch(gc_graph *g) {
+    return gc_alloc(g->ctx, &g->sort_buf, std::max(4 * (size_t)g->cap_N, gc_flow_queue_words(g->cap_N)), "sort buffers");
+}
+
 // Sorts vertex ids by descending key (ascending id on ties) into `out`.  key_bits: number of low
 // key bits that may be non-zero; 0 means "all keys equal" (a stable compaction by id).  `filter`
 // selects which vertices take part (SORT_KEEP_*); their number is left in *d_count.
@@ -356,7 +360,7 @@ gc_status gc_sort_vertices(gc_graph *g, const uint32_t *keys, int key_bits, int 
     gc_status s;
     const uint32_t N = g->N;
     if (N == 0) return GC_OK;
-    if ((s = gc_alloc(ctx, &g->sort_buf, 4 * (size_t)g->cap_N, "sort buffers")) != GC_OK) return s;
+    if ((s = gc_sort_scratch(g)) != GC_OK) return s;
     const int passes = key_bits <= 0 ? 1 : (key_bits + 7) / 8;
     const uint32_t ntiles = (N + SORT_TILE - 1) / SORT_TILE;
     // digit totals and bases (4 passes at most), tile counters, then the tiles' status words per pass.  Allocated
