@@ -71,9 +71,16 @@ constexpr uint32_t FLOW_FEW_N = 1u << 18;
 // on its way one load earlier.  rem is the top field: one subtraction too many (a self-loop, a CSR that
 // is not symmetric) wraps there and leaves the others alone.  A vertex that thousands name one-sidedly would become
 // ready a second time, take another's place in its array, and leave that one without a color: the subtraction
-// that finds FLOW_ASKEW in rem stops the kernel long before.
+// that finds a multiple of FLOW_LEAF in rem stops the kernel long before.
 constexpr unsigned long long FLOW_ONE = 1ull << 48;
-constexpr uint32_t FLOW_ASKEW = 0x8000u;
+
+// Leaves (every neighbour precedes them) make nobody ready.  In graphs whose longest lists are far above the mean
+// -- trees, hubs with their leaves -- they are most of the vertices, and a warp that queues dozens of them per
+// hop holds up the chain.  There the leaves stay out of the queues: rem starts at FLOW_LEAF + the predecessors,
+// so it never says ready, and a pass after the flow colors them all (trees of 2^20 vertices, first fit, leaves
+// queued / apart: arity 30 286 / 175 us, 60 338 / 199; a path of 5,000 with 100 leaves each 15,600 / 6,200).
+constexpr uint32_t FLOW_LEAF = 0x4000u;
+constexpr uint32_t FLOW_SKEW = 4;  // leaves apart where the largest degree is above this many times the mean
 // W words of 32 mask bits per vertex (bit j of word w: neighbour 32 w + j precedes).
 constexpr int FLOW_WIDE = 4;
 template <int W>
@@ -119,7 +126,7 @@ __device__ __forceinline__ void flow_push(uint32_t *fq, uint32_t stride, uint32_
 }
 
 // Four lanes per vertex, vertices in id order (records, CSR offsets and rows stream).
-template <int W>
+template <int W, bool LEAVES>
 __global__ void __launch_bounds__(FLOW_THREADS) k_flow_init(const uint32_t *__restrict__ V, const uint32_t *__restrict__ E,
                                                             const uint32_t *__restrict__ key, uint32_t N,
                                                             unsigned long long *__restrict__ word,
@@ -127,6 +134,11 @@ __global__ void __launch_bounds__(FLOW_THREADS) k_flow_init(const uint32_t *__re
                                                             int *__restrict__ color,
                                                             uint32_t *__restrict__ fq, uint32_t stride) {
     constexpr int LOADS = 8;
+    __shared__ uint32_t apart[LEAVES ? FLOW_QUEUES : 1];  // vertices that stay out of each array
+    if (LEAVES) {
+        if (threadIdx.x < FLOW_QUEUES) apart[threadIdx.x] = 0;
+        __syncthreads();
+    }
     const int lane = threadIdx.x & 31, q = lane & 3, qbase = lane & ~3;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint64_t keep = l2_keep_policy();  // the keys (4N bytes) stay in L2 while E streams past
@@ -158,11 +170,17 @@ __global__ void __launch_bounds__(FLOW_THREADS) k_flow_init(const uint32_t *__re
             cnt += __popc(m[w]);
         }
         if (valid && q == 0) {
-            word[u] = (unsigned long long)cnt * FLOW_ONE | (unsigned long long)d << 32 | beg;
+            const bool out = LEAVES && cnt == d;
+            word[u] = (unsigned long long)(out && d ? cnt | FLOW_LEAF : cnt) << 48 | (unsigned long long)d << 32 | beg;
             mask[u] = FlowMask<W>::put(m);
             color[u] = cnt == 0 ? 1 : 0;
-            if (cnt == 0) flow_push(fq, stride, u, beg);
+            if (out) atomicAdd(apart + u % FLOW_QUEUES, 1u);
+            else if (cnt == 0) flow_push(fq, stride, u, beg);
         }
+    }
+    if (LEAVES) {
+        __syncthreads();
+        if (threadIdx.x < FLOW_QUEUES && apart[threadIdx.x]) atomicAdd(flow_skip(fq, threadIdx.x), apart[threadIdx.x]);
     }
 }
 
@@ -267,22 +285,23 @@ __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsign
             for (int w = 0; w < W; w++) {
                 const uint32_t left = (uint32_t)(old[w] >> 48);
                 bool ready = left == 1u;
-                if (left == FLOW_ASKEW) st_relaxed_u32(&st->flow_stall, 1u);
                 const unsigned int rm = __ballot_sync(FULL, ready);
-                if (!rm) continue;
-                if (!more) {
-                    more = true;
-                    const int first = __ffs(rm) - 1;
-                    u = __shfl_sync(FULL, keep[w], first);
-                    const uint32_t lo = __shfl_sync(FULL, (uint32_t)old[w], first);
-                    const uint32_t hi = __shfl_sync(FULL, (uint32_t)(old[w] >> 32), first);
-                    fetch(lo, hi);
-                    if (lane == first) {
-                        ready = false;
-                        atomicAdd(flow_skip(fq, u % FLOW_QUEUES), 1u);
+                if (rm) {
+                    if (!more) {
+                        more = true;
+                        const int first = __ffs(rm) - 1;
+                        u = __shfl_sync(FULL, keep[w], first);
+                        const uint32_t lo = __shfl_sync(FULL, (uint32_t)old[w], first);
+                        const uint32_t hi = __shfl_sync(FULL, (uint32_t)(old[w] >> 32), first);
+                        fetch(lo, hi);
+                        if (lane == first) {
+                            ready = false;
+                            atomicAdd(flow_skip(fq, u % FLOW_QUEUES), 1u);
+                        }
                     }
+                    if (ready) flow_push(fq, stride, keep[w], (uint32_t)old[w]);
                 }
-                if (ready) flow_push(fq, stride, keep[w], (uint32_t)old[w]);
+                if (left && left % FLOW_LEAF == 0) st_relaxed_u32(&st->flow_stall, 1u);
             }
             uint32_t used[W];
 #pragma unroll
@@ -316,6 +335,56 @@ __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsign
     }
 }
 
+// The leaves: a warp looks through 32 vertices and colors four leaves at a time, eight lanes each.
+template <int W>
+__global__ void __launch_bounds__(FLOW_THREADS) k_flow_leaves(const unsigned long long *__restrict__ word,
+                                                              const uint32_t *__restrict__ E, uint32_t N, int *color,
+                                                              DevState *st) {
+    constexpr unsigned int FULL = 0xffffffffu;
+    constexpr int LOADS = 4;
+    if (st->flow_stall) return;
+    const int lane = threadIdx.x & 31, q = lane & 7;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < N; base += nwarps * 32) {
+        const unsigned long long mine = base + lane < N ? word[base + lane] : 0ull;
+        unsigned int found = __ballot_sync(FULL, ((uint32_t)(mine >> 48) & ~127u) == FLOW_LEAF);
+        while (found) {
+            int src = -1;  // the leaf of this lane's group
+            for (int k = 0; k < 4 && found; k++, found &= found - 1)
+                if (k == lane >> 3) src = __ffs(found) - 1;
+            const unsigned long long w0 = __shfl_sync(FULL, mine, max(src, 0));
+            const uint32_t beg = (uint32_t)w0, d = src < 0 ? 0u : (uint32_t)(w0 >> 32) & 0xffffu;
+            uint32_t used[W];
+#pragma unroll
+            for (int x = 0; x < W; x++) used[x] = 0;
+            for (uint32_t j = q; j < d; j += 8 * LOADS) {
+                uint32_t v[LOADS], c[LOADS];
+#pragma unroll
+                for (int k = 0; k < LOADS; k++) v[k] = j + 8 * k < d ? ld_stream(E + beg + j + 8 * k) : 0u;
+#pragma unroll
+                for (int k = 0; k < LOADS; k++) c[k] = j + 8 * k < d ? (uint32_t)color[v[k]] : 1u << 31;
+#pragma unroll
+                for (int k = 0; k < LOADS; k++) {
+                    // (in a symmetric CSR a leaf's neighbours all have their colors)
+                    if (c[k] == 0 && v[k] != base + src) st_relaxed_u32(&st->flow_stall, 1u);
+#pragma unroll
+                    for (int x = 0; x < W; x++)
+                        if ((c[k] - 1u) >> 5 == (uint32_t)x) used[x] |= 1u << ((c[k] - 1u) & 31u);
+                }
+            }
+            __syncwarp();
+            int c = 0;
+#pragma unroll
+            for (int x = 0; x < W; x++) {
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) used[x] |= __shfl_xor_sync(FULL, used[x], o);
+                if (c == 0 && ~used[x]) c = 32 * x + __ffs(~used[x]);
+            }
+            if (src >= 0 && q == 0) color[base + src] = c;
+        }
+    }
+}
+
 template <int W>
 gc_status flow_run(gc_graph *g, uint32_t stride) {
     gc_ctx *ctx = g->ctx;
@@ -337,11 +406,12 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
                                                 ctx->stream), "flow queues")) != GC_OK)
         return s;
     const uint32_t N = g->N;
+    const bool leaves = (uint64_t)g->max_deg * N > (uint64_t)FLOW_SKEW * g->M;
     {
         ProfScope ps(ctx, "flow_init", ctx->stream);
         const uint32_t blocks = std::min<uint32_t>((uint32_t)ctx->num_sms * 8, (N + 63) / 64);
-        k_flow_init<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(g->V, g->E, g->key, N, word, mask, g->color, fq,
-                                                                 stride);
+        (leaves ? k_flow_init<W, true> : k_flow_init<W, false>)<<<blocks, FLOW_THREADS, 0, ctx->stream>>>(
+            g->V, g->E, g->key, N, word, mask, g->color, fq, stride);
     }
     {
         ProfScope ps(ctx, "jp_flow", ctx->stream);
@@ -356,6 +426,12 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
                                                                ctx->dstate, std::min(ctx->spin_limit, ctx->flow_limit));
     }
     ctx->launches += 2;
+    if (leaves) {
+        ProfScope ps(ctx, "flow_leaves", ctx->stream);
+        const uint32_t blocks = std::min<uint32_t>((uint32_t)ctx->num_sms * 8, (N + FLOW_THREADS - 1) / FLOW_THREADS);
+        k_flow_leaves<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, g->E, N, g->color, ctx->dstate);
+        ctx->launches++;
+    }
     return gc_check_launch(ctx, "jp flow");
 }
 
@@ -364,13 +440,16 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
 // Which graphs go by dataflow: a maximum degree below 64 always (whole calls, largest degree first, dataflow /
 // tickets: Erdos-Renyi 200,000 x 16 167 / 281 us, 1 M x 24 545 / 1,038, 4 M x 16 1,607 / 3,459); below 128 up to
 // FLOW_WIDE_MAX_N vertices, the largest size measured, since the wide kernel keeps half as many vertices in
-// flight (250,000 x 40 363 / 397, 500,000 x 34 461 / 639, 1 M x 34 939 / 1,185).  Larger degrees would put long
+// flight (250,000 x 40 363 / 397, 500,000 x 34 461 / 639, 1 M x 34 939 / 1,185), and not where the mean degree is
+// below FLOW_WIDE_MEAN: there most vertices are a whole warp's work for a few entries (arity-100 tree of 2^20
+// vertices, dataflow / tickets: random priorities 429 / 248, first fit 213 / 187).  Larger degrees would put long
 // lists on the chain, and power-law graphs have their chains colored inside one cluster (k_jp_core).
 // Plain graphs only: a batch is captured, and the stall flag needs the host.
-constexpr uint32_t FLOW_WIDE_MAX_N = 1u << 20;
+constexpr uint32_t FLOW_WIDE_MAX_N = 1u << 20, FLOW_WIDE_MEAN = 4;
 
 bool gc_flow_eligible(const gc_graph *g) {
-    const uint32_t widest = g->N <= FLOW_WIDE_MAX_N ? 32u * FLOW_WIDE : 64u;
+    const bool wide = g->N <= FLOW_WIDE_MAX_N && g->M / FLOW_WIDE_MEAN >= g->N;
+    const uint32_t widest = wide ? 32u * FLOW_WIDE : 64u;
     return g->n_seg == 0 && g->N > 0 && g->max_deg < std::min(g->ctx->flow_max_deg, widest);
 }
 
