@@ -289,9 +289,11 @@ gc_status color_by_keys(gc_ctx *ctx, gc_graph *g, bool *unread) {
     return GC_OK;
 }
 
+// After a dataflow coloring that stopped.
 gc_status color_by_tickets(gc_ctx *ctx, gc_graph *g) {
+    const bool narrow = ctx->hstate->flow_stall == gc::FLOW_NARROW;
     gc_status s = gc_reset_state(ctx);
-    return s == GC_OK ? gc_jp_color(g) : s;
+    return s == GC_OK ? gc_jp_color(g, narrow) : s;
 }
 
 // The coloring by the current keys (when `first`), then `rounds` Culberson rounds, then the color count
@@ -395,6 +397,7 @@ gc_status gc_ctx_create(int device, gc_ctx **out) {
     if (const char *e = getenv("GC_JP_FLOW")) ctx->flow_max_deg = (uint32_t)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_FLOW_CTAS")) ctx->flow_ctas_per_sm = std::max(1, atoi(e));
     if (const char *e = getenv("GC_JP_FLOW_LIMIT")) ctx->flow_limit = (unsigned int)strtoul(e, nullptr, 10);
+    if (const char *e = getenv("GC_JP_NARROW")) ctx->narrow_window = (unsigned int)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_SMALL")) ctx->small_max = (uint32_t)strtoul(e, nullptr, 10);
     if (const char *e = getenv("GC_JP_CLASSES")) ctx->jp_classes = atoi(e) != 0;
     if (const char *e = getenv("GC_JP_DECIDE")) ctx->jp_decide = atoi(e) != 0;

@@ -59,6 +59,7 @@ struct gc_ctx {
     uint32_t flow_max_deg = 128;         // coloring: graphs with a smaller maximum degree go by dataflow (0: none; GC_JP_FLOW)
     int flow_ctas_per_sm = 8;            // dataflow kernel: CTAs per SM at most (GC_JP_FLOW_CTAS)
     unsigned int flow_limit = 1u << 16;  // dataflow kernel: fruitless polls before a warp looks whether anything moves (GC_JP_FLOW_LIMIT)
+    unsigned int narrow_window = 1u << 18;  // cycles after which a coloring is found narrow (0: never; GC_JP_NARROW)
     uint32_t small_max = GC_SMALL_AUTO;  // coloring: graphs of up to this many vertices that fit go in one CTA (0: none; GC_JP_SMALL)
     bool small_ready = false;            // that kernel's shared-memory limit is set
     int round_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each Culberson kernel
@@ -252,10 +253,12 @@ gc_status gc_priority_gnn(gc_graph *g, const gc_model *m);         // GraphSAGE 
 // N (ERR_BOUND, reported by the next gc_read_state) and writes row 0 for one that is out of range.
 gc_status gc_gnn_rows_begin(gc_graph *g);
 gc_status gc_gnn_row_ids(gc_graph *g, uint32_t first, uint32_t count);
-gc_status gc_jp_color(gc_graph *g);                                // JP by current keys (k_jp.cu)
+// JP by current keys in ticket order (k_jp.cu).  `narrow`: few vertices become ready at a time, so as many of the
+// first tickets as fit are colored inside one cluster.
+gc_status gc_jp_color(gc_graph *g, bool narrow = false);
 // JP by current keys as a dataflow, on graphs of small maximum degree (k_flow.cu).  Queued only: once
 // the state has been read, a set flow_stall means that the colors are incomplete and gc_jp_color must
-// run instead.
+// run instead (narrow: FLOW_NARROW).
 bool gc_flow_eligible(const gc_graph *g);
 gc_status gc_jp_flow(gc_graph *g);
 size_t gc_flow_queue_words(uint32_t cap_N);

@@ -30,6 +30,13 @@
 // which the CTAs start) has that remainder: the first five CTAs that run serve them all, so the kernel
 // advances whatever else occupies the GPU.
 //
+// A DAG that is narrow -- a band, a strip, a path, a caterpillar -- has its next vertices known long before:
+// its hops cost 0.63 to 3 us here, 0.1 to 0.3 among tickets whose colors stay in one cluster's shared memory
+// (k_jp_core).  So one CTA only counts what becomes ready, in windows of 133 us, and stops a coloring that it finds
+// narrow (flow_watch); the tickets then color the graph, as many as fit in the cluster.  First fit, dataflow to
+// the end / this: a path of 20,000 12.8 / 5.2 ms, 20,000 rows of a band matrix with 31 entries on either side 22.9
+// / 2.4, a 5-point strip of 4 x 5,000 3.5 / 1.6, a path of 10,000 with 50 leaves each 23.6 / 2.9.
+//
 // A CSR that is not symmetric (a caller's mistake that the upload does not check) can leave vertices
 // that never become ready.  Idle warps watch the counters; when none moves for a while they set
 // DevState::flow_stall and every warp leaves.  The host then runs the ticket kernels, whose waits
@@ -191,6 +198,54 @@ __device__ __forceinline__ uint32_t flow_progress(uint32_t *fq, int lane) {
     return __reduce_add_sync(0xffffffffu, n);
 }
 
+// The watching CTA.  A coloring is narrow when in the first window fewer than FLOW_THIN vertices a microsecond became
+// ready (at 1.965 GHz; latencies and the clock change together), or in a later one fewer than FLOW_FEW, while half
+// of what was not ready at the start is still to come and would take four windows more.  By tickets in the cluster, strips of 4 to 50
+// vertices' width run at 11 to 55 a microsecond, bars of 4 x 4 to 16 x 16 at 8 to 23; wavefronts start narrow as
+// well but have passed FLOW_THIN by the end of the first window (a mesh's corner: 50 a microsecond, a square 5-point
+// grid 40), and a second window costs less than a wrong turn.
+// To stop it, FLOW_VOID is added to the counters, so that no vertex becomes ready any more, and to the arrays' skip
+// counters, so that nobody waits for one.  What has started runs to its end, since it only waits for what has started.
+// (The warps that color know nothing of this: a look at a flag in their loops cost path and mesh 40 %.)
+constexpr uint32_t FLOW_THIN = 16, FLOW_FEW = 30, FLOW_MHZ = 1965, FLOW_VOID = 0x2000u;
+
+__device__ void flow_watch(unsigned long long *word, uint32_t *fq, uint32_t N, uint32_t window, DevState *st, uint32_t check) {
+    __shared__ bool stop;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        uint32_t since = (uint32_t)clock(), ready = flow_progress(fq, lane), last = ready, same = 0;
+        const uint32_t left0 = N - min(ready, N);
+        bool first = true, narrow = false;
+        for (;;) {
+            const uint32_t now = flow_progress(fq, lane), left = N - min(now, N);
+            if (left == 0 || __shfl_sync(0xffffffffu, lane == 0 ? ld_relaxed_u32(&st->flow_stall) : 0u, 0)) break;
+            same = now == last ? same + 1u : 0u;
+            last = now;
+            if (same > check) break;
+            const uint32_t dt = __shfl_sync(0xffffffffu, (uint32_t)clock() - since, 0);
+            if (dt >= window) {
+                const unsigned long long got = now - ready;
+                narrow = got * FLOW_MHZ < (unsigned long long)dt * (first ? FLOW_THIN : FLOW_FEW) && left >= left0 / 2 &&
+                         (unsigned long long)left * dt >= 4 * got * window;
+                if (narrow) break;
+                since += dt;
+                ready = now;
+                first = false;
+            }
+            __nanosleep(500);
+        }
+        if (lane == 0) {
+            stop = narrow;
+            if (narrow) st_relaxed_u32(&st->flow_stall, FLOW_NARROW);
+        }
+    }
+    __syncthreads();
+    if (!stop) return;
+    for (uint32_t v = threadIdx.x; v < N; v += FLOW_THREADS) atomicAdd(word + v, (unsigned long long)FLOW_VOID << 48);
+    __syncthreads();
+    if (threadIdx.x < FLOW_QUEUES) atomicAdd(flow_skip(fq, threadIdx.x), N);
+}
+
 // One more fruitless poll of a warp: true when the warp must leave.  After `check` polls the warp
 // compares the tails with their last sum; unchanged means that nothing moves.
 struct FlowWait {
@@ -201,7 +256,7 @@ struct FlowWait {
         if (spins <= check) return false;
         const uint32_t now = flow_progress(fq, lane);
         if (now == seen) {
-            if (lane == 0) st_relaxed_u32(&st->flow_stall, 1u);
+            if (lane == 0) st_relaxed_u32(&st->flow_stall, FLOW_STUCK);
             return true;
         }
         seen = now;
@@ -214,11 +269,16 @@ template <int W>
 __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsigned long long *word,
                                                           const typename FlowMask<W>::T *__restrict__ mask,
                                                           const uint32_t *__restrict__ E, uint32_t M, int *color, uint32_t *fq,
-                                                          uint32_t N, uint32_t stride, DevState *st, uint32_t check) {
+                                                          uint32_t N, uint32_t stride, DevState *st, uint32_t check,
+                                                          uint32_t window) {
     constexpr unsigned int FULL = 0xffffffffu;
     __shared__ uint32_t cta_s;
     if (threadIdx.x == 0) cta_s = atomicAdd(fq + FLOW_CTA, 1u);
     __syncthreads();
+    if (window && cta_s == FLOW_MIN_CTAS) {
+        flow_watch(word, fq, N, window, st, check);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const uint32_t k = (cta_s * (FLOW_THREADS / 32) + (threadIdx.x >> 5)) % FLOW_QUEUES;
     const uint32_t nk = k < N ? (N - k + FLOW_QUEUES - 1) / FLOW_QUEUES : 0u;  // vertices of this array
@@ -301,7 +361,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, W <= 2 ? 8 : 4) k_jp_flow(unsign
                     }
                     if (ready) flow_push(fq, stride, keep[w], (uint32_t)old[w]);
                 }
-                if (left && left % FLOW_LEAF == 0) st_relaxed_u32(&st->flow_stall, 1u);
+                if (left && left % FLOW_LEAF == 0) st_relaxed_u32(&st->flow_stall, FLOW_STUCK);
             }
             uint32_t used[W];
 #pragma unroll
@@ -366,7 +426,7 @@ __global__ void __launch_bounds__(FLOW_THREADS) k_flow_leaves(const unsigned lon
 #pragma unroll
                 for (int k = 0; k < LOADS; k++) {
                     // (in a symmetric CSR a leaf's neighbours all have their colors)
-                    if (c[k] == 0 && v[k] != base + src) st_relaxed_u32(&st->flow_stall, 1u);
+                    if (c[k] == 0 && v[k] != base + src) st_relaxed_u32(&st->flow_stall, FLOW_STUCK);
 #pragma unroll
                     for (int x = 0; x < W; x++)
                         if ((c[k] - 1u) >> 5 == (uint32_t)x) used[x] |= 1u << ((c[k] - 1u) & 31u);
@@ -421,9 +481,12 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
         // geometric 200,000 108 / 99; 500,000 149 / 195, Erdos-Renyi 600,000 226 / 279)
         const int per_sm = std::min(occ, N <= FLOW_FEW_N ? std::max(1, ctx->flow_ctas_per_sm / 2) : ctx->flow_ctas_per_sm);
         const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)per_sm;
-        const uint32_t blocks = std::max<uint32_t>(FLOW_MIN_CTAS, std::min<uint32_t>(most, (N + 31) / 32));
+        // (a long path stays: one successor per hop is 0.63 us here, and past the cluster's tickets 0.73 there)
+        const uint32_t window = g->max_deg <= 2 && N > (1u << 17) ? 0u : ctx->narrow_window;
+        const uint32_t blocks = std::max<uint32_t>(FLOW_MIN_CTAS + 1, std::min<uint32_t>(most, (N + 31) / 32));
         k_jp_flow<W><<<blocks, FLOW_THREADS, 0, ctx->stream>>>(word, mask, g->E, g->M, g->color, fq, N, stride,
-                                                               ctx->dstate, std::min(ctx->spin_limit, ctx->flow_limit));
+                                                               ctx->dstate, std::min(ctx->spin_limit, ctx->flow_limit),
+                                                               window);
     }
     ctx->launches += 2;
     if (leaves) {

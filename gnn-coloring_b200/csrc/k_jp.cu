@@ -1279,9 +1279,10 @@ gc_status core_cluster_config(gc_ctx *ctx) {
 // 2.2 M, LF 1,172 / 1,110, GNN2 2,287 / 2,245).
 constexpr uint32_t CORE_DEFAULT = 2048, CORE_MIN_N = 65536, CORE_MIN_BATCH = 1u << 19;
 
-uint32_t core_tickets(const gc_graph *g) {
+uint32_t core_tickets(const gc_graph *g, bool narrow) {
     const uint32_t most = g->ctx->jp_core_max;
     if (most != GC_CORE_AUTO) return most;
+    if (narrow) return CORE_MAX;
     return g->N > (g->n_seg ? CORE_MIN_BATCH : CORE_MIN_N) ? CORE_DEFAULT : 0u;
 }
 
@@ -1333,7 +1334,7 @@ int bit_length(uint64_t x) {
 
 }  // namespace
 
-gc_status gc_jp_color(gc_graph *g) {
+gc_status gc_jp_color(gc_graph *g, bool narrow) {
     gc_ctx *ctx = g->ctx;
     gc_status s;
     const uint32_t N = g->N;
@@ -1371,7 +1372,7 @@ gc_status gc_jp_color(gc_graph *g) {
             ctx->launches += 2;
         }
         k_jp_init_colors<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(g->pc, N, g->color, ctx->dstate,
-                                                                ctx->jp_core_max != GC_CORE_AUTO || g->n_seg ? CORE_FORCED : 0u);
+                                                                narrow || ctx->jp_core_max != GC_CORE_AUTO || g->n_seg ? CORE_FORCED : 0u);
         ctx->launches++;
     }
     if ((s = gc_check_launch(ctx, "jp split")) != GC_OK) return s;
@@ -1386,7 +1387,7 @@ gc_status gc_jp_color(gc_graph *g) {
 
     if ((s = gc_alloc(ctx, &g->jprec, g->cap_N, "ticket records")) != GC_OK) return s;
     uint32_t core = 0;  // core tickets colored in one cluster (at most)
-    const uint32_t wanted = core_tickets(g);
+    const uint32_t wanted = core_tickets(g, narrow);
     if (wanted && (s = core_cluster_config(ctx)) == GC_OK && ctx->jp_core_cluster > 0) core = core_fit(ctx, wanted);
     if (s != GC_OK) return s;
     if (core && (s = gc_alloc(ctx, &g->rank, g->cap_N, "core ranks")) != GC_OK) return s;

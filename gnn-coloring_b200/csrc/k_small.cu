@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__re
     if (t < sizeof(DevState) / 4)  // (the host's copy)
         reinterpret_cast<uint32_t *>(state)[t] = t == offsetof(DevState, max_color) / 4    ? top
                                                  : t == offsetof(DevState, invalid) / 4    ? invalid
-                                                 : t == offsetof(DevState, flow_stall) / 4 ? (done ? 0u : 1u)
+                                                 : t == offsetof(DevState, flow_stall) / 4 ? (done ? 0u : FLOW_STUCK)
                                                                                            : 0u;
 }
 
