@@ -277,11 +277,11 @@ gc_status reupload_overlapped(gc_ctx *ctx, gc_graph *g, const uint32_t *V, const
 }
 
 // Colors by the current keys: the dataflow kernels where the graph allows them, else the tickets.  The
-// dataflow's result stands only once the state shows that it did not stall (`*unread` is then true:
-// the caller reads the state, and calls color_by_tickets when flow_stall is set).
+// result stands only once the state shows that they did not stop (`*unread` is then true: the caller
+// reads the state, and calls color_by_tickets when flow_stall is set).
 gc_status color_by_keys(gc_ctx *ctx, gc_graph *g, bool *unread) {
-    *unread = gc_flow_eligible(g);
-    if (!*unread) return gc_jp_color(g);
+    *unread = true;
+    if (!gc_flow_eligible(g)) return gc_jp_color(g);
     gc_status s = gc_jp_flow(g);
     if (s != GC_OK) return s;
     g->has_colors = false;  // (until the state has been read)
@@ -289,7 +289,7 @@ gc_status color_by_keys(gc_ctx *ctx, gc_graph *g, bool *unread) {
     return GC_OK;
 }
 
-// After a dataflow coloring that stopped.
+// After a coloring that stopped.
 gc_status color_by_tickets(gc_ctx *ctx, gc_graph *g) {
     const bool narrow = ctx->hstate->flow_stall == gc::FLOW_NARROW;
     gc_status s = gc_reset_state(ctx);
@@ -312,7 +312,7 @@ gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *co
         }
     }
     if ((s = gc_reset_state(ctx)) != GC_OK) return s;
-    bool unread = false;  // a dataflow coloring whose stall flag has not been read
+    bool unread = false;  // a coloring whose stall flag has not been read
     if (first && (s = color_by_keys(ctx, g, &unread)) != GC_OK) return s;
     for (int it = 0; it < rounds;) {
         // the next keys are these colors: they must be known to stand
@@ -322,7 +322,6 @@ gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *co
             if ((by_class || unread) && (s = gc_read_state(ctx)) != GC_OK) return s;
             if (!unread || !ctx->hstate->flow_stall) break;
             if ((s = color_by_tickets(ctx, g)) != GC_OK) return s;
-            unread = false;
         }
         unread = false;
         if (by_class) {
@@ -339,7 +338,6 @@ gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *co
         if ((s = gc_read_state(ctx)) != GC_OK) return s;
         if (!unread || !ctx->hstate->flow_stall) break;
         if ((s = color_by_tickets(ctx, g)) != GC_OK) return s;
-        unread = false;
     }
     g->has_colors = true;
     if (colors_used) g->colors_used = *colors_used = gc_colors_of_state(g);

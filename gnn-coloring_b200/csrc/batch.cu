@@ -267,7 +267,7 @@ gc_status fill_graphs(gc_batch *b, uint32_t G, const uint32_t *n, const uint32_t
 
 // Priorities, coloring, Culberson rounds, per-graph statistics and their read-back, all queued
 // on the context's stream without a host synchronisation (so that it can be captured).
-gc_status queue_pipeline(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor) {
+gc_status queue_pipeline(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor, bool narrow) {
     gc_ctx *ctx = b->ctx;
     gc_graph *g = b->g;
     gc_status s;
@@ -277,13 +277,13 @@ gc_status queue_pipeline(gc_batch *b, gc_heuristic h, const gc_model *m, int rec
     if (s != GC_OK) return s;
     g->key_kind = (int)h;
     g->has_keys = true;
-    if ((s = gc_jp_color(g)) != GC_OK) return s;
+    if ((s = gc_jp_color(g, narrow)) != GC_OK) return s;
     if (recolor > 0 && gc_rounds_eligible(g)) {
         if ((s = gc_culberson_rounds(g, recolor, g->max_deg + 1)) != GC_OK) return s;
     } else {
         for (int it = 0; it < recolor; it++) {
             if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
-            if ((s = gc_jp_color(g)) != GC_OK) return s;
+            if ((s = gc_jp_color(g, narrow)) != GC_OK) return s;
         }
     }
     if ((s = gc_segment_stats(g)) != GC_OK) return s;
@@ -294,11 +294,18 @@ gc_status queue_pipeline(gc_batch *b, gc_heuristic h, const gc_model *m, int rec
                                               ctx->stream), "read device state");
 }
 
-// Waits for a queued pipeline and turns its statistics into color counts.
-gc_status finish_pipeline(gc_batch *b, int32_t *colors) {
+// Waits for a queued pipeline and turns its statistics into color counts.  One whose coloring was found narrow runs
+// again, with most tickets in the cluster; `narrow` tells.
+gc_status finish_pipeline(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor, int32_t *colors, bool *narrow) {
     gc_ctx *ctx = b->ctx;
     gc_status s;
-    if ((s = gc_check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "batch execution")) != GC_OK) return s;
+    *narrow = false;
+    for (;;) {
+        if ((s = gc_check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "batch execution")) != GC_OK) return s;
+        if (*narrow || ctx->hstate->flow_stall != gc::FLOW_NARROW) break;
+        *narrow = true;
+        if ((s = queue_pipeline(b, h, m, recolor, true)) != GC_OK) return s;
+    }
     if ((s = gc_check_hstate(ctx)) != GC_OK) return s;
     if (colors)
         for (uint32_t i = 0; i < b->G; i++) colors[i] = b->h_stat[2 * i + 1] ? 0 : std::max(b->h_stat[2 * i], 1);
@@ -317,7 +324,8 @@ gc_status check_heuristic(gc_ctx *ctx, gc_heuristic h, const gc_model *m) {
 }
 
 // One uncaptured pass; with `ms` set, timed with CUDA events on the stream.
-gc_status direct_pass(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor, int32_t *colors, float *ms) {
+gc_status direct_pass(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor, int32_t *colors, float *ms,
+                      bool *found_narrow = nullptr) {
     gc_ctx *ctx = b->ctx;
     gc_status s;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -329,9 +337,15 @@ gc_status direct_pass(gc_batch *b, gc_heuristic h, const gc_model *m, int recolo
         }
         cudaEventRecord(e0, ctx->stream);
     }
-    s = queue_pipeline(b, h, m, recolor);
+    bool narrow = false;
+    s = queue_pipeline(b, h, m, recolor, false);
     if (ms && s == GC_OK) cudaEventRecord(e1, ctx->stream);
-    if (s == GC_OK) s = finish_pipeline(b, colors);
+    if (s == GC_OK) s = finish_pipeline(b, h, m, recolor, colors, &narrow);
+    if (found_narrow) *found_narrow = narrow;
+    if (ms && s == GC_OK && narrow) {  // (the pass that ran again counts too)
+        cudaEventRecord(e1, ctx->stream);
+        s = gc_check_cuda(ctx, cudaEventSynchronize(e1), "event");
+    }
     if (ms) {
         if (s == GC_OK) s = gc_check_cuda(ctx, cudaEventElapsedTime(ms, e0, e1), "event timing");
         cudaEventDestroy(e0);
@@ -340,7 +354,7 @@ gc_status direct_pass(gc_batch *b, gc_heuristic h, const gc_model *m, int recolo
     return s;
 }
 
-gc_status capture(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor, BatchCapture *out) {
+gc_status capture(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor, bool narrow, BatchCapture *out) {
     gc_ctx *ctx = b->ctx;
     gc_status s;
     if ((s = gc_check_cuda(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed), "begin capture")) !=
@@ -349,7 +363,7 @@ gc_status capture(gc_batch *b, gc_heuristic h, const gc_model *m, int recolor, B
     const uint64_t l0 = ctx->launches;
     const bool prof = ctx->prof;
     ctx->prof = false;  // no event records inside the graph
-    s = queue_pipeline(b, h, m, recolor);
+    s = queue_pipeline(b, h, m, recolor, narrow);
     ctx->prof = prof;
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
@@ -623,15 +637,18 @@ gc_status gc_batch_color(gc_ctx *ctx, gc_batch *b, gc_heuristic h, const gc_mode
         if (c.h == (int)h && c.param == param && c.layers == layers && c.md == md && c.recolor == recolor) hit = &c;
     if (!hit) {
         // first pass: runs directly (this also allocates every lazily allocated buffer), then the
-        // same sequence is captured for the next calls
-        if ((s = direct_pass(b, h, m, recolor, colors, nullptr)) != GC_OK) return s;
+        // same sequence is captured for the next calls.  Narrow or not is a property of the graphs and their
+        // priorities, so the capture starts with it -- once a second pass, with warm caches, has found the same
+        bool narrow = false;
+        if ((s = direct_pass(b, h, m, recolor, colors, nullptr, &narrow)) != GC_OK) return s;
+        if (narrow && (s = direct_pass(b, h, m, recolor, colors, nullptr, &narrow)) != GC_OK) return s;
         BatchCapture c;
         c.h = (int)h;
         c.param = param;
         c.layers = layers;
         c.md = md;
         c.recolor = recolor;
-        if ((s = capture(b, h, m, recolor, &c)) != GC_OK) return s;
+        if ((s = capture(b, h, m, recolor, narrow, &c)) != GC_OK) return s;
         b->caps.push_back(c);
         g->has_colors = true;
         return GC_OK;
@@ -640,7 +657,8 @@ gc_status gc_batch_color(gc_ctx *ctx, gc_batch *b, gc_heuristic h, const gc_mode
     ctx->launches += hit->launches;
     g->key_kind = (int)h;
     g->has_keys = g->has_colors = true;
-    return finish_pipeline(b, colors);
+    bool narrow = false;
+    return finish_pipeline(b, h, m, recolor, colors, &narrow);
 }
 
 gc_status gc_batch_color_once(gc_ctx *ctx, gc_batch *b, gc_heuristic h, const gc_model *m, int recolor,

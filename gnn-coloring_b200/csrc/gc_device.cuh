@@ -30,12 +30,12 @@ struct DevState {
     unsigned int isolated;      // preparation: vertices without neighbours (outside the hub list)
     unsigned int first_colors;  // Culberson rounds: colors of the coloring they start from
     unsigned int core_pred;     // coloring: predecessors of the core's tickets
-    unsigned int flow_stall;    // coloring: the dataflow kernel stopped before every vertex was queued (FlowStop)
+    unsigned int flow_stall;    // coloring: a kernel stopped before every vertex had its color (FlowStop)
 };
 
 enum FlowStop : unsigned int {
     FLOW_STUCK = 1u,   // nothing moved (a CSR that is not symmetric), or a small graph's kernel refused
-    FLOW_NARROW = 2u,  // few vertices become ready at a time: a cluster is faster
+    FLOW_NARROW = 2u,  // few vertices get their colors at a time: a cluster is faster
 };
 
 enum DevErr : unsigned int {

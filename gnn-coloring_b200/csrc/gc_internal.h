@@ -253,8 +253,9 @@ gc_status gc_priority_gnn(gc_graph *g, const gc_model *m);         // GraphSAGE 
 // N (ERR_BOUND, reported by the next gc_read_state) and writes row 0 for one that is out of range.
 gc_status gc_gnn_rows_begin(gc_graph *g);
 gc_status gc_gnn_row_ids(gc_graph *g, uint32_t first, uint32_t count);
-// JP by current keys in ticket order (k_jp.cu).  `narrow`: few vertices become ready at a time, so as many of the
-// first tickets as fit are colored inside one cluster.
+// JP by current keys in ticket order (k_jp.cu).  Queued only, as gc_jp_flow: a flow_stall of FLOW_NARROW says that few
+// vertices got their colors at a time, and that it must run again with `narrow`, which colors as many of the first
+// tickets as fit inside one cluster and does not stop.
 gc_status gc_jp_color(gc_graph *g, bool narrow = false);
 // JP by current keys as a dataflow, on graphs of small maximum degree (k_flow.cu).  Queued only: once
 // the state has been read, a set flow_stall means that the colors are incomplete and gc_jp_color must

@@ -975,6 +975,59 @@ __device__ __forceinline__ int color_light(const uint32_t *__restrict__ list, ui
     return __ffsll((long long)~used);  // at most 63 bits are set: a free color <= 64 exists
 }
 
+// A narrow DAG (a band with long lists, a wheel) has few vertices in flight here, 0.5 to 1.3 us per hop, where the
+// cluster takes 0.1 to 0.3.  So CTA 0 first watches a sample of the tickets for two windows of 133 us, and stops the
+// coloring when in both they got their colors at fewer than NARROW_RATE a microsecond (at 1.965 GHz), while half of
+// them and four windows' work are still to come: no more tickets, and -1 for every color, which ends all waits.  The
+// host then colors the graph with as many tickets as fit in the cluster.  (R-MAT of 2^18 vertices in a batch, largest
+// degree first, spends one window in its clique of hubs, and is done in the next.)  With more tickets than NARROW_MAX
+// the cluster would take too few of them.  First fit, not watched / watched: wheels of
+// 9,000 and 50,000 vertices 6.7 / 2.7 and 37.5 / 21.4 ms, 30,000 rows of a band matrix with 100 entries on either side
+// 24.4 / 12.3, 50,000 with 200 44.2 / 29.3.  (As a function of its own the watch cost the kernel 3 %.)
+constexpr uint32_t NARROW_RATE = 16, NARROW_WINDOWS = 2, NARROW_MHZ = 1965, NARROW_MIN = 512, NARROW_MAX = 131072, NARROW_SAMPLES = 4;
+
+__device__ __forceinline__ void ticket_watch(const uint4 *__restrict__ rec, int *color, DevState *st, uint32_t window) {
+    const uint32_t n = ld_relaxed_u32(&st->ordered), samples = min(n, NARROW_SAMPLES * blockDim.x);
+    if (n < NARROW_MIN || n > NARROW_MAX) return;
+    uint32_t v[NARROW_SAMPLES];
+#pragma unroll
+    for (uint32_t k = 0; k < NARROW_SAMPLES; k++) {
+        const uint32_t i = k * blockDim.x + threadIdx.x;
+        v[k] = i < samples ? rec[(unsigned long long)i * n / samples].x : 0xffffffffu;
+    }
+    uint32_t since = 0, first = 0, start = 0, windows = 0;
+    for (bool begin = true;;) {
+        int c[NARROW_SAMPLES];
+#pragma unroll
+        for (uint32_t k = 0; k < NARROW_SAMPLES; k++) c[k] = v[k] != 0xffffffffu ? ld_relaxed(color + v[k]) : 0;
+        uint32_t done = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < NARROW_SAMPLES; k++) done += __syncthreads_count(c[k] != 0);
+        if (done == samples || __syncthreads_or(threadIdx.x == 0 && ld_relaxed_u32(&st->err))) return;
+        if (begin) {
+            first = done;
+            if (!windows) start = done;
+            since = (uint32_t)clock();
+            begin = false;
+        }
+        const uint32_t dt = (uint32_t)clock() - since;
+        if (__syncthreads_or(threadIdx.x == 0 && dt >= window)) {
+            const unsigned long long got = (unsigned long long)(done - first) * n / samples, left = samples - done;
+            const bool narrow = got * NARROW_MHZ < (unsigned long long)dt * NARROW_RATE && 2 * left >= samples - start &&
+                                left * n / samples * dt >= 4 * got * window;
+            if (!__syncthreads_or(threadIdx.x == 0 && narrow)) return;
+            if (++windows == NARROW_WINDOWS) break;
+            begin = true;
+        }
+    }
+    if (threadIdx.x == 0) {
+        st_relaxed_u32(&st->flow_stall, FLOW_NARROW);
+        atomicMax(&st->ticket, n);
+        atomicMax(&st->ticket_light, n);
+    }
+    for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) st_relaxed(color + rec[t].x, -1);
+}
+
 // A warp takes its next ticket only when it is free: a ticket held ahead by a warp still waiting on
 // its current vertex would stall every vertex that waits on the held one (measured several times
 // slower on R-MAT 22).
@@ -991,7 +1044,8 @@ __global__ void __launch_bounds__(COLOR_WARPS_PER_CTA * 32, 5) k_jp_color(const 
                                                                        unsigned long long *fmask,
                                                                        const unsigned long long *epoch_word,
                                                                        const uint4 *__restrict__ split, uint32_t cap,
-                                                                       int light_warps) {
+                                                                       int light_warps, uint32_t window) {
+    if (window && blockIdx.x == 0) ticket_watch(rec, color, st, window);
     __shared__ uint32_t forbid[COLOR_WARPS_PER_CTA][32];
     __shared__ uint32_t pending[COLOR_WARPS_PER_CTA][PENDING];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1060,7 +1114,7 @@ __global__ void __launch_bounds__(COLOR_THREADS, 6) k_jp_big_leaves(const uint32
                                                                  DevState *st, unsigned int spin_limit) {
     __shared__ uint32_t forbid[COLOR_WARPS][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t n = st->big_leaves;
+    const uint32_t n = st->flow_stall ? 0u : st->big_leaves;  // (a coloring that stopped leaves neighbours without colors)
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps) {
         const uint32_t u = big[i];
@@ -1207,8 +1261,14 @@ __global__ void k_keys_from_colors(const int *__restrict__ color, uint32_t N, ui
 // Also advances the epoch of the published forbidden colors (never 0: the buffer starts zeroed).
 // The ordered kernel's first ticket: past the core tickets the cluster colored, of kmax (0: none, or
 // streams without them).
+// In a captured pass a round may follow a coloring that stopped: its colors are none, waits on them would run to
+// their limit, and the pass is thrown away, so there are no tickets then.
 __global__ void k_reset_ticket(DevState *st, unsigned long long *epoch_word, uint32_t kmax = 0) {
     st->ticket = core_size(st, kmax);
+    if (st->flow_stall) {
+        st->ticket = st->ordered;
+        st->n_heavy = st->n_light = 0;
+    }
     st->big_leaves = 0;
     if (epoch_word) {
         const unsigned long long e = (*epoch_word + 1) & 0xffffffffull;
@@ -1268,8 +1328,10 @@ gc_status core_cluster_config(gc_ctx *ctx) {
 // Core tickets wanted for a coloring.  None up to 65,536 vertices, whose clique of hubs is small (sort to
 // leaves, without / with a core: R-MAT 50,000 x 10 LF 129 / 148 us, FF 118 / 141, 20,000 x 24 141 / 149, 132 / 148;
 // 100,003 x 16 179 / 179, 157 / 180; 300,007 x 32 LF 342 / 264; 2^22 x 32 1,517 / 1,188; batches of 8,000 vertices
-// 123 / 149, 132 / 159).
-// Above that the device decides (core_size): the hubs must come first in the ticket order.  Then the first
+// 123 / 149, 132 / 159).  Dense graphs -- one in CORE_GRAPH_DENSE of all possible entries and more -- have one all
+// the same, of CORE_MAX tickets: their chains go through everything (first fit, without / with: cliques of 600 535 /
+// 360 us, of 2,000 8,281 / 6,170, Erdos-Renyi 5,000 x 400 360 / 238, 10,000 x 400 417 / 302; 2,000 x 200 208 / 198).
+// Above 65,536 the device decides (core_size): the hubs must come first in the ticket order.  Then the first
 // 2,048 tickets hold a good part of the K^2 / 2 predecessors that a clique would have: R-MAT of 131,072 / 2^20
 // vertices by LF, SL and LLF 0.10 / 0.34, likewise by the weights of a trained GNN (R-MAT 2^11: as LF to 1 %).  By FF
 // it is 0.02 / 0.03, by random GNN weights or random priorities 0.001 to 0.004, and then the ticket kernel
@@ -1277,7 +1339,7 @@ gc_status core_cluster_config(gc_ctx *ctx) {
 // / 1,681; the empty core kernels cost 15).  The line is 2 / CORE_DENSE.  Batches always have a core above
 // 2^19 vertices and none below (without / with: 20 graphs, 163,000 vertices, LF 249 / 283, GNN2 434 / 453; 64 graphs,
 // 2.2 M, LF 1,172 / 1,110, GNN2 2,287 / 2,245).
-constexpr uint32_t CORE_DEFAULT = 2048, CORE_MIN_N = 65536, CORE_MIN_BATCH = 1u << 19;
+constexpr uint32_t CORE_DEFAULT = 2048, CORE_MIN_N = 65536, CORE_MIN_BATCH = 1u << 19, CORE_GRAPH_DENSE = 32;
 
 uint32_t core_tickets(const gc_graph *g, bool narrow) {
     const uint32_t most = g->ctx->jp_core_max;
@@ -1342,6 +1404,8 @@ gc_status gc_jp_color(gc_graph *g, bool narrow) {
         g->has_colors = true;
         return GC_OK;
     }
+    const bool by_rule = ctx->jp_core_max == GC_CORE_AUTO;  // (a core that was asked for is what it is)
+    narrow = narrow || (by_rule && g->n_seg <= 1 && (uint64_t)g->M * CORE_GRAPH_DENSE >= (uint64_t)N * N);
     if ((s = gc_alloc(ctx, &g->P, g->cap_M, "predecessor lists")) != GC_OK) return s;
     if ((s = gc_alloc(ctx, &g->pc, g->cap_N, "predecessor counts")) != GC_OK) return s;
     if ((s = gc_alloc(ctx, &g->order, g->cap_N, "ticket order")) != GC_OK) return s;
@@ -1372,7 +1436,7 @@ gc_status gc_jp_color(gc_graph *g, bool narrow) {
             ctx->launches += 2;
         }
         k_jp_init_colors<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(g->pc, N, g->color, ctx->dstate,
-                                                                narrow || ctx->jp_core_max != GC_CORE_AUTO || g->n_seg ? CORE_FORCED : 0u);
+                                                                narrow || !by_rule || g->n_seg ? CORE_FORCED : 0u);
         ctx->launches++;
     }
     if ((s = gc_check_launch(ctx, "jp split")) != GC_OK) return s;
@@ -1437,7 +1501,7 @@ gc_status gc_jp_color(gc_graph *g, bool narrow) {
         ProfScope ps(ctx, "jp_color", ctx->stream);
         k_jp_color<<<ctx->num_sms * blocks, COLOR_WARPS_PER_CTA * 32, 0, ctx->stream>>>(
             g->jprec, g->P, g->pc, g->key, g->color, ctx->dstate, ctx->spin_limit, tight, nap, fmask, epoch_word, split,
-            g->cap_N, light_warps);
+            g->cap_N, light_warps, by_rule && !narrow ? ctx->narrow_window : 0u);
         ctx->launches++;
     }
     // 4. leaves

@@ -49,11 +49,15 @@ enum { RC_HUB = 0, RC_MED, RC_LIGHT, RC_CTA, RC_N_HUB, RC_N_MED, RC_WORDS = 8 };
 __device__ __forceinline__ uint32_t tier_of(uint32_t d) { return d > ROUND_MED_DEG ? 2u : d > ROUND_LIGHT_DEG ? 1u : 0u; }
 
 // Old colors from the coloring (first round) or from the last round's new colors; the sort keys, with
-// the tier above key_bits when the graph has more than the light one, and the tiers' sizes.
+// the tier above key_bits when the graph has more than the light one, and the tiers' sizes.  In a captured pass the
+// coloring before may have stopped: its colors are none, waits on them would run to their limit, and the pass is
+// thrown away, so all vertices count as taken then.
 template <typename T>
 __global__ void __launch_bounds__(256) k_round_begin(const int *__restrict__ color, T *__restrict__ word,
                                                      const uint32_t *__restrict__ V, uint32_t N, int tiers, int key_bits,
-                                                     uint32_t *__restrict__ key, uint32_t *__restrict__ ctr) {
+                                                     uint32_t *__restrict__ key, uint32_t *__restrict__ ctr,
+                                                     const DevState *st) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && st->flow_stall) ctr[RC_HUB] = ctr[RC_MED] = ctr[RC_LIGHT] = N;
     constexpr int HALF = 4 * sizeof(T);  // bits of a color
     const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t hubs = 0, meds = 0;
@@ -519,10 +523,10 @@ gc_status gc_culberson_rounds(gc_graph *g, int rounds, uint32_t colors) {
             ProfScope ps(ctx, "round_begin", ctx->stream);
             if (narrow)
                 k_round_begin<uint16_t><<<sweep, 256, 0, ctx->stream>>>(it ? nullptr : g->color, word16, g->V, N, 0, key_bits,
-                                                                        g->key, g->round_ctr);
+                                                                        g->key, g->round_ctr, ctx->dstate);
             else
                 k_round_begin<uint32_t><<<sweep, 256, 0, ctx->stream>>>(it ? nullptr : g->color, g->pc, g->V, N, tiers,
-                                                                        key_bits, g->key, g->round_ctr);
+                                                                        key_bits, g->key, g->round_ctr, ctx->dstate);
             ctx->launches++;
         }
         if ((s = gc_sort_order_bits(g, key_bits + 2 * tiers, false, &ctx->dstate->ordered)) != GC_OK) return s;

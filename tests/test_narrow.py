@@ -101,3 +101,64 @@ def test_narrow_off():
     assert np.array_equal(g.colors(), O.greedy_color(N, V, E, g.priorities())[0])
     g.close()
     ctx.close()
+
+
+def _wheel(n):
+    i = np.arange(1, n)
+    return _pairs(n, np.concatenate([i, np.zeros(n - 1, int)]), np.concatenate([np.where(i + 1 < n, i + 1, 1), i]))
+
+
+@pytest.mark.parametrize("name", ["wheel", "band100", "band200"])
+def test_narrow_tickets_match_oracle(gpu_ctx, name):
+    N, V, E = {"wheel": lambda: _wheel(12000), "band100": lambda: _band(20000, 100), "band200": lambda: _band(30000, 200)}[name]()
+    g = gcn.Graph(gpu_ctx, N, V, E)
+    for heur in ("FF", "SL"):
+        g.priority(heur)
+        ref, _ = O.greedy_color(N, V, E, g.priorities())
+        for rounds, count in ((0, True), (0, False), (2, True)):
+            want = O.culberson(N, V, E, ref, rounds) if rounds else ref
+            g.priority(heur)
+            names, got = _kernels(gpu_ctx, lambda: g.color(rounds, count=count))
+            assert "jp_core" in names and "jp_flow" not in names, names
+            assert got == (O.validate(N, V, E, want) if count else 0)
+            assert np.array_equal(g.colors(), want), (name, heur, rounds)
+    g.close()
+
+
+@pytest.mark.parametrize("classes", ["0", "1"])
+def test_narrow_batches_match_oracle(classes):
+    """The first pass is found narrow and runs again; the captured one starts with the cluster.  A batch pass with
+    streams is stopped like one without."""
+    graphs = [_band(9000, 1), _band(3000, 15), _strip(2000, 3), _wheel(500), _band(2, 1)]
+    for light in ("0", str(1 << 19)):
+        ctx = _context(GC_JP_CLASSES=classes, GC_JP_LIGHT_MIN=light)
+        b = gcn.Batch(ctx, graphs=graphs)
+        for heur in ("LF", "FF"):
+            ref = [O.greedy_color(*g, O.ordering(heur, *g))[0] for g in graphs]
+            for rounds in (0, 1):
+                want = [O.culberson(*g, c, rounds) if rounds else c for g, c in zip(graphs, ref)]
+                for _ in range(3):
+                    counts = b.color(heur, recolor=rounds)
+                    assert np.array_equal(b.colors(), np.concatenate(want)), (heur, rounds, light)
+                    assert counts.tolist() == [O.validate(*g, c) for g, c in zip(graphs, want)]
+        b.close()
+        ctx.close()
+
+
+def test_rounds_after_a_stopped_coloring_do_not_wait(gpu_ctx):
+    """The rounds queued behind a coloring that stops have no colors to work on; their waits must not run to the limit
+    (seconds)."""
+    import time
+    graphs = [_band(20000, 2), _wheel(3000), _strip(3000, 3)]
+    ref = [O.greedy_color(*g, O.ordering("LF", *g))[0] for g in graphs]
+    want = np.concatenate([O.culberson(*g, c, 2) for g, c in zip(graphs, ref)])
+    for classes in ("1", "0"):  # class by class, by tickets
+        ctx = _context(GC_JP_CLASSES=classes)
+        b = gcn.Batch(ctx, graphs=graphs)
+        b.color("FF")  # (kernels are loaded)
+        t = time.perf_counter()
+        b.color("LF", recolor=2)
+        assert time.perf_counter() - t < 0.5
+        assert np.array_equal(b.colors(), want)
+        b.close()
+        ctx.close()
