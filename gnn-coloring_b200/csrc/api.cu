@@ -300,6 +300,7 @@ gc_status color_by_tickets(gc_ctx *ctx, gc_graph *g) {
 // when it is asked for.  The last coloring's errors, stall flag and statistics come back in one read.
 gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *colors_used) {
     gc_status s;
+    bool narrow = false;
     if ((first || rounds > 0) && gc_small_eligible(g, rounds)) {
         if (!first) {
             if ((s = gc_keys_from_colors(g)) != GC_OK) return s;
@@ -310,10 +311,13 @@ gc_status color_rounds(gc_ctx *ctx, gc_graph *g, bool first, int rounds, int *co
             if (colors_used) g->colors_used = *colors_used = gc_colors_of_state(g);
             return GC_OK;
         }
+        narrow = first && ctx->hstate->flow_stall == gc::FLOW_NARROW;
     }
     if ((s = gc_reset_state(ctx)) != GC_OK) return s;
     bool unread = false;  // a coloring whose stall flag has not been read
-    if (first && (s = color_by_keys(ctx, g, &unread)) != GC_OK) return s;
+    if (narrow) s = gc_jp_color(g, true);
+    else if (first) s = color_by_keys(ctx, g, &unread);
+    if (s != GC_OK) return s;
     for (int it = 0; it < rounds;) {
         // the next keys are these colors: they must be known to stand
         const bool by_class = gc_rounds_eligible(g);

@@ -261,6 +261,7 @@ gc_status gc_jp_color(gc_graph *g, bool narrow = false);
 // the state has been read, a set flow_stall means that the colors are incomplete and gc_jp_color must
 // run instead (narrow: FLOW_NARROW).
 bool gc_flow_eligible(const gc_graph *g);
+inline bool gc_nearly_complete(const gc_graph *g) { return 4ull * g->M >= (uint64_t)g->N * g->N; }
 gc_status gc_jp_flow(gc_graph *g);
 size_t gc_flow_queue_words(uint32_t cap_N);
 gc_status gc_keys_from_colors(gc_graph *g);                        // Culberson step (k_jp.cu)

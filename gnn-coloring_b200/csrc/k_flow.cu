@@ -508,11 +508,13 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
 // vertices, dataflow / tickets: random priorities 429 / 248, first fit 213 / 187).  Larger degrees would put long
 // lists on the chain, and power-law graphs have their chains colored inside one cluster (k_jp_core).
 // Plain graphs only: a batch is captured, and the stall flag needs the host.
-constexpr uint32_t FLOW_WIDE_MAX_N = 1u << 20, FLOW_WIDE_MEAN = 4;
+// (And no nearly complete graphs: one chain, for the cluster.)
+constexpr uint32_t FLOW_WIDE_MAX_N = 1u << 20, FLOW_WIDE_MEAN = 4, FLOW_CLIQUE = 100;
 
 bool gc_flow_eligible(const gc_graph *g) {
     const bool wide = g->N <= FLOW_WIDE_MAX_N && g->M / FLOW_WIDE_MEAN >= g->N;
     const uint32_t widest = wide ? 32u * FLOW_WIDE : 64u;
+    if (g->N > FLOW_CLIQUE && gc_nearly_complete(g)) return false;
     return g->n_seg == 0 && g->N > 0 && g->max_deg < std::min(g->ctx->flow_max_deg, widest);
 }
 

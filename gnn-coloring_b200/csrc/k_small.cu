@@ -32,6 +32,11 @@ using namespace gc;
 
 constexpr int SMALL_THREADS = 1024;
 constexpr uint32_t HEAVY = 96, LONG = 64;
+// A coloring whose levels are mostly of SLIM vertices or fewer is a chain, 0.6 us a level here and 0.1 to 0.3 among
+// tickets inside a cluster (k_jp_core).  So after SLIM_LEVELS of those, with half of the vertices to come, this kernel
+// gives up (FLOW_NARROW): 3,000 vertices in a path 1.78 / 0.93 ms, 2,900 rows of a band with 15 entries on either side 1.72 /
+// 0.57.  (One warp that colors such levels without barriers takes 0.42 us for each.)
+constexpr uint32_t SLIM = 3, SLIM_LEVELS = 128;
 constexpr size_t SMALL_BYTES = 226 * 1024;  // (a CTA may have 227 KB; the rest is static)
 constexpr unsigned int FULL = 0xffffffffu;
 
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__re
     if (t < 3) s.light(t) = s.heavy(t) = 0;
     if (t == 0) invalid = top = sides = 0;
     bool done = true;
-    uint32_t hashes = 0;
+    uint32_t hashes = 0, slim = 0;
     for (int it = 0; it <= rounds; it++) {
         __syncthreads();
         auto found = [&](uint32_t u, uint32_t cnt, bool big) {
@@ -202,6 +207,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__re
             const uint32_t nl = s.light(l), nh = s.heavy(l), next = l == 2 ? 0 : l + 1;
             if (t == 0) s.light(l == 0 ? 2 : l - 1) = s.heavy(l == 0 ? 2 : l - 1) = 0;
             if (nl + nh == 0) break;
+            if (it == 0 && nl + nh <= SLIM && ++slim > SLIM_LEVELS && la + ha < N / 2) break;
             const uint32_t per = nl > nwarps ? 4u : 1u, items = nh + (nl + per - 1) / per;
             const uint32_t lb = la + nl, hb = ha + nh;
             for (uint32_t i = warp; i < items; i += nwarps) {
@@ -220,6 +226,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__re
         __syncthreads();
         if (t < 3) s.light(t) = s.heavy(t) = 0;
         done = la + ha == N;
+        if (done) slim = 0;
         if (!done || it == rounds) break;
         const uint32_t x = s.a_;  // the next keys are these colors
         s.a_ = s.b_;
@@ -244,7 +251,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__re
     if (t < sizeof(DevState) / 4)  // (the host's copy)
         reinterpret_cast<uint32_t *>(state)[t] = t == offsetof(DevState, max_color) / 4    ? top
                                                  : t == offsetof(DevState, invalid) / 4    ? invalid
-                                                 : t == offsetof(DevState, flow_stall) / 4 ? (done ? 0u : FLOW_STUCK)
+                                                 : t == offsetof(DevState, flow_stall) / 4 ? (done ? 0u : slim > SLIM_LEVELS ? FLOW_NARROW : FLOW_STUCK)
                                                                                            : 0u;
 }
 
@@ -256,11 +263,16 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(const uint32_t *__re
 // 88 / 55 us, 2,000 x 16 90 / 71, 3,000 x 24 119 / 109, 4,000 x 12 79 / 87, 6,000 x 8 68 / 93; with two rounds
 // 201 / 89, 208 / 120, 264 / 200, 210 / 168, 203 / 186), against the ticket kernels, whose graphs have long lists
 // and many levels, one of entries (R-MAT 1,000 x 16, 12,000 entries 125 / 86, 1,000 x 32, 21,000 128 / 119, 1,400
-// x 32, 28,000 124 / 145; with two rounds 274 / 164, 320 / 223, 312 / 278, 4,000 x 16, 52,000 371 / 447).
+// x 32, 28,000 124 / 145; with two rounds 274 / 164, 320 / 223, 312 / 278, 4,000 x 16, 52,000 371 / 447).  A quarter
+// of all entries and more makes a chain of nearly all vertices, which the cluster takes faster from some hundred on
+// (tickets / this: cliques of 64 139 / 73 us, of 120 160 / 188, of 140 174 / 243).
+constexpr uint32_t SMALL_CLIQUE = 100;
+
 bool gc_small_eligible(const gc_graph *g, int rounds) {
     if (g->n_seg || !g->N || small_bytes(g->N, g->M) > SMALL_BYTES) return false;
     const uint32_t most = g->ctx->small_max;
     if (most != GC_SMALL_AUTO) return g->N <= std::min<uint32_t>(most, 65535u);
+    if (g->N > SMALL_CLIQUE && gc_nearly_complete(g)) return false;
     return gc_flow_eligible(g) ? g->N <= (rounds ? 6144u : 3072u) : g->M <= (rounds ? 36864u : 20480u);
 }
 
