@@ -976,15 +976,15 @@ __device__ __forceinline__ int color_light(const uint32_t *__restrict__ list, ui
 }
 
 // A narrow DAG (a band with long lists, a wheel) has few vertices in flight here, 0.5 to 1.3 us per hop, where the
-// cluster takes 0.1 to 0.3.  So CTA 0 first watches a sample of the tickets for two windows of 133 us, and stops the
-// coloring when in both they got their colors at fewer than NARROW_RATE a microsecond (at 1.965 GHz), while half of
+// cluster takes 0.1 to 0.3.  So CTA 0 first watches a sample of the tickets for three windows of 133 us, and stops the
+// coloring when in all they got their colors at fewer than NARROW_RATE a microsecond (at 1.965 GHz), while half of
 // them and four windows' work are still to come: no more tickets, and -1 for every color, which ends all waits.  The
-// host then colors the graph with as many tickets as fit in the cluster.  (R-MAT of 2^18 vertices in a batch, largest
-// degree first, spends one window in its clique of hubs, and is done in the next.)  With more tickets than NARROW_MAX
-// the cluster would take too few of them.  First fit, not watched / watched: wheels of
-// 9,000 and 50,000 vertices 6.7 / 2.7 and 37.5 / 21.4 ms, 30,000 rows of a band matrix with 100 entries on either side
-// 24.4 / 12.3, 50,000 with 200 44.2 / 29.3.  (As a function of its own the watch cost the kernel 3 %.)
-constexpr uint32_t NARROW_RATE = 16, NARROW_WINDOWS = 2, NARROW_MHZ = 1965, NARROW_MIN = 512, NARROW_MAX = 131072, NARROW_SAMPLES = 4;
+// host then colors the graph with as many tickets as fit in the cluster.  (R-MAT without a core spends two windows in
+// its clique of hubs, and is done in the third.)  With more tickets than NARROW_MAX the cluster would take too few of
+// them.  First fit, not watched / watched: wheels of
+// 9,000 and 50,000 vertices 6.7 / 2.9 and 37.5 / 21.6 ms, 30,000 rows of a band matrix with 100 entries on either side
+// 24.4 / 12.4, 50,000 with 200 44.2 / 29.4.  (As a function of its own the watch cost the kernel 3 %.)
+constexpr uint32_t NARROW_RATE = 16, NARROW_WINDOWS = 3, NARROW_MHZ = 1965, NARROW_MIN = 512, NARROW_MAX = 131072, NARROW_SAMPLES = 4;
 
 __device__ __forceinline__ void ticket_watch(const uint4 *__restrict__ rec, int *color, DevState *st, uint32_t window) {
     const uint32_t n = ld_relaxed_u32(&st->ordered), samples = min(n, NARROW_SAMPLES * blockDim.x);
@@ -1336,7 +1336,7 @@ gc_status core_cluster_config(gc_ctx *ctx) {
 // vertices by LF, SL and LLF 0.10 / 0.34, likewise by the weights of a trained GNN (R-MAT 2^11: as LF to 1 %).  By FF
 // it is 0.02 / 0.03, by random GNN weights or random priorities 0.001 to 0.004, and then the ticket kernel
 // follows their chains as fast beside all else (FF 300,007 269 / 310, 2^22 2,545 / 2,600; GNN3 369 / 410, 1,521
-// / 1,681; the empty core kernels cost 15).  The line is 2 / CORE_DENSE.  Batches always have a core above
+// / 1,681; the empty core kernels cost 15).  The line is 2 / CORE_DENSE.  Batches of several graphs always have a core above
 // 2^19 vertices and none below (without / with: 20 graphs, 163,000 vertices, LF 249 / 283, GNN2 434 / 453; 64 graphs,
 // 2.2 M, LF 1,172 / 1,110, GNN2 2,287 / 2,245).
 constexpr uint32_t CORE_DEFAULT = 2048, CORE_MIN_N = 65536, CORE_MIN_BATCH = 1u << 19, CORE_GRAPH_DENSE = 32;
@@ -1345,7 +1345,7 @@ uint32_t core_tickets(const gc_graph *g, bool narrow) {
     const uint32_t most = g->ctx->jp_core_max;
     if (most != GC_CORE_AUTO) return most;
     if (narrow) return CORE_MAX;
-    return g->N > (g->n_seg ? CORE_MIN_BATCH : CORE_MIN_N) ? CORE_DEFAULT : 0u;
+    return g->N > (g->n_seg > 1 ? CORE_MIN_BATCH : CORE_MIN_N) ? CORE_DEFAULT : 0u;
 }
 
 // The most core tickets, up to kmax, whose replicas and published sets fit the core kernel's shared
@@ -1436,7 +1436,7 @@ gc_status gc_jp_color(gc_graph *g, bool narrow) {
             ctx->launches += 2;
         }
         k_jp_init_colors<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(g->pc, N, g->color, ctx->dstate,
-                                                                narrow || !by_rule || g->n_seg ? CORE_FORCED : 0u);
+                                                                narrow || !by_rule || g->n_seg > 1 ? CORE_FORCED : 0u);
         ctx->launches++;
     }
     if ((s = gc_check_launch(ctx, "jp split")) != GC_OK) return s;
