@@ -37,10 +37,11 @@ constexpr uint32_t ROUND_LIGHT_DEG = 64;   // eight lanes per vertex, colors in 
 constexpr uint32_t ROUND_MED_DEG = 1024;   // a warp per vertex
 constexpr int ROUND_THREADS = 256;
 constexpr int ROUND_MED_WARPS = 2;         // of a mixed CTA's warps, those on the middle tier while it lasts
+constexpr uint32_t ROUND_MED_MANY = 48;    // middle vertices per CTA above which all its warps end up there
 constexpr uint32_t ROUND_HUB_EVERY = 4;    // every fourth CTA takes the top tier while it lasts
 constexpr uint32_t HUB_WORDS = 2048;       // bitmap of colors 1..65,536
 constexpr uint32_t HUB_PEND = 2048;        // uncolored predecessors a CTA remembers
-constexpr uint32_t MED_PEND = 64;          // the same for a warp
+constexpr uint32_t MED_PEND = 64;          // the same for a warp (256: cliques of 600 0.98 -> 1.68 ms a round)
 constexpr uint32_t MED_WINDOW = 1024;      // colors per pass of a warp over its list
 
 // Work counters of a round, zeroed before it.
@@ -459,16 +460,22 @@ __global__ void __launch_bounds__(ROUND_THREADS, 5) k_jp_round(const uint32_t *_
         round_light(order, N, V, E, word, ctr + RC_LIGHT, batch, st, limit);
         return;
     }
+    static_assert(ROUND_THREADS / 32 * MED_PEND <= HUB_PEND && ROUND_THREADS <= HUB_WORDS, "the warps share the CTA's arrays");
     __shared__ uint32_t bm[TIERS ? HUB_WORDS : 1], pend[TIERS ? HUB_PEND : 1], shared[4];
     const uint32_t nh = ctr[RC_N_HUB], nm = ctr[RC_N_MED];
     if (threadIdx.x == 0) shared[3] = atomicAdd(ctr + RC_CTA, 1u);
     __syncthreads();
     if (shared[3] % ROUND_HUB_EVERY == 0) round_hub(order, nh, V, E, word, ctr + RC_HUB, bm, pend, shared, st, limit);
     __syncthreads();
+    // the middle tier by some warps at once, and where it is large by the others too when there are no light vertices
+    // left to take (a round, without / with: 500 complete bipartite graphs of 120 + 120 253 / 191 us, 8,000 cliques of
+    // 120 1,597 / 977, Erdos-Renyi 50,000 x 200 236 / 203; but 30,000 rows of a band of 100 281 / 308)
     const int warp = threadIdx.x >> 5;
-    if (warp < ROUND_MED_WARPS)
-        round_med(order + nh, nm, V, E, word, ctr + RC_MED, bm + 32 * warp, pend + MED_PEND * warp, st, limit);
-    round_light(order + nh + nm, N - nh - nm, V, E, word, ctr + RC_LIGHT, batch, st, limit);
+    const int passes = nm >= ROUND_MED_MANY * gridDim.x ? 3 : 2;
+    for (int pass = warp < ROUND_MED_WARPS ? 0 : 1; pass < passes; pass++) {
+        if (pass == 1) round_light(order + nh + nm, N - nh - nm, V, E, word, ctr + RC_LIGHT, batch, st, limit);
+        else round_med(order + nh, nm, V, E, word, ctr + RC_MED, bm + 32 * warp, pend + MED_PEND * warp, st, limit);
+    }
 }
 
 }  // namespace
