@@ -72,8 +72,8 @@ struct gc_ctx {
     int jp_core_warps = 16;              // core kernel: warps per CTA, 1..32 (GC_JP_CORE_WARPS)
     bool jp_core_decide = true;          // core kernel: early decisions from published seen colors (GC_JP_CORE_DECIDE)
     size_t jp_core_smem = 0;             // core kernel: shared memory per CTA (the device's opt-in maximum)
-    int jp_light_warps = 4;              // batches: warps per CTA on the light stream (0: no split; GC_JP_LIGHT_WARPS)
-    uint32_t jp_light_min = 1u << 19;    // batches of more vertices than this have a light stream (GC_JP_LIGHT_MIN)
+    int jp_light_warps = 4;              // warps per CTA on the light stream (0: no split; GC_JP_LIGHT_WARPS)
+    uint32_t jp_light_min = 1u << 19;    // batches, and graphs without a clique of hubs, of more vertices than this have a light stream (GC_JP_LIGHT_MIN)
     int gnn_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each GNN layer kernel
     uint32_t gnn_warp_deg = GC_GNN_WIDE_DEGREE;  // GNN: above this many neighbours a vertex gets a warp (GC_GNN_WARP_DEGREE)
     uint32_t hub_deg = GC_GNN_HUB_DEGREE;    // plain graphs: above this many neighbours a vertex is a hub (GC_HUB_DEGREE)
