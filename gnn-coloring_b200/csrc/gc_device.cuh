@@ -8,6 +8,7 @@ namespace gc {
 constexpr int FEAT = 16;           // GraphSAGE width (reference src/fast_gnn.c:6)
 constexpr int LAYER_PARAMS = 528;  // 32x16 weights + 16 biases per layer (src/fast_gnn.c:256)
 constexpr int WARP = 32;
+constexpr uint32_t TINY_DEGREE = 4;  // GNN: up to this many neighbours a group's 32 sums are made at once
 
 // Device-side status block, one per context.  Kernels report problems by OR-ing a code into
 // `err` and recording where in `err_info`; the host reads it after a launch sequence.
@@ -30,6 +31,7 @@ struct DevState {
     unsigned int isolated;      // preparation: vertices without neighbours (outside the hub list)
     unsigned int first_colors;  // Culberson rounds: colors of the coloring they start from
     unsigned int core_pred;     // coloring: predecessors of the core's tickets
+    unsigned int tiny;          // preparation: vertices with at most TINY_DEGREE neighbours, of the thin ones
     unsigned int flow_stall;    // coloring: a kernel stopped before every vertex had its color (FlowStop)
 };
 

@@ -163,6 +163,7 @@ struct gc_graph {
     bool gnn_warp_auto = true, hub_auto = true;  // chosen by the graph's size, not set
     uint32_t gnn_warp_now = GC_GNN_WIDE_DEGREE, hub_now = GC_GNN_HUB_DEGREE;  // in force (gc_graph_prepare)
     uint32_t n_thin = 0;             // trailing vorder entries that k_gnn_thin takes
+    bool tiny = false;               // most of those have at most TINY_DEGREE neighbours
     uint32_t n_iso = 0;              // of those, the trailing entries without neighbours (degree schedule only)
                                      // (degree schedule only; 0 with the graph-major schedule)
     // GNN scratch (allocated on first use).  Feature rows (x, y, t01) are stored in degree order:

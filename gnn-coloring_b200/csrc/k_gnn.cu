@@ -337,10 +337,11 @@ __global__ void __launch_bounds__(GNN_THREADS, 4) k_gnn_layer(const uint2 *__res
     // Dynamic hand-out (work_ctr): items are sorted heaviest first, so the warp-tier vertices
     // (work_ctr[0]) and the leading `heavy` four-lane items (work_ctr[1]) go one at a time
     // and spread over the warps; the rest go `grab` at a time (work_ctr[2]).  Otherwise a fixed
-    // stride.  One call site, so the item body is inlined once.
+    // stride.  A part without items costs no atomic.  One call site, so the item body is inlined once.
     const uint32_t n_first = n_wide;
     const uint32_t heavy_end = min(n_items, n_first + heavy);
-    uint32_t phase = 0, cur = 0, end = 0, sit = warp;
+    const uint32_t after_heavy = heavy_end < n_items ? 2u : 3u, after_first = n_first < heavy_end ? 1u : after_heavy;
+    uint32_t phase = n_first ? 0u : after_first, cur = 0, end = 0, sit = warp;
     for (;;) {
         uint32_t it;
         if (work_ctr) {
@@ -348,11 +349,11 @@ __global__ void __launch_bounds__(GNN_THREADS, 4) k_gnn_layer(const uint2 *__res
                 if (phase == 0) {
                     const uint32_t x = grab_work(work_ctr, 1u, lane);
                     if (x < n_first) cur = x, end = x + 1;
-                    else phase = 1;
+                    else phase = after_first;
                 } else if (phase == 1) {
                     const uint32_t x = n_first + grab_work(work_ctr + 1, 1u, lane);
                     if (x < heavy_end) cur = x, end = x + 1;
-                    else phase = 2;
+                    else phase = after_heavy;
                 } else {
                     const uint32_t x = heavy_end + grab_work(work_ctr + 2, grab, lane);
                     if (x < n_items) cur = x, end = min(x + grab, n_items);
@@ -470,7 +471,11 @@ struct LayerArg {
     float w[LAYER_PARAMS];
 };
 
-template <int MODE>
+// TINY: groups whose degrees are at most TINY_DEGREE have the sums of all 32 vertices made at once, so that a step is
+// one load deep (3 layers over a tree of 2^20 vertices 237 -> 205 us, Erdos-Renyi 1 M x 2 243 -> 214, a path of 200,000 88
+// -> 79, 100 stars of 20,000 583 -> 525).  Its registers cost
+// the other groups 5 to 10 %, so the host asks for it where most are such.
+template <int MODE, bool TINY>
 __global__ void __launch_bounds__(THIN_THREADS, 4) k_gnn_thin(const uint2 *__restrict__ vrow, const uint32_t *__restrict__ E,
                                                               const uint32_t *__restrict__ vorder, uint32_t row0, uint32_t first,
                                                               uint32_t n_vorder, const float2 *__restrict__ t01,
@@ -547,8 +552,36 @@ __global__ void __launch_bounds__(THIN_THREADS, 4) k_gnn_thin(const uint2 *__res
                 for (int j = 0; j < FEAT; j++) c[j] = __fmaf_rn(W[i * FEAT + j], a, c[j]);
             }
         } else {
+            const uint32_t dall = TINY ? __reduce_max_sync(FULL, bd.y) : 0xffffffffu;
+            if (TINY && dall <= TINY_DEGREE) {
+                uint32_t id[4], dq[4];
+                float4 s[4];
+#pragma unroll
+                for (int sub = 0; sub < 4; sub++) {
+                    const int v = 8 * sub + (lane >> 2);
+                    const uint32_t beg = __shfl_sync(FULL, bd.x, v);
+                    dq[sub] = __shfl_sync(FULL, bd.y, v);
+                    id[sub] = q < (int)dq[sub] ? ld_stream(E + beg + q) : 0u;
+                    s[sub] = zero4;
+                }
+#pragma unroll
+                for (int k = 0; k < (int)TINY_DEGREE; k++) {
+                    if ((uint32_t)k >= dall) break;
+                    float4 r[4];
+#pragma unroll
+                    for (int sub = 0; sub < 4; sub++) {
+                        const uint32_t e = __shfl_sync(FULL, id[sub], qbase + k);
+                        r[sub] = k < (int)dq[sub] ? __ldg(X4 + (size_t)e * 4 + q) : zero4;
+                    }
+#pragma unroll
+                    for (int sub = 0; sub < 4; sub++)
+                        if (k < (int)dq[sub]) s[sub] = add4(s[sub], r[sub]);
+                }
+#pragma unroll
+                for (int sub = 0; sub < 4; sub++) slab4[chunk(8u * sub + (lane >> 2), q)] = s[sub];
+            }
 #pragma unroll 1
-            for (int sub = 0; sub < 4; sub++) {
+            for (int sub = TINY && dall <= TINY_DEGREE ? 4 : 0; sub < 4; sub++) {
                 const uint32_t v = 8u * sub + (lane >> 2);
                 const uint32_t beg = __shfl_sync(FULL, bd.x, (int)v), d = __shfl_sync(FULL, bd.y, (int)v);
                 const uint32_t dmax = __reduce_max_sync(FULL, d);
@@ -1311,20 +1344,22 @@ gc_status launch_layer(gc_graph *g, const float *Wb, const float *Wh, const floa
         const uint32_t first_thin = g->n_vorder - g->n_thin;
         const int bb = g->n_hubs && ctx->hub_stream && blocks > 1 ? blocks - 1 : blocks;
         if (first_thin) {
-            k_gnn_layer<MODE><<<ctx->num_sms * bb, GNN_THREADS, 0, ctx->stream>>>(
+            // a warp per item at most (a grid of idle CTAs costs a layer of a small graph 2 us)
+            const uint32_t items = g->n_wide_gnn + (first_thin - std::min(first_thin, g->n_wide_gnn) + 7) / 8;
+            const uint32_t grid = std::min<uint32_t>((uint32_t)(ctx->num_sms * bb), (items + GNN_THREADS / 32 - 1) / (GNN_THREADS / 32));
+            k_gnn_layer<MODE><<<grid, GNN_THREADS, 0, ctx->stream>>>(
                 g->vrow, g->Er, g->vorder, g->n_hubs, g->n_wide_gnn, first_thin, g->t01, x, y, g->key, Wb, ctr,
                 ctx->gnn_grab, ctx->gnn_heavy);
             ctx->launches++;
         }
         const uint32_t end_thin = g->n_vorder - n_iso;
         if (end_thin > first_thin) {
-            const uint32_t grid = std::min<uint32_t>((uint32_t)ctx->num_sms * 4,
-                                                     (end_thin - first_thin + THIN_THREADS - 1) / THIN_THREADS);
             LayerArg la;
             memcpy(la.w, Wh, sizeof(la.w));
-            k_gnn_thin<MODE><<<grid, THIN_THREADS, 0, ctx->stream>>>(g->vrow, g->Er, g->vorder, g->n_hubs, first_thin,
-                                                                     end_thin, g->t01, x, y, g->key, la, ctr + 5,
-                                                                     ctx->gnn_grab);
+            const uint32_t grid = std::min<uint32_t>((uint32_t)ctx->num_sms * 4,
+                                                     (end_thin - first_thin + THIN_THREADS - 1) / THIN_THREADS);
+            (g->tiny ? k_gnn_thin<MODE, true> : k_gnn_thin<MODE, false>)<<<grid, THIN_THREADS, 0, ctx->stream>>>(
+                g->vrow, g->Er, g->vorder, g->n_hubs, first_thin, end_thin, g->t01, x, y, g->key, la, ctr + 5, ctx->gnn_grab);
             ctx->launches++;
         }
     }

@@ -42,6 +42,7 @@ __global__ void k_degree_classes(const uint32_t *__restrict__ V, uint32_t N, uin
         }
         if (d > gnn_warp_deg && d <= hub_deg) atomicAdd(&st->gnn_wide, 1u);  // counts the GNN warp tier
         if (d <= thin_deg && d <= gnn_warp_deg) atomicAdd(&st->thin, 1u);     // counts the GNN thin tier
+        if (d <= gc::TINY_DEGREE && d <= gnn_warp_deg) atomicAdd(&st->tiny, 1u);
         if (d == 0) atomicAdd(&st->isolated, 1u);
     }
 }
@@ -83,7 +84,8 @@ __global__ void k_hub_degrees(const uint32_t *__restrict__ V, const uint32_t *__
     }
 }
 
-constexpr uint32_t THIN_WHOLE = 128, THIN_MIN_PER_SM = 1024;  // (32 resident warps of 32 vertices)
+constexpr uint32_t TINY_MUL = 1, TINY_DIV = 2;
+constexpr uint32_t THIN_WHOLE = 128, THIN_SKEW = 16, THIN_MIN_PER_SM = 1024;  // (32 resident warps of 32 vertices)
 
 // Degree thresholds of a graph of M directed edges, where nobody has set them.  A vertex's FP32
 // sums are serial: about 0.03 us a neighbour in the GNN's warp tier and 0.12 us in its four-lane tier,
@@ -171,6 +173,7 @@ gc_status gc_graph_prepare(gc_graph *g) {
         g->giant_rows = 0;
         g->n_vorder = 0;
         g->n_thin = 0;
+        g->tiny = false;
         g->n_iso = 0;
         g->n_wide_gnn = 0;
         return GC_OK;
@@ -190,17 +193,23 @@ gc_status gc_graph_prepare(gc_graph *g) {
     uint32_t n_tasks = ctx->hstate->count, n_hubs = ctx->hstate->count2;
     g->n_wide = ctx->hstate->min_deg;
     // The GNN's thin tier: up to ctx->gnn_thin_deg neighbours, or the whole graph where no vertex has
-    // more than THIN_WHOLE (one kernel per layer instead of two: 3 layers over an Erdos-Renyi graph of 400,000
-    // vertices 297 -> 186 us; in a skewed graph the other tiers run anyway, and groups of up to 64
-    // neighbours only lengthen its tail: R-MAT of 100,003 vertices 230 us with 16, 280 with 64).
+    // more than THIN_WHOLE (half that up to 2^19 vertices) or THIN_SKEW times the mean (one kernel per layer instead of two: 3 layers over an Erdos-Renyi
+    // graph of 400,000 vertices 297 -> 186 us; in a skewed graph the other tiers run anyway, and groups of up to 64
+    // neighbours only lengthen its tail: R-MAT of 100,003 vertices 230 us with 16, 280 with 64, a path of 5,000 with 100
+    // leaves each 176 with 16, 335 throughout; 2,000 cliques of 100 257 with the quad tier, 291 throughout, but 8,000 of
+    // 120 1,220 and 1,193, Erdos-Renyi 1 M x 60 1,162 and 1,111).
     // Below one group for each resident warp the chip is half idle and a vertex's own chain is what
     // counts, which the quad tier keeps shorter: Erdos-Renyi 65,536 90 us here, 80 there; 150,000
     // 136 and 123; 200,000 144 and 139; 400,000 186 and 233; R-MAT 100,003 193 and 183, 1 M 429 and 551.
-    const bool whole = g->max_deg <= THIN_WHOLE && ctx->gnn_thin_auto;
+    const bool whole = g->max_deg <= (g->N > (1u << 19) ? THIN_WHOLE : THIN_WHOLE / 2) && ctx->gnn_thin_auto &&
+                       (uint64_t)g->max_deg * g->N <= (uint64_t)THIN_SKEW * g->M;
     g->n_iso = by_degree ? ctx->hstate->isolated : 0u;  // the last entries of the degree order
     g->n_thin = !by_degree ? 0u : whole ? g->N - n_hubs : ctx->hstate->thin;
     if (ctx->gnn_thin_auto && g->n_thin < (uint32_t)ctx->num_sms * THIN_MIN_PER_SM)
         g->n_thin = g->n_iso;
+    // the short form for groups of up to TINY_DEGREE neighbours, where they are TINY_SHARE of the tier
+    const uint32_t n_tiny = std::min(ctx->hstate->tiny, g->n_thin);
+    g->tiny = g->n_thin > g->n_iso && n_tiny - g->n_iso >= (g->n_thin - g->n_iso) / TINY_DIV * TINY_MUL;
     g->n_wide_gnn = g->sched == GC_SCHEDULE_DEGREE ? ctx->hstate->gnn_wide : g->n_wide;
     // lists: the hub list and the degree order fit in cap_N; the task list grows when needed
     if (2 * (size_t)n_tasks > g->big_cap) {
