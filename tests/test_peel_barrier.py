@@ -47,3 +47,20 @@ def test_contexts_that_peel_together():
     for t in threads:
         t.join()
     assert results == {k: True for k in range(4)}
+
+
+@pytest.mark.parametrize("name", ["dense", "dense_many", "mixed", "cliques"])
+def test_rounds_that_take_most_vertices(gpu_ctx, name):
+    """SLL thresholds above nearly all degrees: the first round takes (almost) everything, kept or on lists."""
+    N, V, E = {"dense": lambda: gcn.gen_er(20000, 1000000, 1), "dense_many": lambda: gcn.gen_er(620003, 12000000, 2),
+               "mixed": lambda: gcn.gen_rmat(1 << 15, 32, 3),
+               "cliques": lambda: gcn.csr_from_pairs(3000, *[np.asarray(x, np.uint32) for x in (
+                   np.concatenate([np.triu_indices(30, 1)[0] + 30 * k for k in range(100)]),
+                   np.concatenate([np.triu_indices(30, 1)[1] + 30 * k for k in range(100)]))])}[name]()
+    g = gcn.Graph(gpu_ctx, N, V, E)
+    for heur in ("SLL", "SL"):
+        want = O.ordering(heur, N, V, E)
+        for _ in range(2):
+            g.priority(heur)
+            assert np.array_equal(g.priorities(), want), (name, heur)
+    g.close()
