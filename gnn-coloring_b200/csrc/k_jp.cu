@@ -1158,7 +1158,7 @@ __device__ __forceinline__ void stats_record(int *stat, DevState *st, uint32_t n
     }
 }
 
-constexpr int STATS_LOADS = 4;
+constexpr int STATS_LOADS = 4, STATS_WIDE_LOADS = 16;  // (a list of 1,500 by one warp: 25.0 us with 4, 20.3 with 16)
 
 __global__ void __launch_bounds__(256) k_color_stats(const uint32_t *__restrict__ V, const uint32_t *__restrict__ E,
                                                      const int *__restrict__ color, const uint32_t *__restrict__ vorder,
@@ -1185,15 +1185,15 @@ __global__ void __launch_bounds__(256) k_color_stats(const uint32_t *__restrict_
             }
             const int cu = color[u];
             bool hit = false;
-            for (uint32_t j = b + lane; j < e; j += 32 * STATS_LOADS) {
-                uint32_t v[STATS_LOADS];
-                int c[STATS_LOADS];
+            for (uint32_t j = b + lane; j < e; j += 32 * STATS_WIDE_LOADS) {
+                uint32_t v[STATS_WIDE_LOADS];
+                int c[STATS_WIDE_LOADS];
 #pragma unroll
-                for (int k = 0; k < STATS_LOADS; k++) v[k] = j + 32 * k < e ? ld_stream(E + j + 32 * k) : 0u;
+                for (int k = 0; k < STATS_WIDE_LOADS; k++) v[k] = j + 32 * k < e ? ld_stream(E + j + 32 * k) : 0u;
 #pragma unroll
-                for (int k = 0; k < STATS_LOADS; k++) c[k] = j + 32 * k < e ? color[v[k]] : -1;
+                for (int k = 0; k < STATS_WIDE_LOADS; k++) c[k] = j + 32 * k < e ? color[v[k]] : -1;
 #pragma unroll
-                for (int k = 0; k < STATS_LOADS; k++) hit |= j + 32 * k < e && c[k] == cu;
+                for (int k = 0; k < STATS_WIDE_LOADS; k++) hit |= j + 32 * k < e && c[k] == cu;
             }
             if (__any_sync(0xffffffffu, hit) && lane == 0)
                 stats_record(stat, st, nseg, nseg ? seg_of(voff, nseg, u) : 0u, 0, true);
