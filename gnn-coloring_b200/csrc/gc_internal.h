@@ -59,7 +59,7 @@ struct gc_ctx {
     uint32_t flow_max_deg = 128;         // coloring: graphs with a smaller maximum degree go by dataflow (0: none; GC_JP_FLOW)
     int flow_ctas_per_sm = 8;            // dataflow kernel: CTAs per SM at most (GC_JP_FLOW_CTAS)
     unsigned int flow_limit = 1u << 16;  // dataflow kernel: fruitless polls before a warp looks whether anything moves (GC_JP_FLOW_LIMIT)
-    unsigned int narrow_window = 1u << 18;  // cycles after which a coloring is found narrow (0: never; GC_JP_NARROW)
+    unsigned int narrow_window = 192;    // looks at its progress after which a coloring is found narrow (0: never; GC_JP_NARROW)
     uint32_t small_max = GC_SMALL_AUTO;  // coloring: graphs of up to this many vertices that fit go in one CTA (0: none; GC_JP_SMALL)
     bool small_ready = false;            // that kernel's shared-memory limit is set
     int round_blocks_per_sm[3] = {0, 0, 0};  // resident CTAs of each Culberson kernel

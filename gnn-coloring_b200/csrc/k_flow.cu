@@ -21,7 +21,9 @@
 // The queue is FLOW_QUEUES arrays, vertex v in array v mod FLOW_QUEUES, each with its own head and tail
 // counter: a single counter serves an atomic every 0.7 ns, which alone would cost 10 ms for 16.8 M
 // vertices.  The powers of two have 36 different remainders modulo 37, so the strides of a mesh spread over
-// the arrays (modulo 31 they have five, and the 256^3 stencil took 10.5 ms first fit, now 5.1).  Hundreds of
+// the arrays (modulo 31 they have five, and the 256^3 stencil took 10.5 ms first fit, now 5.1).  Where the sides are 2
+// modulo 37 a whole wavefront has one remainder, which costs nothing that shows (first fit 112^3 / 113^3 1,410 / 1,421
+// us, 149^3 / 150^3 2,076 / 2,099).  Hundreds of
 // warps wait at an array's end, each for a slot of its own, so consecutive slots lie in different lines: side
 // by side, their polls and stores met in a few lines (256^3 GNN4 9.0 -> 7.5 ms, Erdos-Renyi 400,000 GNN3 184 ->
 // 134 us, 65,536 LF 96 -> 86).  Every vertex is either queued in its array once or gone on with once (the
@@ -32,7 +34,7 @@
 //
 // A DAG that is narrow -- a band, a strip, a path, a caterpillar -- has its next vertices known long before:
 // its hops cost 0.63 to 3 us here, 0.1 to 0.3 among tickets whose colors stay in one cluster's shared memory
-// (k_jp_core).  So one CTA only counts what becomes ready, in windows of 133 us, and stops a coloring that it finds
+// (k_jp_core).  So one CTA only counts what becomes ready, in windows of 120 us, and stops a coloring that it finds
 // narrow (flow_watch); the tickets then color the graph, as many as fit in the cluster.  First fit, dataflow to
 // the end / this: a path of 20,000 12.8 / 5.2 ms, 20,000 rows of a band matrix with 31 entries on either side 22.9
 // / 2.4, a 5-point strip of 4 x 5,000 3.5 / 1.6, a path of 10,000 with 50 leaves each 23.6 / 2.9.
@@ -48,8 +50,8 @@
 // took up to 15 % longer (256^3 GNN4 10.5 -> 9.0 ms, Erdos-Renyi 400,000 GNN3 229 -> 184 us).
 // Elsewhere the vertices in flight (one per warp, 2 to 3 us each).
 // Measured on a B200, coloring kernels of one job, tickets (sort, cluster core, streams, ticket kernel,
-// leaves) -> dataflow: 256^3 stencil with GNN4 keys 272 -> 8.1 ms, 97 x 61 x 113 stencil first fit
-// 8.9 -> 1.1 ms, random geometric 2^23 GNN4 4.0 -> 2.6 ms, Erdos-Renyi 65,536 LF 0.36 -> 0.10 ms.
+// leaves) -> dataflow: 256^3 stencil with cut-outs, GNN4 keys 272 -> 8.9 ms (the full grid 7.2, first fit 5.7), 97 x 61 x
+// 113 stencil first fit 8.9 -> 1.1 ms, random geometric 2^23 GNN4 4.0 -> 2.6 ms, Erdos-Renyi 65,536 LF 0.36 -> 0.11 ms.
 // Measured and not kept: eight lanes per vertex and four vertices per warp (hops of 3.3 us: the longer
 // code path of a lane is on the chain), a separate 16-byte record (hops of 1.9 us), a slot taken
 // before the color is stored, four slots taken at once under backlog; ready vertices handed to waiting
@@ -198,41 +200,44 @@ __device__ __forceinline__ uint32_t flow_progress(uint32_t *fq, int lane) {
     return __reduce_add_sync(0xffffffffu, n);
 }
 
-// The watching CTA.  A coloring is narrow when in the first window fewer than FLOW_THIN vertices a microsecond became
-// ready (at 1.965 GHz; latencies and the clock change together), or in a later one fewer than FLOW_FEW, while half
-// of what was not ready at the start is still to come and would take four windows more.  By tickets in the cluster, strips of 4 to 50
-// vertices' width run at 11 to 55 a microsecond, bars of 4 x 4 to 16 x 16 at 8 to 23; wavefronts start narrow as
-// well but have passed FLOW_THIN by the end of the first window (a mesh's corner: 50 a microsecond, a square 5-point
-// grid 40), and a second window costs less than a wrong turn.
+// The watching CTA.  A coloring is narrow when in the first window fewer than FLOW_THIN vertices became ready for each
+// look at the counters, or in a later one fewer than FLOW_FEW, while half of what was not ready at the start is
+// still to come and would take four windows more.  A look is a trip to L2 (0.63 us on an idle GPU), as a hop is one or
+// two, and beside other streams' work both get longer together: the clock would take a mesh there for narrow.  Windows
+// begin when all CTAs run.  By tickets in the cluster, strips of 4 to 50 vertices' width run at 11 to 55 vertices a
+// microsecond, bars of 4 x 4 to 16 x 16 at 8 to 23; wavefronts start narrow as well but have passed FLOW_THIN by the end
+// of the first window (a mesh's corner: 50, a square 5-point grid 40), and a second window costs less than a wrong turn.
 // To stop it, FLOW_VOID is added to the counters, so that no vertex becomes ready any more, and to the arrays' skip
 // counters, so that nobody waits for one.  What has started runs to its end, since it only waits for what has started.
 // (The warps that color know nothing of this: a look at a flag in their loops cost path and mesh 40 %.)
-constexpr uint32_t FLOW_THIN = 16, FLOW_FEW = 30, FLOW_MHZ = 1965, FLOW_VOID = 0x2000u;
+constexpr uint32_t FLOW_THIN = 10, FLOW_FEW = 19, FLOW_VOID = 0x2000u;  // (16 and 30 a microsecond)
 
 __device__ void flow_watch(unsigned long long *word, uint32_t *fq, uint32_t N, uint32_t window, DevState *st, uint32_t check) {
     __shared__ bool stop;
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < 32) {
-        uint32_t since = (uint32_t)clock(), ready = flow_progress(fq, lane), last = ready, same = 0;
-        const uint32_t left0 = N - min(ready, N);
-        bool first = true, narrow = false;
+        uint32_t looks = 0, same = 0, ready = 0, last = 0, left0 = 0;
+        bool begun = false, first = true, narrow = false;
         for (;;) {
+            const uint32_t flag = lane == 0 ? ld_relaxed_u32(&st->flow_stall) : 0u;
+            const uint32_t ctas = begun ? gridDim.x : ld_relaxed_u32(fq + FLOW_CTA);
             const uint32_t now = flow_progress(fq, lane), left = N - min(now, N);
-            if (left == 0 || __shfl_sync(0xffffffffu, lane == 0 ? ld_relaxed_u32(&st->flow_stall) : 0u, 0)) break;
+            if (left == 0 || __shfl_sync(0xffffffffu, flag, 0)) break;
             same = now == last ? same + 1u : 0u;
             last = now;
             if (same > check) break;
-            const uint32_t dt = __shfl_sync(0xffffffffu, (uint32_t)clock() - since, 0);
-            if (dt >= window) {
-                const unsigned long long got = now - ready;
-                narrow = got * FLOW_MHZ < (unsigned long long)dt * (first ? FLOW_THIN : FLOW_FEW) && left >= left0 / 2 &&
-                         (unsigned long long)left * dt >= 4 * got * window;
+            if (!begun) {
+                begun = ctas >= gridDim.x;
+                ready = now;
+                left0 = left;
+            } else if (++looks == window) {
+                const uint32_t got = now - ready;
+                narrow = got < window * (first ? FLOW_THIN : FLOW_FEW) && left >= left0 / 2 && left >= 4ull * got;
                 if (narrow) break;
-                since += dt;
+                looks = 0;
                 ready = now;
                 first = false;
             }
-            __nanosleep(500);
         }
         if (lane == 0) {
             stop = narrow;
@@ -477,8 +482,8 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
         ProfScope ps(ctx, "jp_flow", ctx->stream);
         // at least FLOW_MIN_CTAS; a warp per four vertices at most; up to FLOW_FEW_N
         // vertices half of what fits, since the chains are then all there is and idle warps' polls slow them
-        // (8 / 4 per SM, one slot's list fetched later: Erdos-Renyi 65,536 LF 113 / 102 us, GNN3 128 / 115, random
-        // geometric 200,000 108 / 99; 500,000 149 / 195, Erdos-Renyi 600,000 226 / 279)
+        // (colorings with keys by degree, 8 / 4 per SM: Erdos-Renyi 65,536 130 / 126 us, random geometric 200,000 116 /
+        // 126, 500,000 189 / 226, Erdos-Renyi 600,000 270 / 360)
         const int per_sm = std::min(occ, N <= FLOW_FEW_N ? std::max(1, ctx->flow_ctas_per_sm / 2) : ctx->flow_ctas_per_sm);
         const uint32_t most = (uint32_t)ctx->num_sms * (uint32_t)per_sm;
         // (a long path stays: one successor per hop is 0.63 us here, and past the cluster's tickets 0.73 there)
@@ -507,8 +512,10 @@ gc_status flow_run(gc_graph *g, uint32_t stride) {
 // below FLOW_WIDE_MEAN: there most vertices are a whole warp's work for a few entries (arity-100 tree of 2^20
 // vertices, dataflow / tickets: random priorities 429 / 248, first fit 213 / 187).  Larger degrees would put long
 // lists on the chain, and power-law graphs have their chains colored inside one cluster (k_jp_core).
-// Plain graphs only: a batch is captured, and the stall flag needs the host.
-// (And no nearly complete graphs: one chain, for the cluster.)
+// (The line is the whole graph's: one vertex of 200 neighbours sends a mesh to the tickets, 112^3 first fit 1.4 -> 6.8 ms
+// by two streams.)
+// Plain graphs only: the rule, the masks' width and the queues are one graph's.  And no nearly complete graphs: one
+// chain, for the cluster.
 constexpr uint32_t FLOW_WIDE_MAX_N = 1u << 20, FLOW_WIDE_MEAN = 4, FLOW_CLIQUE = 100;
 
 bool gc_flow_eligible(const gc_graph *g) {

@@ -983,15 +983,16 @@ __device__ __forceinline__ int color_light(const uint32_t *__restrict__ list, ui
 }
 
 // A narrow DAG (a band with long lists, a wheel) has few vertices in flight here, 0.5 to 1.3 us per hop, where the
-// cluster takes 0.1 to 0.3.  So CTA 0 first watches a sample of the tickets for three windows of 133 us, and stops the
-// coloring when in all they got their colors at fewer than NARROW_RATE a microsecond (at 1.965 GHz), while half of
-// them and four windows' work are still to come: no more tickets, and -1 for every color, which ends all waits.  The
+// cluster takes 0.1 to 0.3.  So CTA 0 first watches a sample of the tickets for three windows, and stops the
+// coloring when in all of them they got their colors at fewer than NARROW_RATE a look (0.8 us on an idle GPU, longer
+// beside other work, as hops are; 16 a microsecond), while half of them and four windows' work are still to come: no
+// more tickets, and -1 for every color, which ends all waits.  The windows, 155 us each, begin when all CTAs run.  The
 // host then colors the graph with as many tickets as fit in the cluster.  (R-MAT without a core spends two windows in
 // its clique of hubs, and is done in the third.)  With more tickets than NARROW_MAX the cluster would take too few of
-// them.  First fit, not watched / watched: wheels of
-// 9,000 and 50,000 vertices 6.7 / 2.9 and 37.5 / 21.6 ms, 30,000 rows of a band matrix with 100 entries on either side
-// 24.4 / 12.4, 50,000 with 200 44.2 / 29.4.  (As a function of its own the watch cost the kernel 3 %.)
-constexpr uint32_t NARROW_RATE = 16, NARROW_WINDOWS = 3, NARROW_MHZ = 1965, NARROW_MIN = 512, NARROW_MAX = 131072, NARROW_SAMPLES = 4;
+// them.  First fit, not watched / watched: wheels of 9,000 and 50,000 vertices 6.7 / 3.0 and 38.0 / 21.9 ms, 30,000
+// rows of a band matrix with 100 entries on either side 24.5 / 12.6, 50,000 with 200 44.3 / 29.7.  (As a function of
+// its own the watch cost the kernel 3 %.)
+constexpr uint32_t NARROW_RATE = 13, NARROW_WINDOWS = 3, NARROW_MIN = 512, NARROW_MAX = 131072, NARROW_SAMPLES = 4;
 
 __device__ __forceinline__ void ticket_watch(const uint4 *__restrict__ rec, int *color, DevState *st, uint32_t window) {
     const uint32_t n = ld_relaxed_u32(&st->ordered), samples = min(n, NARROW_SAMPLES * blockDim.x);
@@ -1002,7 +1003,7 @@ __device__ __forceinline__ void ticket_watch(const uint4 *__restrict__ rec, int 
         const uint32_t i = k * blockDim.x + threadIdx.x;
         v[k] = i < samples ? rec[(unsigned long long)i * n / samples].x : 0xffffffffu;
     }
-    uint32_t since = 0, first = 0, start = 0, windows = 0;
+    uint32_t looks = 0, first = 0, start = 0, windows = 0;
     for (bool begin = true;;) {
         int c[NARROW_SAMPLES];
 #pragma unroll
@@ -1012,18 +1013,15 @@ __device__ __forceinline__ void ticket_watch(const uint4 *__restrict__ rec, int 
         for (uint32_t k = 0; k < NARROW_SAMPLES; k++) done += __syncthreads_count(c[k] != 0);
         if (done == samples || __syncthreads_or(threadIdx.x == 0 && ld_relaxed_u32(&st->err))) return;
         if (begin) {
+            // (the first window waits until all CTAs run)
+            if (windows || __syncthreads_or(threadIdx.x == 0 && ld_relaxed_u32(&st->count) >= gridDim.x)) begin = false;
             first = done;
             if (!windows) start = done;
-            since = (uint32_t)clock();
-            begin = false;
-        }
-        const uint32_t dt = (uint32_t)clock() - since;
-        if (__syncthreads_or(threadIdx.x == 0 && dt >= window)) {
+        } else if (++looks == window) {
             const unsigned long long got = (unsigned long long)(done - first) * n / samples, left = samples - done;
-            const bool narrow = got * NARROW_MHZ < (unsigned long long)dt * NARROW_RATE && 2 * left >= samples - start &&
-                                left * n / samples * dt >= 4 * got * window;
-            if (!__syncthreads_or(threadIdx.x == 0 && narrow)) return;
+            if (got >= (unsigned long long)window * NARROW_RATE || 2 * left < samples - start || left * n / samples < 4 * got) return;
             if (++windows == NARROW_WINDOWS) break;
+            looks = 0;
             begin = true;
         }
     }
@@ -1052,7 +1050,10 @@ __global__ void __launch_bounds__(COLOR_WARPS_PER_CTA * 32, 5) k_jp_color(const 
                                                                        const unsigned long long *epoch_word,
                                                                        const uint4 *__restrict__ split, uint32_t cap,
                                                                        int light_warps, uint32_t window) {
-    if (window && blockIdx.x == 0) ticket_watch(rec, color, st, window);
+    if (window) {
+        if (threadIdx.x == 0) atomicAdd(&st->count, 1u);
+        if (blockIdx.x == 0) ticket_watch(rec, color, st, window);
+    }
     __shared__ uint32_t forbid[COLOR_WARPS_PER_CTA][32];
     __shared__ uint32_t pending[COLOR_WARPS_PER_CTA][PENDING];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1277,6 +1278,7 @@ __global__ void k_reset_ticket(DevState *st, unsigned long long *epoch_word, uin
         st->n_heavy = st->n_light = 0;
     }
     st->big_leaves = 0;
+    st->count = 0;
     if (epoch_word) {
         const unsigned long long e = (*epoch_word + 1) & 0xffffffffull;
         *epoch_word = e ? e : 1;
