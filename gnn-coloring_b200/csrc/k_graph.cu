@@ -192,12 +192,12 @@ gc_status gc_graph_prepare(gc_graph *g) {
     g->max_deg = ctx->hstate->max_color;
     uint32_t n_tasks = ctx->hstate->count, n_hubs = ctx->hstate->count2;
     g->n_wide = ctx->hstate->min_deg;
-    // The GNN's thin tier: up to ctx->gnn_thin_deg neighbours, or the whole graph where no vertex has
-    // more than THIN_WHOLE (half that up to 2^19 vertices) or THIN_SKEW times the mean (one kernel per layer instead of two: 3 layers over an Erdos-Renyi
-    // graph of 400,000 vertices 297 -> 186 us; in a skewed graph the other tiers run anyway, and groups of up to 64
-    // neighbours only lengthen its tail: R-MAT of 100,003 vertices 230 us with 16, 280 with 64, a path of 5,000 with 100
-    // leaves each 176 with 16, 335 throughout; 2,000 cliques of 100 257 with the quad tier, 291 throughout, but 8,000 of
-    // 120 1,220 and 1,193, Erdos-Renyi 1 M x 60 1,162 and 1,111).
+    // The GNN's thin tier: up to ctx->gnn_thin_deg neighbours, or the whole graph where no vertex has more than
+    // THIN_WHOLE (half that up to 2^19 vertices) or THIN_SKEW times the mean (one kernel per layer instead of two: 3
+    // layers over an Erdos-Renyi graph of 400,000 vertices 297 -> 186 us; in a skewed graph the other tiers run anyway,
+    // and groups of up to 64 neighbours only lengthen its tail: R-MAT of 100,003 vertices 230 us with 16, 280 with 64,
+    // a path of 5,000 with 100 leaves each 176 with 16, 335 throughout; 2,000 cliques of 100 257 with the quad tier,
+    // 291 throughout, but 8,000 of 120 1,220 and 1,193, Erdos-Renyi 1 M x 60 1,162 and 1,111).
     // Below one group for each resident warp the chip is half idle and a vertex's own chain is what
     // counts, which the quad tier keeps shorter: Erdos-Renyi 65,536 90 us here, 80 there; 150,000
     // 136 and 123; 200,000 144 and 139; 400,000 186 and 233; R-MAT 100,003 193 and 183, 1 M 429 and 551.

@@ -832,14 +832,15 @@ __global__ void __launch_bounds__(CORE_WARPS * 32, 1) k_jp_core(const uint4 *__r
 // 400 graphs, 17 M vertices, largest degree first: 7.5 ms a pass with half of each CTA's warps on the
 // light stream, 15.1 ms without streams; eight lanes per light vertex, with early decisions, 11.9 ms.
 // A power-law graph keeps one stream: its chains run through its hubs and light vertices in turn, and a lane tells
-// its color only when its whole warp is through (core + streams + ticket kernel of R-MAT 100,003, GNN3 keys: 0.28
-// ms with streams, 0.13 without; 2^20 vertices, first fit: 1.55 and 0.70).  In other graphs of that size the hubs are not
-// on the chains (whole calls, first fit / random priorities, one stream -> two: 27-point stencil of 1.4 M and a vertex
-// of 200 neighbours 20.4 -> 6.8 ms / 1,354 -> 735 us, Erdos-Renyi 2 M x 8 and 20 hubs of 5,000 1,443 -> 564 / 1,625 ->
-// 793, 1 M x 8 and 20,000 of 300 939 -> 557 / 1,048 -> 676; 5-point grid 3.4 -> 7.4 ms / 662 -> 325), but trees have
-// too few inner vertices to split (arity 300 176 -> 184 / 234 -> 250: a mean degree of STREAMS_MEAN).  Where two hubs are sure to be neighbours, were the edges drawn at random -- the largest
-// degree squared is above STREAMS_CLIQUE entries -- there is a clique of them (R-MAT of 2^20 to 2^22 vertices 42 to 208
-// times the entries, the others 6 at most).
+// its color only when its whole warp is through (core + streams + ticket kernel of R-MAT 100,003, GNN3 keys: 0.28 ms
+// with streams, 0.13 without; 2^20 vertices, first fit: 1.55 and 0.70).  In other graphs of that size the hubs are
+// not on the chains (whole calls, first fit / random priorities, one stream -> two: 27-point stencil of 1.4 M and a
+// vertex of 200 neighbours 20.4 -> 6.8 ms / 1,354 -> 735 us, Erdos-Renyi 2 M x 8 and 20 hubs of 5,000 1,443 -> 564 /
+// 1,625 -> 793, 1 M x 8 and 20,000 of 300 939 -> 557 / 1,048 -> 676; 5-point grid 3.4 -> 7.4 ms / 662 -> 325), but
+// trees have too few inner vertices to split (arity 300 176 -> 184 / 234 -> 250: a mean degree of STREAMS_MEAN).
+// Where two hubs are sure to be neighbours, were the edges drawn at random -- the largest degree squared is above
+// STREAMS_CLIQUE entries -- there is a clique of them (R-MAT of 2^20 to 2^22 vertices 42 to 208 times the entries,
+// the others 6 at most).
 // A batch or graph of up to jp_light_min vertices, few of which wait for a warp, keeps one stream too (passes with /
 // without: 4 graphs, 20,000 vertices, largest degree first 196 / 156 us; 8 of 418,000, first fit 1,042 / 486; 96 of
 // 622,000, 715 / 991; 64 of 2.2 M, largest degree first 1,121 / 1,527).

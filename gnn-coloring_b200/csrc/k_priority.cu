@@ -47,11 +47,12 @@ __global__ void k_simple_keys(const uint32_t *__restrict__ V, uint32_t N, int h,
 //     takes what that array has lost since it last looked off the vertex's degree.  So nobody reads what
 //     others are counting down, and a removed vertex's neighbours are counted down at once: lists of up to
 //     PEEL_WARP_DEG by its warp, eight lanes each, longer ones by its CTA.
-//   - The decrements go to every neighbour without asking whether it is still there (nothing reads a
-//     removed vertex's degree again), so nothing waits for their results.  They do ask where most vertices of a
-//     graph with a mean degree of PEEL_DENSE and more leave together: in the first round of a graph whose vertices are all kept, by their lists' lengths, and after a
-//     round over lists that took three quarters of what there was, by the degrees, which then say GONE.  SLL on Erdos-Renyi graphs of
-//     300,000 x 200 and 1 M x 100: 578 and 851 us without asking, 404 and 575 so.
+//   - The decrements go to every neighbour without asking whether it is still there (nothing reads a removed vertex's
+//     degree again), so nothing waits for their results.  They do ask where most vertices of a graph with a mean
+//     degree of PEEL_DENSE and more leave together: in the first round of a graph whose vertices are all kept, by
+//     their lists' lengths, and after a round over lists that took three quarters of what there was, by the degrees,
+//     which then say GONE.  SLL on Erdos-Renyi graphs of 300,000 x 200 and 1 M x 100: 578 and 851 us without asking,
+//     404 and 575 so.
 //   - SL tries delta + 1 first; only when that removes nothing does it look for the smallest remaining
 //     degree (one more barrier).
 //   - The barrier's counter and the round's count are one 64-bit word, polled by one thread per CTA: a scalar

@@ -19,11 +19,12 @@
 // The rounds are queued without host synchronisation (the number of colors never grows, so the first
 // round's bound on the key width holds for all), and can be captured.
 //
-// What bounds it: each round reads E once and gathers one word per edge.  On the 256^3 stencil (1.16 ms)
+// What bounds it: each round reads E once and gathers one word per edge.  On the 256^3 stencil (1.12 ms, 1.35 with the
+// sort)
 // the rows in class order cost 1.6 x their bytes in 64-byte pieces, and half the issue slots go by waiting
 // for them; on the random geometric graph the L1 serves one gather per cycle (80 % of its peak).
-// Measured per round (B200), lists of predecessors + class by class before -> this: 256^3 stencil
-// 3.3 -> 1.4 ms, random geometric 2^23 1.9 -> 0.77 ms, R-MAT of 100,003 vertices 1.25 -> 0.25 ms (there a
+// Measured per round with its sort (B200), lists of predecessors + class by class before -> this: 256^3 stencil
+// 3.3 -> 1.35 ms, random geometric 2^23 1.9 -> 0.77 ms, R-MAT of 100,003 vertices 1.25 -> 0.25 ms (there a
 // warp colored up to 32 large vertices of a class in turn).
 #include <algorithm>
 
@@ -366,7 +367,7 @@ __device__ __forceinline__ void round_hub(const uint32_t *__restrict__ order, ui
 // (old color << 8 | new), and a predecessor's color sets its own bit of one 32-bit mask -- bit 0 when it
 // has none yet, so that one reduction over the group's lanes gives both the free color and whether
 // anything must be waited for.  Per entry that leaves a compare, a shift and an or: a round on the 256^3
-// stencil takes 1.16 ms in 32 registers (a full SM of warps) against 1.23 ms in the general kernel.
+// stencil took 1.16 ms in 32 registers (a full SM of warps) against 1.23 ms in the general kernel.
 // With longer lists the extra entries cost more than that (random geometric, 2^23 vertices, at most 37
 // neighbours: 0.69 ms here with eight entries per lane, 0.81 with the entries past 32 read in place, 0.65
 // in the general kernel).

@@ -97,7 +97,8 @@ __device__ __forceinline__ void for_vertices(const Small &s, F f, G g) {
     }
 }
 
-// Colors u by G lanes with UN entries in flight each (32 / G vertices per warp, all lanes take part; `valid`: this group has a vertex).
+// Colors u by G lanes with UN entries in flight each (32 / G vertices per warp, all lanes take part; `valid`: this group
+// has a vertex).
 template <int G, int UN>
 __device__ __forceinline__ void color_vertex(const Small &s, uint32_t u, bool valid, uint32_t lbase, uint32_t hbase,
                                              uint32_t slot) {
