@@ -14,8 +14,8 @@ JP.  Metric: colored edges/s = |E| (directed CSR length, the reference's |E|) / 
           from pinned memory, H2D of V/E and D2H of p/colors inside every timed step.
   roofline  the dominant bandwidth-bound kernel's algorithmic bytes per launch / its average
           event-timed duration, against MEASURED_PEAKS.json's HBM copy bandwidth.  Kernels with no
-          byte roofline (the JP core, a chain of dependent colors; the exact hub sums, bound by
-          their add arithmetic) are listed in `other_bounds` with their share of the job.
+          byte roofline (the coloring kernels, chains of dependent colors; the exact hub sums, bound
+          by their add arithmetic) are listed in `other_bounds` with their share of the job.
   cpu_baseline  the reference's own OpenMP code (oracle/_ref) on the host cores, same job; its
           p and colors are the parity check of the GPU result (`parity`), and the other
           workloads (`configs`) are checked the same way, Culberson round by round.
@@ -139,10 +139,13 @@ def algorithmic_bytes(kernel: str, N: int, M: int, P: int) -> float:
         "gnn_output": 4 * M + 4 * N + 64 * N + 4 * N,    # E, V, own x row, key
         "gnn_table0": 4 * N + 8 * N,
         "jp_split": 4 * M + 4 * N + 4 * N + 4 * P + 4 * N + 4 * N,  # E, V, key, P written, pc, color reset
-        "jp_color": 4 * N + 4 * N + 4 * N + 4 * P + 4 * N,          # order, V, pc, P read, color written
         "sort_pass": 4 * N * 4,                                      # keys+ids read and written
     }
     return float(table.get(kernel, 0))
+
+
+# Groups that wait for one vertex's color after another, or for one round after another: no byte roofline.
+CHAINS = ("jp_core", "jp_color", "jp_flow", "jp_small", "jp_round", "peel")
 
 
 def step_bytes(N: int, M: int, layers: int = 3) -> float:
@@ -460,7 +463,7 @@ def run_ours(args):
     byte_bound = [k for k in kernels if algorithmic_bytes(k, N, M, P) > 0]
     dominant = max(byte_bound, key=lambda k: kernels[k]["ms_per_step"]) if byte_bound else None
     other_bounds = {k: {"ms_per_step": v["ms_per_step"], "share": v["ms_per_step"] / ms_per_step,
-                        "bound": "dependency chain (latency)" if k.startswith("jp_core") else
+                        "bound": "dependency chain (latency)" if k in CHAINS else
                         "FP32 add arithmetic (exact sums); the span from the layer's start on a high-priority "
                         "side stream, whose CTAs take SMs as the layer kernel's leave them, so it overlaps the "
                         "layer kernels' time" if k.startswith("gnn_hub") else "launch/latency"}
