@@ -993,7 +993,8 @@ __device__ __forceinline__ int color_light(const uint32_t *__restrict__ list, ui
 // them.  First fit, not watched / watched: wheels of 9,000 and 50,000 vertices 6.7 / 3.0 and 38.0 / 21.9 ms, 30,000
 // rows of a band matrix with 100 entries on either side 24.5 / 12.6, 50,000 with 200 44.3 / 29.7.  (As a function of
 // its own the watch cost the kernel 3 %.)
-constexpr uint32_t NARROW_RATE = 13, NARROW_WINDOWS = 3, NARROW_MIN = 512, NARROW_MAX = 131072, NARROW_SAMPLES = 4;
+constexpr uint32_t NARROW_RATE = 13, NARROW_WINDOWS = 3, NARROW_MIN = 512, NARROW_MAX = 131072, NARROW_SAMPLES = 4,
+                   NARROW_START = 16;
 
 __device__ __forceinline__ void ticket_watch(const uint4 *__restrict__ rec, int *color, DevState *st, uint32_t window) {
     const uint32_t n = ld_relaxed_u32(&st->ordered), samples = min(n, NARROW_SAMPLES * blockDim.x);
@@ -1014,15 +1015,16 @@ __device__ __forceinline__ void ticket_watch(const uint4 *__restrict__ rec, int 
         for (uint32_t k = 0; k < NARROW_SAMPLES; k++) done += __syncthreads_count(c[k] != 0);
         if (done == samples || __syncthreads_or(threadIdx.x == 0 && ld_relaxed_u32(&st->err))) return;
         if (begin) {
-            // (the first window waits until all CTAs run)
+            // (the first window waits until all CTAs run, within a limit: then this one colors too)
             if (windows || __syncthreads_or(threadIdx.x == 0 && ld_relaxed_u32(&st->count) >= gridDim.x)) begin = false;
+            else if (++looks == NARROW_START * window) return;
+            if (!begin) looks = 0;
             first = done;
             if (!windows) start = done;
         } else if (++looks == window) {
             const unsigned long long got = (unsigned long long)(done - first) * n / samples, left = samples - done;
             if (got >= (unsigned long long)window * NARROW_RATE || 2 * left < samples - start || left * n / samples < 4 * got) return;
             if (++windows == NARROW_WINDOWS) break;
-            looks = 0;
             begin = true;
         }
     }
